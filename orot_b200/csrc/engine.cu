@@ -203,9 +203,29 @@ static uint64_t put_table(std::vector<uint8_t>& buf, const std::vector<T>& v) {
   return off;
 }
 
+// Tiles per search group: one CTA per SM searches a group, so the pass takes
+// (waves of groups) x (tiles per group, plus what staging a group and the
+// last long chains of its lanes cost, about a tile's time).
+uint32_t Engine::search_group() const {
+  if (lazy_run_override) return std::min(kSearchTiles, lazy_run_override);
+  uint32_t best = 1;
+  uint64_t best_cost = ~uint64_t(0);
+  for (uint32_t G = 1; G <= kSearchTiles; ++G) {
+    uint64_t groups = 0;
+    for (uint32_t si : lists[kLazySegs]) groups += (segs[si].tile_count + G - 1) / G;
+    const uint64_t cost = (groups + sms - 1) / sms * (G + 1);
+    if (cost <= best_cost) {
+      best_cost = cost;
+      best = G;
+    }
+  }
+  return best;
+}
+
 bool Engine::plan(const std::vector<Job>& jobs) {
   streams.clear(); segs.clear(); tiles.clear(); cks.clear();
   for (auto& l : lists) l.clear();
+  any_lazy = any_opt = false;
   uint64_t total = 0;
   max_out_cap = 0;
   for (const Job& j : jobs) {
@@ -282,16 +302,26 @@ bool Engine::plan(const std::vector<Job>& jobs) {
         g.tile_count = nt;
         const uint32_t seg_index = uint32_t(segs.size());
         lists[kLazySegs].push_back(seg_index);
+        (lv >= 10 ? any_opt : any_lazy) = true;
+        // the tiles' bit buffers lie back to back, 2 bytes per position and
+        // more each: the links (2 bytes per position) live there until the
+        // tiles are encoded
+        g.links = scratch;
+        const uint64_t bits0 = scratch;
+        for (uint32_t t = 0; t < nt; ++t)
+          scratch += lazy_stream_bytes(uint32_t(std::min<uint64_t>(LT, len - std::min<uint64_t>(len, uint64_t(t) * LT))));
+        uint64_t bits_at = bits0;
+        g.toks = scratch;
+        scratch += align_up(uint64_t(len) * 4 + 4, 256);
         for (uint32_t t = 0; t < nt; ++t) {
           Tile tl{};
           tl.seg = seg_index;
           tl.start = t * LT;
           tl.len = uint32_t(std::min<uint64_t>(LT, len - std::min<uint64_t>(len, uint64_t(t) * LT)));
           tl.index = t;
-          tl.scratch = scratch;
-          scratch += lazy_stream_bytes(tl.len);
-          tl.tok = scratch;
-          scratch += align_up(uint64_t(tl.len) * 4 + 4, 256);
+          tl.scratch = bits_at;
+          bits_at += lazy_stream_bytes(tl.len);
+          tl.tok = g.toks + uint64_t(tl.start) * 4;
           tl.hist = scratch;
           scratch += 320 * 4;
           lists[kLazyTiles].push_back(uint32_t(tiles.size()));
@@ -350,10 +380,10 @@ bool Engine::plan(const std::vector<Job>& jobs) {
   off_segs = put_table(buf, segs);
   off_tiles = put_table(buf, tiles);
   off_ck = put_table(buf, cks);
-  // Lazy tiles go to CTAs in runs of consecutive tiles of one segment (the
-  // window slides from tile to tile, and every run first builds the links of
-  // its whole window).  Short runs give small passes enough CTAs for every
-  // SM; long runs build fewer windows.  The run length per level group and
+  // Links are built in runs of consecutive tiles of one segment (one CTA goes
+  // through a run after entering the 32 KiB before it in its table).  Short
+  // runs give small passes enough CTAs for every SM; long runs enter fewer
+  // windows.  The run length per level group and
   // pass size is the autotuner's (geometry_table.h).
   if (!lists[kLazySegs].empty()) {
     const GeometryRow& geo = geometry(total);
@@ -364,6 +394,17 @@ bool Engine::plan(const std::vector<Job>& jobs) {
       for (uint32_t t = 0; t < g.tile_count; t += R) {
         lists[kLazyRuns].push_back(g.tile_first + t);
         lists[kLazyRuns].push_back(std::min(R, g.tile_count - t));
+      }
+    }
+    const uint32_t G = search_group();
+    for (uint32_t si : lists[kLazySegs]) {
+      const Segment& g = segs[si];
+      const uint32_t n = (g.tile_count + G - 1) / G;  // groups of nearly equal size
+      for (uint32_t k = 0, t = 0; k < n; ++k) {
+        const uint32_t c = (g.tile_count - t + (n - k) - 1) / (n - k);
+        lists[kLazyGroups].push_back(g.tile_first + t);
+        lists[kLazyGroups].push_back(c);
+        t += c;
       }
     }
   }
@@ -436,11 +477,15 @@ bool Engine::launch(cudaStream_t st) {
     LazyLists L{};
     L.runs = list(kLazyRuns);
     L.n_runs = uint32_t(lists[kLazyRuns].size() / 2);
+    L.groups = list(kLazyGroups);
+    L.n_groups = uint32_t(lists[kLazyGroups].size() / 2);
     L.tiles = list(kLazyTiles);
     L.n_tiles = uint32_t(lists[kLazyTiles].size());
     L.segs = list(kLazySegs);
     L.n_segs = uint32_t(lists[kLazySegs].size());
     L.counter = counters + 2;
+    L.any_lazy = any_lazy;
+    L.any_opt = any_opt;
     launches += launch_lazy(w, L, st, sms, &marks);
   }
   launch_plan(w, max_out_cap, st);

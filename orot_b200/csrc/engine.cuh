@@ -66,6 +66,8 @@ struct Segment {
   uint64_t hdr_off;    // scratch byte offset of the HLIT..code-lengths bits
   uint32_t hdr_bits;
   uint32_t eob;        // EOB code | (code length << 16)
+  uint64_t links;      // scratch byte offset of the links (u16 per position, 16-byte aligned)
+  uint64_t toks;       // scratch byte offset of the token words (u32 per position)
   // filled by the planner kernel
   uint32_t block_type;
   uint32_t piece_off;  // first copy slot of this block, from the stream's piece_first
@@ -146,10 +148,11 @@ __host__ __device__ inline uint64_t lazy_stream_bytes(uint32_t tile_len) { retur
 // Levels 4+: tiles of 16 x 258 bytes, each searching a 32 KiB window before
 // it.  A multiple of the longest match keeps runs of 258-byte matches (zero
 // fill, short periods) aligned with tile boundaries, so cutting the input
-// into independent tiles costs no extra token on such data.  One CTA walks a
-// run of kLazyRun consecutive tiles, sliding its window.
+// into independent tiles costs no extra token on such data.  One CTA links
+// a run of at most kLazyRun consecutive tiles.
 constexpr uint32_t kLazyTile = 16 * 258;
 constexpr uint32_t kLazyRun = 32;
+constexpr uint32_t kSearchTiles = 9;  // and searches at most this many
 constexpr uint32_t kLazyWindow = 32768;
 
 }  // namespace orotb

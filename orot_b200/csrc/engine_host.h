@@ -55,7 +55,7 @@ struct Job {
 enum ListId {
   kLast12, kMulti12, kWalk12,
   kLast14, kMulti14, kWalk14,
-  kLazyTiles, kLazySegs, kLazyRuns,
+  kLazyTiles, kLazySegs, kLazyRuns, kLazyGroups,
   kNumLists
 };
 
@@ -83,6 +83,7 @@ class Engine {
   void use_stream_ordered_arenas();
   uint32_t pick_tile(uint64_t total_bytes, int hash_bits) const;
   const GeometryRow& geometry(uint64_t total_bytes) const;
+  uint32_t search_group() const;
 
   int device = 0, sms = 148;
   bool ok = false;  // the stream and the device's constant tables are set up
@@ -100,6 +101,7 @@ class Engine {
   std::vector<CkBlock> cks;
   std::vector<uint32_t> lists[kNumLists];
   uint32_t n_pieces = 0;
+  bool any_lazy = false, any_opt = false;  // segments of levels 4-9 / 10-12 in the pass
   uint64_t scratch_bytes = 0, upload_bytes = 0;
   uint64_t max_out_cap = 0;  // largest output slot of the planned pass
   uint64_t off_streams = 0, off_segs = 0, off_tiles = 0, off_ck = 0, off_pieces = 0, off_counters = 0;

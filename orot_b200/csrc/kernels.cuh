@@ -47,11 +47,14 @@ struct FastLists {
 struct LazyLists {
   const uint32_t* runs;      // (first tile, tile count) of every run, count <= kLazyRun
   uint32_t n_runs;
+  const uint32_t* groups;    // (first tile, tile count) of every search group, count <= kSearchTiles
+  uint32_t n_groups;
   const uint32_t* tiles;     // tiles to encode
   uint32_t n_tiles;
   const uint32_t* segs;      // segments needing Huffman tables
   uint32_t n_segs;
   uint32_t* counter;
+  bool any_lazy, any_opt;    // tiles of levels 4-9 / 10-12 among them
 };
 
 // Optional per-phase CUDA events: mark(id) records an event after phase id.

@@ -25,13 +25,14 @@
 //     the ITU-T T.81 Annex K.3 length limiter, and the block type is chosen
 //     on exact sizes (the reference uses a flat header estimate).
 //
-//   k_lz     one CTA per run of consecutive tiles, sliding the staged window,
-//            the links and the hash table from tile to tile: links built in
-//            parallel chunks plus one ordered table pass, the match searched
-//            at every position (lanes take new positions as their chains
-//            end), the lazy parse split
-//            across lanes with a convergence fix-up, then a block-wide
-//            max-scan marks covered bytes and fills the histogram.
+//   k_link   one CTA per run of tiles: the link of every position to the
+//            previous one with the same hash, into scratch.
+//   k_search one CTA per group of tiles: their input, window and links
+//            staged by bulk copies, the match searched at every position
+//            (lanes take new positions as their chains end).
+//   k_lparse one CTA per tile: the lazy parse split across lanes with a
+//            convergence fix-up (levels 10-12: then the optimal parse), token
+//            words and the histogram.
 //   k_huff   one warp per segment: code lengths, canonical codes, block type,
 //            RLE code-length header (deflate_block.cpp:196-290 rules).
 //   k_enc    one warp per tile: resolves tokens 32 positions at a time and
@@ -48,23 +49,8 @@ namespace {
 
 constexpr uint32_t kAll = 0xFFFFFFFFu;
 constexpr uint32_t T = kLazyTile, W = kLazyWindow;
-constexpr uint32_t kRegion = W + T;                            // positions with links
-constexpr uint32_t kDataBytes = (W + T + 48 + 127) / 128 * 128;  // + align + over-read tail
-constexpr uint32_t kLinkBytes = (kRegion * 2 + 127) / 128 * 128;  // u16 per position
-constexpr uint32_t kTblBytes = 65536;                          // u16 per 15-bit hash, kept across a run
-constexpr uint32_t kFBytes = T * 4;                            // F[T]; link marks before the search
-constexpr uint32_t kTokBytes = T * 4;
-constexpr uint32_t kFmWords = T / 32;
-constexpr uint32_t kOptBytes = T * 2 + 320 * 2 + 260 * 2;      // optimal parse: choice[T], symbol and length costs
-constexpr uint32_t kSmemLz = kDataBytes + kLinkBytes + kTblBytes + kFBytes + kTokBytes + kFmWords * 4 + 320 * 4 +
-                             64 * 4 + kOptBytes;
-static_assert(T % 32 == 0, "tiles are whole windows of 32 positions");
-static_assert(kSmemLz <= 227 * 1024, "one CTA per SM");
-static_assert((T & 1) == 0 && (W & 1) == 0, "window shifts move whole u32 words of links");
-static_assert((kRegion + 31) / 32 * 8 <= kFBytes, "first/last marks of every link chunk fit F");
-
-constexpr uint32_t kSerialParse = 128;  // at most this many match positions: serial parse
-constexpr int kStepsPerRound = 8;       // chain steps a searching lane takes between re-balancing rounds
+constexpr uint32_t kMaxDist = 32767;     // farthest candidate a search takes
+constexpr uint32_t kLinkDiff = 0x8000u;  // link flag: the linked position starts with other 4 bytes (alone: no link)
 
 // chain, nice, lazy depth, miss limit, optimal parse (levels 10-12)
 struct LazyCfg { int chain, nice, lazy, miss, opt; };
@@ -81,209 +67,14 @@ struct SmemBytes {
     const uint32_t i = r + boff;
     return __funnelshift_r(w[i >> 2], w[(i >> 2) + 1], (i & 3) * 8);
   }
-  __device__ __forceinline__ uint32_t byte(uint32_t r) const {
-    const uint32_t i = r + boff;
-    return (w[i >> 2] >> ((i & 3) * 8)) & 0xFFu;
-  }
 };
 
 __device__ __forceinline__ uint32_t hash16(uint32_t v) { return (v * 0x9E3779B1u) >> 16; }
 __device__ __forceinline__ uint32_t hash15(uint32_t v) { return (v * 0x9E3779B1u) >> 17; }
 
-// The longest match at region position r, walking the chain newest first
-// with the reference's rules (src/deflate/lz77.cpp:66-156): candidates of the
-// same 15-bit bucket but another 16-bit hash are skipped, `chain` candidates
-// with the same 16-bit hash are examined, miss_limit consecutive 4-byte
-// mismatches end the walk, the quick reject at byte `best` skips candidates
-// that cannot be longer, ties keep the nearest, nice length ends the walk.
-// The walk advances one candidate per lz_step call so that a lane can start
-// its next position as soon as its chain ends.
-struct LzState {
-  uint32_t r, v4p, h16p, q, maxm, best, bd;
-  uint32_t pqr;  // the 4 bytes of r ending at byte `best` (the quick reject's p side), once best >= 4
-  uint32_t nl;   // link of the current candidate (loaded with it, so the next step does not wait for it)
-  int steps, miss, bud;
-};
-
-__device__ __forceinline__ void lz_begin(LzState& s, const SmemBytes& sd, const uint16_t* __restrict__ link, uint32_t r,
-                                         uint32_t maxm, int chain) {
-  s.r = r;
-  s.q = r;
-  s.nl = link[r];
-  s.v4p = sd.load4(r);
-  s.h16p = hash16(s.v4p);
-  s.maxm = maxm;
-  s.best = 2;
-  s.bd = 0;
-  s.pqr = 0;
-  s.steps = chain;
-  s.miss = 0;
-  s.bud = 2 * chain + 64;  // bounds the filtered candidates too
-}
-
-// One candidate; returns true once the search has ended.
-__device__ __forceinline__ bool lz_step(LzState& s, const SmemBytes& sd, const uint16_t* __restrict__ link, int nice,
-                                        int miss_limit) {
-  if (s.bud-- <= 0) return true;
-  const uint32_t l = s.nl;
-  if (!l) return true;
-  s.q -= l;
-  const uint32_t q = s.q, r = s.r;
-  if (r - q > 32767u) return true;
-  s.nl = link[q];
-  const uint32_t v = sd.load4(q);
-  if (v != s.v4p && hash16(v) != s.h16p) return false;  // same 15-bit bucket, other 16-bit chain
-  if (s.steps-- == 0) return true;
-  if (v != s.v4p) return ++s.miss >= miss_limit;
-  s.miss = 0;
-  // quick reject (src/deflate/lz77.cpp:137-142), on the 4 bytes ending at
-  // byte `best`: a longer match needs all of them
-  const uint32_t maxm = s.maxm, mb = s.best;
-  if (mb >= 4 && mb < maxm && sd.load4(q + mb - 3) != s.pqr) return false;
-  // the comparison from byte 4: aligned words on both sides, each loaded once
-  uint32_t len = 4;
-  {
-    const uint32_t pi = r + 4 + sd.boff, qi = q + 4 + sd.boff;
-    const uint32_t ps = (pi & 3) * 8, qs = (qi & 3) * 8;
-    const uint32_t* pw = sd.w + (pi >> 2);
-    const uint32_t* qw = sd.w + (qi >> 2);
-    uint32_t plo = pw[0], qlo = qw[0];
-    for (uint32_t k = 1; len < maxm; ++k) {
-      const uint32_t phi = pw[k], qhi = qw[k];
-      const uint32_t x = __funnelshift_r(plo, phi, ps) ^ __funnelshift_r(qlo, qhi, qs);
-      if (x) { len += (__ffs(x) - 1) >> 3; break; }
-      len += 4;
-      plo = phi;
-      qlo = qhi;
-    }
-  }
-  if (len > maxm) len = maxm;
-  if (len > s.best) {
-    s.best = len;
-    s.bd = r - q;
-    if (int(len) >= nice || len >= maxm) return true;
-    if (len >= 4) s.pqr = sd.load4(r + len - 3);
-  }
-  return false;
-}
-
-// First position >= i where a match starts (a set bit of fm), or tl.
-__device__ __forceinline__ uint32_t next_head(const uint32_t* fm, uint32_t i, uint32_t tl) {
-  if (i >= tl) return tl;
-  uint32_t w = i >> 5;
-  uint32_t bits = fm[w] & (kAll << (i & 31));
-  while (!bits && ++w < (tl + 31) / 32) bits = fm[w];
-  return bits ? min(w * 32 + __ffs(bits) - 1, tl) : tl;
-}
-
-// One step of the lazy parse from head i (F[i] != 0): up to `lazy` moves to
-// i + 1 while the match there is longer by two or more (the reference's lazy
-// rule, lz77.cpp:449-493; the match at i + 1 is the full search of i + 1,
-// where the reference searches again with half the chain).  Returns
-// {match position, len << 16 | dist}.
-__device__ __forceinline__ uint2 lazy_step(const uint32_t* F, uint32_t i, uint32_t tl, int lazy) {
-  uint32_t m = F[i];
-  int k = lazy;
-  while (k > 0 && i + (m >> 16) + 1 < tl && i + 4 <= tl) {
-    const uint32_t g = F[i + 1];
-    if ((g >> 16) > (m >> 16) + 1) {
-      ++i;
-      m = g;
-      --k;
-    } else {
-      break;
-    }
-  }
-  return make_uint2(i, m);
-}
-
-// Clears the bits of positions [lo, hi).
-__device__ __forceinline__ void clear_bits(uint32_t* bm, uint32_t lo, uint32_t hi) {
-  while (lo < hi) {
-    const uint32_t w = lo >> 5, b0 = lo & 31, n = min(32u - b0, hi - lo);
-    const uint32_t mask = (n == 32 ? kAll : ((1u << n) - 1)) << b0;
-    bm[w] &= ~mask;
-    lo += n;
-  }
-}
-
-__device__ __forceinline__ uint32_t block_max_excl(uint32_t v, uint32_t* scan) {
-  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(kAll, inc, o);
-    if (lane >= uint32_t(o)) inc = max(inc, t);
-  }
-  if (lane == 31) scan[wid] = inc;
-  __syncthreads();
-  if (wid == 0) {
-    uint32_t x = lane < (blockDim.x >> 5) ? scan[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(kAll, x, o);
-      if (lane >= uint32_t(o)) x = max(x, t);
-    }
-    scan[32 + lane] = x;  // inclusive over warps
-  }
-  __syncthreads();
-  const uint32_t before_warp = wid ? scan[32 + wid - 1] : 0;
-  const uint32_t excl_lane = __shfl_up_sync(kAll, inc, 1);
-  return max(before_warp, lane ? excl_lane : 0u);
-}
-
-__device__ __forceinline__ uint32_t len_sym(uint32_t len) {
-  uint32_t li, ne, ev;
-  length_code(len, li, ne, ev);
-  return li;
-}
-__device__ __forceinline__ uint32_t dist_sym(uint32_t d) {
-  uint32_t dc, ne, ev;
-  dist_code(d, dc, ne, ev);
-  return dc;
-}
-
-// Literal/length and distance histogram of a tile's tokens (all threads):
-// a block-wide max-scan of match ends marks the bytes matches cover, every
-// other byte is a literal.
-__device__ void tile_histogram(const uint32_t* tok_s, uint32_t tl, const SmemBytes& sd, uint32_t off, uint32_t* hist,
-                               uint32_t* scan) {
-  const uint32_t per = (T + blockDim.x - 1) / blockDim.x;
-  const uint32_t i0 = threadIdx.x * per;
-  uint32_t me = 0;
-  for (uint32_t j = 0; j < per; ++j) {
-    const uint32_t i = i0 + j;
-    const uint32_t tk = i < tl ? tok_s[i] : 0;
-    if (tk) me = max(me, i + ((tk >> 16) & 0x1FFu));
-  }
-  uint32_t run = block_max_excl(me, scan);
-  for (uint32_t j = 0; j < per; ++j) {
-    const uint32_t i = i0 + j;
-    if (i >= tl) break;
-    const uint32_t tk = tok_s[i];
-    if (tk) {
-      const uint32_t len = (tk >> 16) & 0x1FFu;
-      atomicAdd(&hist[257 + len_sym(len)], 1u);
-      atomicAdd(&hist[288 + dist_sym(tk & 0xFFFFu)], 1u);
-      run = max(run, i + len);
-    } else if (run <= i) {
-      atomicAdd(&hist[sd.byte(off + i)], 1u);
-    }
-  }
-  __syncthreads();
-}
-
-// Bit cost (1/16 bit) of a token with `count` in a histogram of `total`
-// symbols: log2(total / count), 1..15 bits; unseen symbols cost 2 bits more
-// than the rarest possible.
-__device__ __forceinline__ uint16_t sym_cost(uint32_t count, uint32_t total) {
-  const float b = count ? __log2f(float(total) / float(count)) : __log2f(float(total)) + 2.0f;
-  return uint16_t(16.0f * fminf(fmaxf(b, 1.0f), 15.0f) + 0.5f);
-}
-
 // -- staging by the bulk-copy engine (TMA, untiled; the source is this GPU's
-// own input arena, no multicast): one thread starts the copy of a tile's
-// window into shared memory and the CTA waits on an mbarrier for its bytes.
+// own memory, no multicast): one thread starts the copies and the CTA waits on
+// an mbarrier for their bytes.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -295,8 +86,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 // later bulk-copy writes (every thread that touched the staged bytes runs it
 // before the barrier that precedes the next copy).
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void bulk_stage(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_u32(dst)),
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
@@ -324,397 +117,867 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, uint64_
     if (global_ns() - t0 > limit_ns) return false;
   return true;
 }
-constexpr uint64_t kStageWaitNs = 1000000000ull;  // a copy of 37 KB that takes a second has failed
+constexpr uint64_t kStageWaitNs = 1000000000ull;  // a copy of at most 111 KB that takes a second has failed
+
+// Lanes of the warp whose low NB bits of `h` equal this lane's, among the
+// lanes of `among`: one ballot per bit, so the cost does not depend on how
+// many values differ (match.any serialises over them).
+template <int NB>
+__device__ __forceinline__ uint32_t same_bits(uint32_t h, uint32_t among) {
+  uint32_t m = among;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const bool on = (h >> b) & 1u;
+    const uint32_t bal = __ballot_sync(kAll, on);
+    m &= on ? bal : ~bal;
+  }
+  return m;
+}
 
 }  // namespace
 
-// ---------------------------------------------------------------- k_lz
-// One CTA per run of up to kLazyRun consecutive tiles of a segment.  The
-// links of the window and the hash table carry from one tile to the next
-// (shifted down by the tile length), so each position is linked once.
-__global__ void __launch_bounds__(1024, 1) k_lz(Work wk, const uint32_t* __restrict__ runs, uint32_t nruns) {
-  extern __shared__ __align__(16) uint8_t sm[];
-  uint32_t* sdata = reinterpret_cast<uint32_t*>(sm);
-  uint16_t* link = reinterpret_cast<uint16_t*>(sm + kDataBytes);
-  uint16_t* tbl = reinterpret_cast<uint16_t*>(sm + kDataBytes + kLinkBytes);
-  uint8_t* fgb = sm + kDataBytes + kLinkBytes + kTblBytes;
-  uint32_t* F = reinterpret_cast<uint32_t*>(fgb);
-  uint32_t* tok_s = reinterpret_cast<uint32_t*>(fgb + kFBytes);
-  uint32_t* fm = tok_s + T;
-  uint32_t* hist = fm + kFmWords;
-  uint32_t* scan = hist + 320;
-  uint16_t* choice = reinterpret_cast<uint16_t*>(scan + 64);  // optimal parse: token length at each position
-  uint16_t* scost = choice + T;                              // symbol costs, 1/16 bit: 0-255 literals, 257+ lengths, 288+ distances
-  uint16_t* lcost = scost + 320;                             // cost of a match length 0..258 (code + extra bits)
+// ---------------------------------------------------------------- k_link
+// link[x] for every position x of a segment: distance to the latest earlier
+// position with the same 15-bit hash (0: none within 32767 bytes), with bit 15
+// set when the 4 bytes there are the same too.  One CTA per run of
+// consecutive tiles: it first fills its last-position table from the 32 KiB
+// before the run (atomicMax, any order), then goes through the run 4,096
+// positions a round.  In a round every warp takes four chunks of 32
+// positions; links inside a chunk come from ballots over the hash bits, and
+// each hash's first and last position in the chunk become one entry.  The
+// entries are partitioned, in order, by the top five hash bits into 32 lists,
+// and warp b owns list b and its 1,024 table slots: so the ordered part
+// (table read, table write) is one warp's walk over 1/32 of the entries, and
+// all warps do it at once.
+//
+// This replaces the ordered pass of one warp over all chunks of a tile inside
+// the search kernel: 30% of that kernel on mixed data, with 31 warps idle.
+// Bound by instruction issue (the ballots) and four barriers per round.
+namespace {
+constexpr uint32_t kLkRound = 4096;             // positions per round: 128 chunks
+constexpr uint32_t kLkChunks = kLkRound / 32;
+constexpr uint32_t kLkRing = 65536;             // staged input, by arena address mod 64 KiB
+struct LinkSmem {
+  uint32_t ring[kLkRing / 4];
+  uint32_t tbl[32768];                          // last position + 1 of every hash (0: none)
+  uint32_t list[kLkRound];                      // first | last << 12, positions in the round
+  uint16_t cnt[32][kLkChunks];                  // entries per list and chunk, then their offsets
+  uint16_t out[kLkRound];
+  uint32_t tot[32];
+  uint64_t bar;
+};
+static_assert(sizeof(LinkSmem) <= 227 * 1024, "one CTA per SM");
+
+struct RingBytes {
+  const uint32_t* w;
+  uint32_t base;  // ring byte of position 0
+  __device__ __forceinline__ uint32_t load4(uint32_t x) const {
+    const uint32_t i = x + base;
+    return __funnelshift_r(w[(i >> 2) & (kLkRing / 4 - 1)], w[((i >> 2) + 1) & (kLkRing / 4 - 1)], (i & 3) * 8);
+  }
+};
+
+// Starts the copy of arena bytes [a, b) (multiples of 16, at most 64 KiB) to
+// their ring places.
+__device__ __forceinline__ void ring_stage(LinkSmem& S, const uint8_t* in, uint64_t a, uint64_t b) {
+  mbar_expect(&S.bar, uint32_t(b - a));
+  uint8_t* ring = reinterpret_cast<uint8_t*>(S.ring);
+  while (a < b) {
+    const uint32_t o = uint32_t(a) & (kLkRing - 1);
+    const uint32_t n = min(uint32_t(b - a), kLkRing - o);
+    bulk_copy(ring + o, in + a, n, &S.bar);
+    a += n;
+  }
+}
+}  // namespace
+
+__global__ void __launch_bounds__(1024, 1) k_link(Work wk, const uint32_t* __restrict__ runs, uint32_t nruns) {
+  extern __shared__ __align__(128) uint8_t link_sm[];
+  LinkSmem& S = *reinterpret_cast<LinkSmem*>(link_sm);
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-
   if (blockIdx.x >= nruns) return;
-  __shared__ __align__(8) uint64_t stage_bar;  // completion of the bulk copy of a tile's window
-  if (tid == 0) mbar_init(&stage_bar, 1);
+  const uint32_t first = runs[2 * blockIdx.x], count = runs[2 * blockIdx.x + 1];
+  const uint32_t seg = wk.tiles[first].seg;
+  const Segment sg = wk.segs[seg];
+  const uint32_t p0 = wk.tiles[first].start;
+  const uint32_t p1 = wk.tiles[first + count - 1].start + wk.tiles[first + count - 1].len;
+  const uint32_t hashed = sg.len >= 4 ? sg.len - 3 : 0;  // positions with 4 bytes
+  uint16_t* link = reinterpret_cast<uint16_t*>(wk.scratch + sg.links);
+  if (p0 >= p1) return;  // an empty segment's tile
+  if (tid == 0) mbar_init(&S.bar, 1);
+  for (uint32_t i = tid; i < 32768 / 4; i += 1024) reinterpret_cast<uint4*>(S.tbl)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  uint32_t stage_phase = 0;
-  const uint32_t first = runs[2 * blockIdx.x];
-  const uint32_t last = first + runs[2 * blockIdx.x + 1];
-  const Segment sg = wk.segs[wk.tiles[first].seg];
-  const LazyCfg cfg = c_lazy[sg.level];
-  uint32_t prev_rs = 0, prev_nreg = 0;
 
-  for (uint32_t ti = first; ti < last; ++ti) {
-    Tile* tp = wk.tiles + ti;
-    const Tile t = *tp;
-    const uint32_t ts = t.start, tl = t.len, tend = ts + tl;
-    const uint32_t rs = ts > W ? ts - W : 0;           // region start (segment-relative)
-    const uint32_t nreg = tend - rs;                    // positions with links
-    const uint32_t copy_end = min(sg.len, tend + 8);    // bytes staged
-    // -- stage bytes [rs, copy_end) at 16-byte granularity
-    const uint64_t g0 = (sg.in_off + rs) & ~uint64_t(15);
-    const uint32_t boff = uint32_t(sg.in_off + rs - g0);
-    const uint32_t n16 = (boff + (copy_end - rs) + 15) / 16;
-    // one thread starts the bulk copy; meanwhile the CTA clears the tail (the
-    // bytes past the copy that whole-word reads may touch) and slides the
-    // links and the table, which do not depend on the new bytes
-    uint4* dst = reinterpret_cast<uint4*>(sm);
-    if (tid == 0) bulk_stage(dst, wk.in + g0, n16 * 16, &stage_bar);
-    for (uint32_t i = n16 + tid; i < kDataBytes / 16; i += blockDim.x) dst[i] = make_uint4(0, 0, 0, 0);
-    for (uint32_t i = tid; i < 320; i += blockDim.x) hist[i] = 0;
-    // -- carry links and table from the previous tile, or start empty
-    uint32_t lstart = 0;
-    if (ti == first) {
-      for (uint32_t i = tid; i < kTblBytes / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(tbl)[i] = kAll;
-    } else {
-      const uint32_t shift = rs - prev_rs;  // even: tiles and the window are even
-      const uint32_t keep = prev_nreg - shift;
-      uint32_t* lw = reinterpret_cast<uint32_t*>(link);
-      constexpr uint32_t kMaxWords = (kRegion / 2 + 1023) / 1024;
-      uint32_t tmp[kMaxWords];
-#pragma unroll
-      for (uint32_t k = 0; k < kMaxWords; ++k) {
-        const uint32_t wi = tid + k * 1024;
-        tmp[k] = wi * 2 < keep ? lw[wi + shift / 2] : 0u;
-      }
-      __syncthreads();
-#pragma unroll
-      for (uint32_t k = 0; k < kMaxWords; ++k) {
-        const uint32_t wi = tid + k * 1024;
-        if (wi * 2 < keep) {
-          // a link that now points before the region start is dropped
-          uint32_t lo = tmp[k] & 0xFFFFu, hi = tmp[k] >> 16;
-          if (lo > wi * 2) lo = 0;
-          if (hi > wi * 2 + 1) hi = 0;
-          lw[wi] = lo | (hi << 16);
-        }
-      }
-      for (uint32_t i = tid; i < 32768; i += blockDim.x) {
-        const uint32_t e = tbl[i];
-        tbl[i] = (e != 0xFFFFu && e >= shift) ? uint16_t(e - shift) : uint16_t(0xFFFFu);
-      }
-      lstart = keep;
-    }
-    const bool staged = mbar_wait(&stage_bar, stage_phase, kStageWaitNs);
-    stage_phase ^= 1u;
+  // staged so far: arena bytes up to `have`; the first copy brings the bytes
+  // before the run and the first round's, each later one a round's
+  const uint32_t warm0 = p0 > kMaxDist ? p0 - kMaxDist : 0;
+  uint64_t have = (sg.in_off + warm0) & ~uint64_t(15);
+  auto stage_to = [&](uint32_t x) {  // bytes of positions below x, and the 8 after them
+    const uint64_t to = (sg.in_off + min(uint64_t(sg.len), uint64_t(x) + 8) + 15) & ~uint64_t(15);
+    if (tid == 0) ring_stage(S, wk.in, have, to);
+    have = to;
+  };
+  stage_to(min(p1, p0 + kLkRound));
+  uint32_t phase = 0;
+  const RingBytes rb{S.ring, uint32_t(sg.in_off) & (kLkRing - 1)};
+
+  for (uint32_t q0 = p0; q0 < p1; q0 += kLkRound) {
+    const bool staged = mbar_wait(&S.bar, phase, kStageWaitNs);
     if (!__syncthreads_and(staged)) {
       // the copy did not complete: mark the stream failed, give the copy
-      // another bounded wait so that no copy is left in flight, and stop
-      if (tid == 0) atomicOr(&wk.segs[t.seg].flags, kSegFault);
-      mbar_wait(&stage_bar, stage_phase ^ 1u, kStageWaitNs);
+      // another bounded wait so that none is left in flight, and stop
+      if (tid == 0) atomicOr(&wk.segs[seg].flags, kSegFault);
+      mbar_wait(&S.bar, phase, kStageWaitNs);
       return;
     }
-    const SmemBytes sd{sdata, boff};
-
-    // -- links of the new positions [lstart, nreg): the previous position
-    // with the same 15-bit hash.  (1) All warps, 32-position chunks: the
-    // nearest earlier lane with the same hash is the link inside the chunk;
-    // the first lane of every hash is marked and, until step (2), holds in
-    // its link the offset to the hash's last lane in the chunk.  (2) Warp 0,
-    // chunk after chunk: each first lane reads the table's position (its
-    // link) and writes its hash's last position in the chunk.  Only step (2)
-    // is sequential: one table read and write per distinct hash, by one lane,
-    // and one warp barrier per chunk (the next chunk's reads come after).
-    {
-      const uint32_t nch = (nreg - lstart + 31) / 32;
-      uint32_t* fbits = F;  // F is free until the searches
-      const uint32_t lt = (1u << lane) - 1;
-      for (uint32_t c = wid; c < nch; c += blockDim.x >> 5) {
-        const uint32_t x = lstart + c * 32 + lane;
-        const bool valid = x < nreg && rs + x + 4 <= sg.len;
-        const uint32_t h = valid ? hash15(sd.load4(x)) : 0x10000u + lane;  // invalid lanes match nobody
-        const uint32_t peers = __match_any_sync(kAll, h);
-        const uint32_t before = peers & lt;
-        const bool is_first = valid && !before;
-        if (x < nreg)
-          link[x] = before ? uint16_t(__clz(before) - (31 - lane))
-                           : is_first ? uint16_t((31 - __clz(peers)) - lane) : uint16_t(0);
-        const uint32_t first = __ballot_sync(kAll, is_first);
-        if (lane == 0) fbits[c] = first;
+    phase ^= 1u;
+    const uint32_t q1 = min(p1, q0 + kLkRound);
+    if (q0 == p0 && warm0 < p0) {
+      // the table at the start of the run; a position followed by one with
+      // the same hash needs no atomic (the later position wins anyway)
+      for (uint32_t x = warm0 + 4 * tid; x < min(p0, hashed); x += 4096) {
+        const uint32_t i = x + rb.base;
+        uint32_t wd[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) wd[j] = S.ring[((i >> 2) + j) & (kLkRing / 4 - 1)];
+        const uint32_t lo = __funnelshift_r(wd[0], wd[1], (i & 3) * 8), hi = __funnelshift_r(wd[1], wd[2], (i & 3) * 8);
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h[j] = hash15(__funnelshift_r(lo, hi, j * 8));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const bool in = x + j < min(p0, hashed), next_in = j < 3 && x + j + 1 < min(p0, hashed);
+          if (in && !(next_in && h[j] == h[j + 1])) atomicMax(&S.tbl[h[j]], x + j + 1);
+        }
       }
       __syncthreads();
-      if (wid == 0) {
-        // eight chunks per round: their marks, hashes and last positions are
-        // loaded first, then the table reads and writes go in chunk order
-        // without waiting for each other's results
-        constexpr uint32_t U = 8;
-        for (uint32_t c0 = 0; c0 < nch; c0 += U) {
-          uint32_t fb[U], h[U], p[U], lastp[U];
-#pragma unroll
-          for (uint32_t u = 0; u < U; ++u) fb[u] = c0 + u < nch ? (fbits[c0 + u] >> lane) & 1u : 0u;
-#pragma unroll
-          for (uint32_t u = 0; u < U; ++u) {
-            const uint32_t x = lstart + (c0 + u) * 32 + lane;
-            h[u] = fb[u] ? hash15(sd.load4(x)) : 0u;
-            lastp[u] = fb[u] ? x + link[x] : 0u;
-          }
-#pragma unroll
-          for (uint32_t u = 0; u < U; ++u) {
-            p[u] = 0xFFFFu;
-            if (fb[u]) {
-              p[u] = tbl[h[u]];
-              tbl[h[u]] = uint16_t(lastp[u]);
-            }
-            __syncwarp();
-          }
-#pragma unroll
-          for (uint32_t u = 0; u < U; ++u) {
-            const uint32_t x = lstart + (c0 + u) * 32 + lane;
-            if (fb[u]) link[x] = p[u] == 0xFFFFu ? uint16_t(0) : uint16_t(x - p[u]);
-          }
-        }
-      }
     }
-    if (tid == 0) scan[62] = 0;
+    // the next round's bytes; their ring places hold bytes more than 32 KiB
+    // behind this round, last read before the barrier above
+    if (q1 < p1) stage_to(min(p1, q1 + kLkRound));
+    reinterpret_cast<uint2*>(S.cnt)[tid] = make_uint2(0, 0);
     __syncthreads();
 
-    // -- searches at every tile position.  Warps take 32-position chunks; a
-    // lane whose chain has ended takes the next position of its warp's chunk
-    // at once, so lanes stay busy across chains of very different lengths.
-    {
-      const uint32_t nsearch = tl >= 4 ? tl - 3 : 0;
-      const uint32_t nch = (nsearch + 31) / 32;
-      for (uint32_t i = nsearch + tid; i < kFmWords * 32; i += blockDim.x) F[i] = 0;
-      const uint32_t lt = (1u << lane) - 1;
-      uint32_t pool = 0, avail = 0;  // warp-uniform: next position of the chunk, positions left
-      bool more = true;
-      uint32_t i = kAll;             // this lane's position
-      LzState st;
-      for (;;) {
-        uint32_t idle = __ballot_sync(kAll, i == kAll);
-        while (idle && (avail || more)) {
-          if (!avail) {
-            uint32_t c = 0;
-            if (lane == 0) c = atomicAdd(&scan[62], 1u);
-            c = __shfl_sync(kAll, c, 0);
-            if (c >= nch) {
-              more = false;
-              break;
-            }
-            pool = c * 32;
-            avail = min(32u, nsearch - pool);
-          }
-          const uint32_t take = min(uint32_t(__popc(idle)), avail);
-          if (i == kAll && __popc(idle & lt) < take) {
-            i = pool + __popc(idle & lt);
-            lz_begin(st, sd, link, ts - rs + i, min(258u, tl - i), cfg.chain);
-          }
-          pool += take;
-          avail -= take;
-          idle = __ballot_sync(kAll, i == kAll);
-        }
-        if (idle == kAll) break;
-        // a few chain steps per round: the warp re-balances (ballot, new
-        // positions for lanes whose chain ended) once per kStepsPerRound steps
-        if (i != kAll) {
-#pragma unroll 1
-          for (int k = 0; k < kStepsPerRound; ++k) {
-            if (lz_step(st, sd, link, cfg.nice, cfg.miss)) {
-              F[i] = st.best >= 3 ? (st.best << 16) | st.bd : 0u;
-              i = kAll;
-              break;
-            }
-          }
-        }
-      }
+    // -- links inside the chunks; one entry per distinct hash of a chunk
+    const uint32_t lt = (1u << lane) - 1;
+    uint32_t entry[4], where[4];  // entry: first | last << 12; where: list | rank << 8, or kAll
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t c = wid * 4 + j, o = c * 32 + lane, x = q0 + o;
+      const bool valid = x < q1 && x < hashed;
+      const uint32_t v = valid ? rb.load4(x) : 0u;
+      const uint32_t h = hash15(v);
+      const uint32_t in_list = same_bits<5>(h >> 10, __ballot_sync(kAll, valid));
+      const uint32_t peers = same_bits<10>(h, in_list);
+      const uint32_t before = valid ? peers & lt : 0u;
+      const uint32_t src = before ? 31 - __clz(before) : lane;
+      const uint32_t vs = __shfl_sync(kAll, v, src);
+      S.out[o] = before ? uint16_t((lane - src) | (vs == v ? 0u : kLinkDiff)) : uint16_t(kLinkDiff);
+      const bool is_first = valid && !before;
+      const uint32_t firsts = __ballot_sync(kAll, is_first) & in_list;
+      const uint32_t rank = __popc(firsts & lt);
+      if (is_first && rank == 0) S.cnt[h >> 10][c] = uint16_t(__popc(firsts));
+      entry[j] = o | ((c * 32 + 31 - __clz(peers | 1u)) << 12);
+      where[j] = is_first ? (h >> 10) | (rank << 8) : kAll;
     }
     __syncthreads();
-    for (uint32_t c = wid; c < kFmWords; c += blockDim.x >> 5) {
-      const uint32_t b = __ballot_sync(kAll, F[c * 32 + lane] != 0);
-      if (lane == 0) fm[c] = b;
-    }
-    for (uint32_t i = tid; i < T; i += blockDim.x) tok_s[i] = 0;
-    __syncthreads();
-
-    // -- parse (reference lazy rule, lz77.cpp:449-493, with n = tile end).
-    // A parse step depends only on its start position (the head), so the
-    // heads are found in parallel: (1) each lane of warp 0 parses one 1/32 of
-    // the tile from its start; (2) lane 0 follows the true parse into every
-    // segment until it meets a head of that segment's parse, after which the
-    // two are the same; (3) every thread emits the matches of its heads.
+    // -- offsets: warp b scans list b's counts over the chunks
     {
-      uint32_t* hd = hist;  // heads, a bit per position (hist is zero until the histogram)
-      uint32_t* sx = scan;  // where each segment's parse leaves it
-      const uint32_t S = (tl + 31) / 32;
-      uint32_t nf = 0;  // positions with a match: few -> one lane parses alone
-      if (wid == 0) {
-        for (uint32_t w = lane; w < kFmWords; w += 32) nf += __popc(fm[w]);
-        nf = __reduce_add_sync(kAll, nf);
+      uint2* row = reinterpret_cast<uint2*>(S.cnt[wid]) + lane;  // four chunks per lane
+      const uint2 r = *row;
+      const uint32_t a = r.x & 0xFFFFu, b = r.x >> 16, c = r.y & 0xFFFFu, d = r.y >> 16;
+      uint32_t incl = a + b + c + d;
+      const uint32_t sum = incl;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t t = __shfl_up_sync(kAll, incl, s);
+        if (lane >= uint32_t(s)) incl += t;
       }
-      if (wid == 0 && nf <= kSerialParse) {
-        if (lane == 0) {
-          uint32_t i = 0;
-          while ((i = next_head(fm, i, tl)) < tl) {
-            hd[i >> 5] |= 1u << (i & 31);
-            const uint2 m = lazy_step(F, i, tl, cfg.lazy);
-            i = (m.x & 0xFFFFu) + (m.y >> 16);
-          }
-        }
-      } else if (wid == 0) {
-        const uint32_t a = min(lane * S, tl), b = min(a + S, tl);
-        uint32_t i = a;
-        while (i < b) {
-          i = next_head(fm, i, tl);
-          if (i >= b) break;
-          atomicOr(&hd[i >> 5], 1u << (i & 31));
-          const uint2 m = lazy_step(F, i, tl, cfg.lazy);
-          i = (m.x & 0xFFFFu) + (m.y >> 16);
-        }
-        sx[lane] = i;
+      const uint32_t e = incl - sum;
+      *row = make_uint2(e | ((e + a) << 16), (e + a + b) | ((e + a + b + c) << 16));
+      if (lane == 31) S.tot[wid] = incl;
+    }
+    __syncthreads();
+    // -- scatter the entries to their lists
+    const uint32_t mytot = S.tot[lane];
+    uint32_t start = mytot;  // exclusive scan over the lists
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const uint32_t t = __shfl_up_sync(kAll, start, s);
+      if (lane >= uint32_t(s)) start += t;
+    }
+    start -= mytot;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t b = where[j] & 31u;
+      const uint32_t sb = __shfl_sync(kAll, start, b);
+      if (where[j] != kAll) S.list[sb + S.cnt[b][wid * 4 + j] + (where[j] >> 8)] = entry[j];
+    }
+    __syncthreads();
+    // -- warp b walks list b in order
+    {
+      const uint32_t l0 = __shfl_sync(kAll, start, wid), n = __shfl_sync(kAll, mytot, wid);
+      uint32_t* tb = S.tbl + (wid << 10);
+      for (uint32_t k = 0; k < n; k += 32) {
+        const bool valid = k + lane < n;
+        const uint32_t e = valid ? S.list[l0 + k + lane] : 0u;
+        const uint32_t x = q0 + (e & 0xFFFu), xl = q0 + (e >> 12);
+        const uint32_t v = rb.load4(x);
+        const uint32_t h = hash15(v) & 1023u;
+        const uint32_t peers = same_bits<10>(h, __ballot_sync(kAll, valid));
+        const uint32_t before = valid ? peers & lt : 0u;
+        const uint32_t pl = __shfl_sync(kAll, xl, before ? 31 - __clz(before) : lane);
+        uint32_t p = pl + 1;  // previous position + 1
+        if (valid && !before) p = tb[h];
         __syncwarp();
-        if (lane == 0) {
-          uint32_t e = sx[0];
-          for (uint32_t sgi = 1; sgi < 32; ++sgi) {
-            const uint32_t a2 = min(sgi * S, tl), b2 = min(a2 + S, tl);
-            if (a2 >= b2) break;
-            clear_bits(hd, a2, min(e, b2));
-            if (e >= b2) continue;
-            uint32_t i2 = e;
-            for (;;) {
-              const uint32_t h = next_head(fm, i2, tl);
-              if (h >= b2) {
-                e = h;
-                break;
-              }
-              if ((hd[h >> 5] >> (h & 31)) & 1u) {
-                e = sx[sgi];
-                break;
-              }
-              hd[h >> 5] |= 1u << (h & 31);
-              const uint2 m = lazy_step(F, h, tl, cfg.lazy);
-              i2 = (m.x & 0xFFFFu) + (m.y >> 16);
-              clear_bits(hd, h + 1, min(i2, b2));
-              if (i2 >= b2) {
-                e = i2;
-                break;
-              }
-            }
+        if (valid && (peers >> lane) == 1u) tb[h] = xl + 1;
+        __syncwarp();
+        if (valid && p && x + 1 - p <= kMaxDist)
+          S.out[e & 0xFFFu] = uint16_t((x + 1 - p) | (rb.load4(p - 1) == v ? 0u : kLinkDiff));
+      }
+    }
+    fence_proxy_async_smem();  // this round's reads of the ring, before a later copy into it
+    __syncthreads();
+    // -- write out; a warp writes the positions whose places it fills next round
+    {
+      const uint32_t o = wid * 128 + lane * 4;
+      const uint2 v = *reinterpret_cast<const uint2*>(S.out + o);
+      if (q0 + o + 4 <= q1) {
+        *reinterpret_cast<uint2*>(link + q0 + o) = v;
+      } else {
+        for (uint32_t i = 0; i < 4; ++i)
+          if (q0 + o + i < q1) link[q0 + o + i] = S.out[o + i];
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// ---------------------------------------------------------------- k_search
+// The longest match at every position, walking the chain newest first
+// with the reference's rules (src/deflate/lz77.cpp:66-156): candidates of the
+// same 15-bit bucket but another 16-bit hash are skipped, `chain` candidates
+// with the same 16-bit hash are examined, miss_limit consecutive 4-byte
+// mismatches end the walk, ties keep the nearest, nice length ends the walk.
+// Result: length << 16 | distance per position, 0 for no match.
+//
+// One CTA of 1024 threads searches up to 9 consecutive tiles: their bytes
+// and links and the 32 KiB before them (210 KB) come in two bulk copies.
+// A warp takes 32 positions at a time and, one per lane, compares each with
+// its first candidate; the positions that must go on are queued.  Chains differ
+// in length by a factor of hundreds, so a lane takes a position from the queue
+// as soon as its chain ends, and only at the end of the whole group do lanes
+// run out of positions.
+//
+// The walk is bound by instruction issue, so a step is one link and one byte:
+//   * while the links carry the same-bytes flag the candidate's 4 bytes are
+//     known equal and are not loaded;
+//   * a longer match must also agree at byte `best`, so one byte rejects most
+//     candidates; lanes whose byte agrees stop and are compared together.
+// When a match gets longer, the chain of the 4 bytes that end one past it is
+// followed a few links: any longer match has these bytes at its own distance,
+// so when that chain holds nothing farther than the current candidate the
+// search is over.  Neither changes a result: both only skip candidates that
+// cannot be longer than the best one.
+// Measured with k_link and k_lparse against one CTA per run that did all three
+// (B200, ms): 64 MiB mixed at level 6 in 128 KiB chunks 9.1 -> 3.9, 32 MiB text
+// at level 9 in 256 KiB chunks 18.7 -> 5.5, the same of 8-byte periods with 1%
+// flips 76 -> 15.3, 8 MiB mixed at level 12 9.7 -> 2.0.  Ten candidates per
+// round of the warp: 4 cost 25% more on text, 14 the same.
+namespace {
+constexpr uint32_t kMaxRegion = W + kSearchTiles * T;  // positions with links
+constexpr uint32_t kDataBytes = (kMaxRegion + 48 + 127) / 128 * 128;  // + alignment + over-read tail
+constexpr uint32_t kLinkBytes = (kMaxRegion * 2 + 127) / 128 * 128;
+constexpr uint32_t kSearchSmem = kDataBytes + kLinkBytes;
+constexpr int kSearchThreads = 1024;
+static_assert(kSearchSmem + kSearchThreads / 32 * 64 * 8 + 64 <= 227 * 1024, "one CTA per SM");
+constexpr int kStopped = 0x7FFFFFFF;
+constexpr int kWalkSteps = 10;    // candidates a lane takes before the warp compares and re-balances
+constexpr int kSlowSteps = 4;    // at most, of the candidates whose 4 bytes are compared
+constexpr int kTailHops = 4;     // links followed on the chain one past a new best match
+
+// Common-prefix length (at most maxm) of the bytes at r and at its candidate
+// c, whose first 4 bytes agree: aligned words on both sides, each loaded once.
+__device__ __forceinline__ uint32_t match_length(const SmemBytes& sd, uint32_t r, uint32_t c, uint32_t maxm) {
+  uint32_t len = 4;
+  const uint32_t pi = r + 4 + sd.boff, qi = c + 4 + sd.boff;
+  const uint32_t ps = (pi & 3) * 8, qs = (qi & 3) * 8;
+  const uint32_t* pw = sd.w + (pi >> 2);
+  const uint32_t* qw = sd.w + (qi >> 2);
+  uint32_t plo = pw[0], qlo = qw[0];
+#pragma unroll 1
+  while (len < maxm) {
+    const uint32_t phi = *++pw, qhi = *++qw;
+    const uint32_t x = __funnelshift_r(plo, phi, ps) ^ __funnelshift_r(qlo, qhi, qs);
+    if (x) { len += (__ffs(x) - 1) >> 3; break; }
+    len += 4;
+    plo = phi;
+    qlo = qhi;
+  }
+  return min(len, maxm);
+}
+
+// Whether r cannot have a match longer than `len` farther than distance bd:
+// such a match has the 4 bytes ending one past `len` at its own distance too,
+// so their chain (followed a few links) would hold a position there.
+__device__ __forceinline__ bool none_longer(const uint16_t* link, uint32_t r, uint32_t len, uint32_t bd) {
+  const int s = int(r + len - 3);
+  int u = s;
+#pragma unroll 1
+  for (int k = 0; k < kTailHops; ++k) {
+    const int d = int(link[u] & 0x7FFFu);
+    u -= d;
+    if (d == 0 || s - u > int(kMaxDist)) return true;
+    if (s - u > int(bd)) break;
+  }
+  return false;
+}
+}  // namespace
+
+__global__ void __launch_bounds__(kSearchThreads, 1) k_search(Work wk, const uint32_t* __restrict__ runs,
+                                                              uint32_t nruns) {
+  extern __shared__ __align__(128) uint8_t search_sm[];
+  const uint32_t* sdata = reinterpret_cast<const uint32_t*>(search_sm);
+  const uint16_t* link = reinterpret_cast<const uint16_t*>(search_sm + kDataBytes);
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t next_chunk;
+  __shared__ uint2 queue[kSearchThreads / 32][64];  // positions to walk: offset | length << 16, distance
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  if (blockIdx.x >= nruns) return;
+  const uint32_t first = runs[2 * blockIdx.x], count = runs[2 * blockIdx.x + 1];
+  const uint32_t seg = wk.tiles[first].seg;
+  const Segment sg = wk.segs[seg];
+  const LazyCfg cfg = c_lazy[sg.level];
+  const uint32_t ts = wk.tiles[first].start, tend = min(sg.len, ts + count * T), tl = tend - ts;
+  uint32_t* F = reinterpret_cast<uint32_t*>(wk.scratch + sg.toks) + ts;
+  const uint32_t rs = ts > W ? ts - W : 0;  // region start; a multiple of 16 positions
+  const uint64_t g0 = (sg.in_off + rs) & ~uint64_t(15);
+  const uint32_t boff = uint32_t(sg.in_off + rs - g0);
+  const uint32_t data16 = (boff + (min(sg.len, tend + 8) - rs) + 15) / 16;
+  const uint32_t link16 = ((tend - rs) * 2 + 15) / 16;
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    next_chunk = 0;
+    mbar_expect(&bar, (data16 + link16) * 16);
+    if (data16) bulk_copy(search_sm, wk.in + g0, data16 * 16, &bar);
+    if (link16) bulk_copy(search_sm + kDataBytes, wk.scratch + sg.links + uint64_t(rs) * 2, link16 * 16, &bar);
+  }
+  __syncthreads();
+  const bool staged = mbar_wait(&bar, 0, kStageWaitNs);
+  if (!__syncthreads_and(staged && !(sg.flags & kSegFault))) {
+    // as in k_link; the tiles are left without matches
+    if (!staged && tid == 0) atomicOr(&wk.segs[seg].flags, kSegFault);
+    mbar_wait(&bar, 0, kStageWaitNs);
+    for (uint32_t i = tid; i < tl; i += kSearchThreads) F[i] = 0;
+    return;
+  }
+  const SmemBytes sd{sdata, boff};
+  const uint8_t* bytes = search_sm + boff;
+  const uint32_t bytes_at = smem_u32(bytes), links_at = smem_u32(link);
+
+  const uint32_t nch = (tl + 31) / 32;
+  const uint32_t lt = (1u << lane) - 1;
+  uint2* wq = queue[tid >> 5];
+  uint32_t nq = 0;   // positions in the warp's queue
+  bool more = true;  // chunks left
+  uint32_t r = 0, maxm = 0, best = 0, bd = 0, pb = 0, l = 0;
+  int pos = 0, pmin = 0, lim = 0, slack = 0, miss = 0;
+  bool busy = false;
+  bool pure = true;  // the candidate at pos has r's 4 bytes
+  for (;;) {
+    const uint32_t idle = __ballot_sync(kAll, !busy);
+    // -- the warp's next chunks of 32 positions, one per lane: the first
+    // candidate, which is all many positions have; the others are queued
+    while (more && nq < uint32_t(__popc(idle))) {
+      uint32_t c = 0;
+      if (lane == 0) c = atomicAdd(&next_chunk, 1u);
+      c = __shfl_sync(kAll, c, 0);
+      if (c >= nch) {
+        more = false;
+        break;
+      }
+      const uint32_t i = c * 32 + lane, p = ts - rs + i;
+      const uint32_t end = min(tl, (c * 32 / T + 1) * T);  // a chunk lies in one tile
+      const uint32_t mx = i + 4 <= end ? min(258u, end - i) : 0u;
+      const uint32_t l1 = mx ? uint32_t(link[p]) : kLinkDiff;
+      uint32_t len = 3, dist = 0;
+      bool walk = l1 > kLinkDiff;  // other 4 bytes in the bucket: the walk sorts it out
+      if (l1 < kLinkDiff) {
+        len = match_length(sd, p, p - l1, mx);
+        dist = l1;
+        walk = int(len) < cfg.nice && len < mx && !none_longer(link, p, len, l1);
+      }
+      if (!walk && i < tl) F[i] = dist ? (len << 16) | dist : 0u;
+      const uint32_t m = __ballot_sync(kAll, walk);
+      if (walk) wq[nq + __popc(m & lt)] = make_uint2(i | (len << 16), dist);
+      nq += __popc(m);
+      __syncwarp();
+    }
+    const uint32_t take = min(uint32_t(__popc(idle)), nq);
+    if (!busy && uint32_t(__popc(idle & lt)) < take) {
+      const uint2 e = wq[nq - 1 - __popc(idle & lt)];
+      const uint32_t i = e.x & 0xFFFFu;
+      busy = true;
+      best = e.x >> 16;
+      bd = e.y;
+      r = ts - rs + i;
+      maxm = min(258u, min(tl, (i / T + 1) * T) - i);
+      pos = int(r - bd);
+      pmin = max(int(r) - int(kMaxDist), 0);
+      l = link[pos];
+      pb = bytes[r + best];
+      lim = cfg.chain - (bd ? 1 : 0);
+      slack = cfg.chain + 64;  // 2 * chain + 64 candidates, skipped ones included
+      miss = 0;
+      pure = true;
+    }
+    nq -= take;
+    __syncwarp();
+    if (idle == kAll && take == 0) break;
+    // -- candidates known to have the same 4 bytes: one link and one byte
+    // each, no branch.  `x` is the shared address of byte `best` of the
+    // candidate and `k2` turns it into its link's.  A flagged link is at least
+    // 32768 and so leads below `lo` like one out of the window; a lane that
+    // has stopped keeps x and loads the same link again.
+    bool hit, done;
+    {
+      const uint32_t to_x = bytes_at + best, k2 = links_at - 2 * to_x;
+      uint32_t x = uint32_t(pos) + to_x;
+      const bool run = busy && pure;
+      int lo = run ? pmin + int(to_x) : kStopped;
+#pragma unroll
+      for (int k = 0; k < kWalkSteps; ++k)
+        asm("{\n"
+            " .reg .pred p, q;\n .reg .s32 nx;\n .reg .u32 a, b;\n"
+            " sub.s32 nx, %0, %1;\n"
+            " setp.ge.s32 p, nx, %2;\n"
+            " setp.gt.and.s32 p, %3, 0, p;\n"
+            " @p mov.s32 %0, nx;\n"
+            " @p add.s32 %3, %3, -1;\n"
+            " mad.lo.u32 a, %0, 2, %4;\n"
+            " ld.shared.u16 %1, [a];\n"
+            " ld.shared.u8 b, [%0];\n"
+            " setp.eq.and.u32 q, b, %5, p;\n"
+            " @q mov.s32 %2, 0x7FFFFFFF;\n"
+            "}"
+            : "+r"(x), "+r"(l), "+r"(lo), "+r"(lim)
+            : "r"(k2), "r"(pb));
+      pos = int(x - to_x);
+      hit = run && lo == kStopped;
+    }
+    // -- the chain's end, or other 4 bytes in the same bucket
+    const int d1 = int(l & 0x7FFFu);
+    // (with no candidate left to count none can be taken, whatever comes)
+    done = busy && !hit && (d1 == 0 || pos - d1 < pmin || lim == 0);
+    bool slow = busy && !hit && !done && (!pure || l >= kLinkDiff);
+    if (__any_sync(kAll, slow)) {
+      const uint32_t v4p = sd.load4(r);
+#pragma unroll 1
+      for (int k = 0; k < kSlowSteps && slow; ++k) {
+        const int d = int(l & 0x7FFFu);
+        if (d == 0 || pos - d < pmin) { done = true; break; }
+        pos -= d;
+        l = link[pos];
+        const uint32_t v = sd.load4(uint32_t(pos));
+        pure = v == v4p;
+        if (!pure && hash16(v) != hash16(v4p)) {  // same 15-bit bucket, other 16-bit chain
+          if (slack) --slack;
+          else if (lim-- == 0) { done = true; break; }
+          continue;
+        }
+        if (lim-- == 0) { done = true; break; }
+        if (!pure) {
+          if (++miss >= cfg.miss) { done = true; break; }
+          continue;
+        }
+        miss = 0;
+        hit = bytes[pos + best] == pb;
+        slow = false;
+      }
+    }
+    // -- candidates that agree at byte `best`
+    if (hit && sd.load4(uint32_t(pos) + best - 3) == sd.load4(r + best - 3)) {
+      const uint32_t len = match_length(sd, r, uint32_t(pos), maxm);
+      if (len > best) {
+        best = len;
+        bd = r - uint32_t(pos);
+        done = int(len) >= cfg.nice || len >= maxm || none_longer(link, r, len, bd);
+        pb = bytes[r + len];
+      }
+    }
+    if (done) {
+      F[r - (ts - rs)] = bd ? (best << 16) | bd : 0u;
+      busy = false;
+    }
+  }
+}
+
+// ---------------------------------------------------------------- k_lparse
+// Parse of one tile per CTA from the matches k_search left in the tile's
+// token words, which the tokens replace (0x80000000 | length << 16 | distance
+// at a match's first position, 0 elsewhere), and its symbol histogram.
+//
+// Lazy parse (reference rule, lz77.cpp:449-493, with n = tile end): a parse
+// step depends only on its start position (the head), so the heads are found
+// in parallel: (1) each lane of warp 0 parses one 1/32 of the tile from its
+// start; (2) lane 0 follows the true parse into every part until it meets a
+// head of that part's parse, after which the two are the same; (3) the
+// threads emit the matches of the heads.  Tiles with few match positions are parsed by one lane.
+//
+// Optimal parse (levels 10-12): costs from the histogram of the lazy parse,
+// then a backward pass finds, for every position, the cheapest way to the
+// tile end (a literal, or the match found there shortened by up to 31 bytes),
+// then the path from position 0 is read.
+//
+// The chains of one warp are bound by latency, so they run apart from the
+// search, 16 and 14 tiles per SM at once, where the search CTA had one parsing
+// warp and 31 waiting ones; the other three warps of a CTA help to read the
+// matches, mark the tokens and fill the histogram.
+namespace {
+constexpr uint32_t kFmWords = T / 32;
+static_assert(T % 32 == 0, "tiles are whole windows of 32 positions");
+constexpr uint32_t kSerialParse = 128;  // at most this many match positions: serial parse
+struct ParseMem {
+  uint16_t len[T];         // match length found at each position (optimal: then the token length)
+  uint32_t fm[kFmWords];   // positions with a match
+  uint32_t hd[kFmWords];   // heads, then the first positions of the parse's matches
+  uint32_t em[kFmWords];
+  uint32_t hist[320];
+  uint32_t sx[32];         // where each part's parse leaves it
+};
+struct OptMem {
+  uint32_t cost[512];      // cost to the tile end, by position mod 512
+  uint32_t ring[128];      // prepared positions, by position mod 128
+  uint16_t scost[320];     // symbol costs, 1/16 bit: 0-255 literals, 257+ lengths, 288+ distances
+  uint16_t lcost[260];     // cost of a match length 0..258 (code + extra bits)
+};
+constexpr int kParseThreads = 128;
+template <bool Opt> struct ParseSmem { ParseMem p; };
+template <> struct ParseSmem<true> { ParseMem p; OptMem o; };
+
+// First position >= i where a match starts (a set bit of fm), or tl.
+__device__ __forceinline__ uint32_t next_head(const uint32_t* fm, uint32_t i, uint32_t tl) {
+  if (i >= tl) return tl;
+  uint32_t w = i >> 5;
+  uint32_t bits = fm[w] & (kAll << (i & 31));
+  while (!bits && ++w < (tl + 31) / 32) bits = fm[w];
+  return bits ? min(w * 32 + __ffs(bits) - 1, tl) : tl;
+}
+
+// One step of the lazy parse from head i (len[i] != 0): up to `lazy` moves to
+// i + 1 while the match there is longer by two or more (the reference's lazy
+// rule, lz77.cpp:449-493; the match at i + 1 is the full search of i + 1,
+// where the reference searches again with half the chain).  Returns the
+// match's position; its length is len there.
+__device__ __forceinline__ uint32_t lazy_step(const uint16_t* len, uint32_t i, uint32_t tl, int lazy) {
+  uint32_t m = len[i];
+  int k = lazy;
+  while (k > 0 && i + m + 1 < tl && i + 4 <= tl) {
+    const uint32_t g = len[i + 1];
+    if (g <= m + 1) break;
+    ++i;
+    m = g;
+    --k;
+  }
+  return i;
+}
+
+// Clears the bits of positions [lo, hi).
+__device__ __forceinline__ void clear_bits(uint32_t* bm, uint32_t lo, uint32_t hi) {
+  while (lo < hi) {
+    const uint32_t w = lo >> 5, b0 = lo & 31, n = min(32u - b0, hi - lo);
+    const uint32_t mask = (n == 32 ? kAll : ((1u << n) - 1)) << b0;
+    bm[w] &= ~mask;
+    lo += n;
+  }
+}
+
+__device__ __forceinline__ uint32_t len_sym(uint32_t len) {
+  uint32_t li, ne, ev;
+  length_code(len, li, ne, ev);
+  return li;
+}
+__device__ __forceinline__ uint32_t dist_sym(uint32_t d) {
+  uint32_t dc, ne, ev;
+  dist_code(d, dc, ne, ev);
+  return dc;
+}
+
+// Bit cost (1/16 bit) of a token with `count` in a histogram of `total`
+// symbols: log2(total / count), 1..15 bits; unseen symbols cost 2 bits more
+// than the rarest possible.
+__device__ __forceinline__ uint16_t sym_cost(uint32_t count, uint32_t total) {
+  const float b = count ? __log2f(float(total) / float(count)) : __log2f(float(total)) + 2.0f;
+  return uint16_t(16.0f * fminf(fmaxf(b, 1.0f), 15.0f) + 0.5f);
+}
+
+// Histogram of the tokens whose first positions are the bits of m.em (lengths
+// in m.len, distances in F's low halves); every byte no match covers is a
+// literal.  With `write`, F's words become the tokens.  The warps of the CTA
+// take a quarter of the windows each; all threads call it.
+__device__ void parse_tokens(ParseMem& m, uint32_t* F, uint32_t tl, const SegBytes& sb, uint32_t ts, bool write) {
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (uint32_t k = threadIdx.x; k < 320; k += kParseThreads) m.hist[k] = 0;
+  __syncthreads();
+  const uint32_t nwin = (tl + 31) / 32;
+  const uint32_t per = (nwin + kParseThreads / 32 - 1) / (kParseThreads / 32);
+  const uint32_t wa = min(nwin, wid * per), wb = min(nwin, wa + per);
+  uint32_t cover = 0;  // end of the last match before the window (a match reaches 8 windows on at most)
+  for (uint32_t w = wa; w > 0 && w + 9 > wa;) {
+    const uint32_t bits = m.em[--w];
+    if (bits) {
+      const uint32_t i = w * 32 + 31 - __clz(bits);
+      cover = i + m.len[i];
+      break;
+    }
+  }
+  constexpr uint32_t B = 8;  // windows whose loads are in flight together
+  for (uint32_t w0 = wa; w0 < wb; w0 += B) {
+    uint32_t v[B];  // the match at a token's position, the byte elsewhere
+#pragma unroll
+    for (uint32_t j = 0; j < B; ++j) {
+      const uint32_t w = w0 + j, i = w * 32 + lane;
+      const bool tok = w < wb && ((m.em[w] >> lane) & 1u);
+      v[j] = tok ? F[i] : w < wb && i < tl ? sb.byte(ts + i) : 0u;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < B; ++j) {
+      const uint32_t w = w0 + j, i = w * 32 + lane;
+      if (w >= wb) break;
+      const uint32_t bits = m.em[w];
+      const bool tok = (bits >> lane) & 1u;
+      const uint32_t len = tok ? m.len[i] : 0u;
+      // matches do not overlap, so the nearest one before a position decides
+      const uint32_t prior = bits & ((1u << lane) - 1);
+      const uint32_t pend = __shfl_sync(kAll, i + len, prior ? 31 - __clz(prior) : 0);
+      const uint32_t end = prior ? pend : cover;
+      if (tok) {
+        atomicAdd(&m.hist[257 + len_sym(len)], 1u);
+        atomicAdd(&m.hist[288 + dist_sym(v[j] & 0xFFFFu)], 1u);
+      } else if (i < tl && end <= i) {
+        atomicAdd(&m.hist[v[j]], 1u);
+      }
+      if (write && i < tl) F[i] = tok ? 0x80000000u | (len << 16) | (v[j] & 0xFFFFu) : 0u;
+      if (bits) cover = __shfl_sync(kAll, i + len, 31 - __clz(bits));
+    }
+  }
+  __syncthreads();
+}
+}  // namespace
+
+template <bool Opt>
+__global__ void __launch_bounds__(kParseThreads) k_lparse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  __shared__ ParseSmem<Opt> S;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (blockIdx.x >= nlist) return;
+  Tile* tp = wk.tiles + list[blockIdx.x];
+  const Tile t = *tp;
+  const Segment sg = wk.segs[t.seg];
+  const LazyCfg cfg = c_lazy[sg.level];
+  if ((cfg.opt != 0) != Opt) return;  // the other kernel's tile
+  ParseMem& m = S.p;
+  uint32_t* F = reinterpret_cast<uint32_t*>(wk.scratch + t.tok);
+  const uint32_t tl = t.len, ts = t.start;
+  const uint64_t o = sg.in_off;
+  const SegBytes sb{reinterpret_cast<const uint32_t*>(wk.in + (o & ~uint64_t(3))), uint32_t(o & 3)};
+
+  // -- lengths and the match bitmap, a warp's loads of eight windows in flight
+  constexpr uint32_t kWarps = kParseThreads / 32;
+  for (uint32_t w0 = 0; w0 < kFmWords; w0 += 8 * kWarps) {
+    uint32_t f[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+      const uint32_t i = (w0 + j * kWarps + wid) * 32 + lane;
+      f[j] = i < tl ? F[i] : 0u;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+      const uint32_t w = w0 + j * kWarps + wid;
+      const uint32_t b = __ballot_sync(kAll, f[j] != 0);
+      if (w < kFmWords) {
+        m.len[w * 32 + lane] = uint16_t(f[j] >> 16);
+        if (lane == 0) m.fm[w] = b;
+      }
+    }
+  }
+  for (uint32_t w = tid; w < kFmWords; w += kParseThreads) m.hd[w] = m.em[w] = 0;
+  __syncthreads();
+
+  // -- heads of the lazy parse
+  uint32_t nf = 0;  // positions with a match: few -> one lane parses alone
+  if (wid == 0) {
+    for (uint32_t w = lane; w < kFmWords; w += 32) nf += __popc(m.fm[w]);
+    nf = __reduce_add_sync(kAll, nf);
+  }
+  if (wid == 0 && nf <= kSerialParse) {
+    if (lane == 0) {
+      uint32_t i = 0;
+      while ((i = next_head(m.fm, i, tl)) < tl) {
+        m.hd[i >> 5] |= 1u << (i & 31);
+        i = lazy_step(m.len, i, tl, cfg.lazy);
+        i += m.len[i];
+      }
+    }
+  } else if (wid == 0) {
+    const uint32_t part = (tl + 31) / 32;
+    const uint32_t a = min(lane * part, tl), b = min(a + part, tl);
+    uint32_t i = a;
+    while (i < b) {
+      i = next_head(m.fm, i, tl);
+      if (i >= b) break;
+      atomicOr(&m.hd[i >> 5], 1u << (i & 31));
+      i = lazy_step(m.len, i, tl, cfg.lazy);
+      i += m.len[i];
+    }
+    m.sx[lane] = i;
+    __syncwarp();
+    if (lane == 0) {
+      uint32_t e = m.sx[0];
+      for (uint32_t k = 1; k < 32; ++k) {
+        const uint32_t a2 = min(k * part, tl), b2 = min(a2 + part, tl);
+        if (a2 >= b2) break;
+        clear_bits(m.hd, a2, min(e, b2));
+        if (e >= b2) continue;
+        uint32_t i2 = e;
+        for (;;) {
+          const uint32_t h = next_head(m.fm, i2, tl);
+          if (h >= b2) {
+            e = h;
+            break;
+          }
+          if ((m.hd[h >> 5] >> (h & 31)) & 1u) {
+            e = m.sx[k];
+            break;
+          }
+          m.hd[h >> 5] |= 1u << (h & 31);
+          i2 = lazy_step(m.len, h, tl, cfg.lazy);
+          i2 += m.len[i2];
+          clear_bits(m.hd, h + 1, min(i2, b2));
+          if (i2 >= b2) {
+            e = i2;
+            break;
           }
         }
       }
-      __syncthreads();
-      for (uint32_t i = tid; i < tl; i += blockDim.x) {
-        if ((hd[i >> 5] >> (i & 31)) & 1u) {
-          const uint2 m = lazy_step(F, i, tl, cfg.lazy);
-          tok_s[m.x & 0xFFFFu] = 0x80000000u | m.y;
-        }
-      }
-      __syncthreads();
-      if (wid == 0) {
-        uint32_t nm = 0;
-        for (uint32_t w = lane; w < kFmWords; w += 32) {
-          nm += __popc(hd[w]);
-          hd[w] = 0;
-        }
-        nm = __reduce_add_sync(kAll, nm);
-        if (lane == 0) scan[63] = nm;
-      }
     }
-    __syncthreads();
+  }
+  __syncthreads();
+  // -- the matches of the heads
+  for (uint32_t w = tid; w < kFmWords; w += kParseThreads) {
+    uint32_t bits = m.hd[w];
+    while (bits) {
+      const uint32_t i = lazy_step(m.len, w * 32 + __ffs(bits) - 1, tl, cfg.lazy);
+      bits &= bits - 1;
+      atomicOr(&m.em[i >> 5], 1u << (i & 31));
+    }
+  }
+  __syncthreads();
 
-    // -- levels 10-12: optimal parse.  Costs come from the histogram of the
-    // lazy parse above; a backward pass finds, for every position, the
-    // cheapest way to the tile end (a literal, or the match found there
-    // shortened by up to 31 bytes), then the path from position 0 is read.
-    if (cfg.opt) {
-      tile_histogram(tok_s, tl, sd, ts - rs, hist, scan);
+  if constexpr (Opt) {
+    OptMem& c = S.o;
+    parse_tokens(m, F, tl, sb, ts, false);
+    if (wid == 0) {
       {
-        uint32_t lt = 1, dt = 0;  // totals (EOB counts once)
-        for (uint32_t k = 0; k < 286; ++k) lt += hist[k];
-        for (uint32_t k = 288; k < 318; ++k) dt += hist[k];
-        for (uint32_t k = tid; k < 320; k += blockDim.x)
-          scost[k] = k < 288 ? sym_cost(hist[k], lt) : sym_cost(hist[k], dt > 0 ? dt : 1);
+        uint32_t ltot = 0, dtot = 0;
+        for (uint32_t k = lane; k < 286; k += 32) ltot += m.hist[k];
+        for (uint32_t k = 288 + lane; k < 318; k += 32) dtot += m.hist[k];
+        ltot = __reduce_add_sync(kAll, ltot) + 1;  // EOB counts once
+        dtot = __reduce_add_sync(kAll, dtot);
+        for (uint32_t k = lane; k < 320; k += 32)
+          c.scost[k] = k < 288 ? sym_cost(m.hist[k], ltot) : sym_cost(m.hist[k], dtot > 0 ? dtot : 1);
       }
-      __syncthreads();
-      for (uint32_t k = tid; k < 320; k += blockDim.x) hist[k] = 0;
-      for (uint32_t k = tid; k < 259; k += blockDim.x) {
-        uint32_t li = 0, lne = 0, lev;
-        if (k >= 3) length_code(k, li, lne, lev);
-        lcost[k] = k >= 3 ? uint16_t(scost[257 + li] + 16 * lne) : uint16_t(0);
+      __syncwarp();
+      for (uint32_t k = lane; k < 259; k += 32) {
+        uint32_t ls = 0, lne = 0, lev;
+        if (k >= 3) length_code(k, ls, lne, lev);
+        c.lcost[k] = k >= 3 ? uint16_t(c.scost[257 + ls] + 16 * lne) : uint16_t(0);
       }
-      // per position, before the backward pass: cost[i] = literal cost,
-      // choice[i] = cost of the distance of the match found at i
-      uint32_t* cost = tok_s;  // cost to the tile end, per position (tokens are rebuilt below)
-      for (uint32_t i = tid; i < tl; i += blockDim.x) {
-        cost[i] = scost[sd.byte(ts - rs + i)];
+      for (uint32_t k = lane; k < 512; k += 32) c.cost[k] = 0;  // positions past the tile end cost nothing
+      for (uint32_t k = lane; k < 128; k += 32) c.ring[k] = 0;  // positions before the tile (a last group of one or two)
+      __syncwarp();
+      // Positions are prepared a window at a time, one per lane: match length |
+      // literal cost << 9 | distance cost << 17, in a ring of four windows; the
+      // loads of the window after next are in flight meanwhile.
+      uint32_t fpre = 0, bpre = 0;
+      auto fetch = [&](int w) {
+        const uint32_t j = uint32_t(w) * 32 + lane;
+        const bool in = w >= 0 && j < tl;
+        fpre = in ? F[j] : 0u;
+        bpre = in ? sb.byte(ts + j) : 0u;
+      };
+      auto prepare = [&](int w) {
         uint32_t dc = 0, dne = 0, dev;
-        if (F[i]) dist_code(F[i] & 0xFFFFu, dc, dne, dev);
-        choice[i] = F[i] ? uint16_t(scost[288 + dc] + 16 * dne) : uint16_t(0);
-      }
-      __syncthreads();
-      if (wid == 0) {
-        uint32_t next = 0;  // cost[i + 1]
-        for (int i = int(tl) - 1; i >= 0; --i) {
-          const uint32_t f = F[i];
-          uint32_t best = ((cost[i] + next) << 9) | 1u;
-          if (f) {
-            const uint32_t flen = f >> 16, dcost = choice[i];
-            const uint32_t L = flen - lane;
-            uint32_t key = kAll;
-            if (lane + 3 <= flen) key = ((lcost[L] + dcost + (i + L < tl ? cost[i + L] : 0u)) << 9) | L;
-            best = __reduce_min_sync(kAll, lane == 0 ? min(key, best) : key);
-          }
-          next = best >> 9;
-          __syncwarp();
-          if (lane == 0) {
-            cost[i] = next;
-            choice[i] = uint16_t(best & 511u);
-          }
+        if (fpre) dist_code(fpre & 0xFFFFu, dc, dne, dev);
+        const uint32_t dcost = fpre ? c.scost[288 + dc] + 16 * dne : 0u;
+        c.ring[(uint32_t(w) * 32 + lane) & 127] = (fpre >> 16) | (uint32_t(c.scost[bpre]) << 9) | (dcost << 17);
+      };
+      // cost << 9 | length of this lane's way to shorten the match of position i
+      auto match_key = [&](int i, uint32_t e) {
+        const uint32_t flen = e & 511u, L = flen - lane;
+        return lane + 3 <= flen ? ((c.lcost[L] + (e >> 17) + c.cost[(uint32_t(i) + L) & 511]) << 9) | L : kAll;
+      };
+      int pw = int(tl + 31) / 32;  // windows from here on are prepared
+      fetch(pw - 1);
+      uint32_t next = 0;  // cost of the position after the current one
+      // Three positions at a time: a match is at least 3 long, so the matches of
+      // all three lead past the first and their minima do not wait for each
+      // other; only the literals go from one position to the next.
+      for (int i = int(tl) - 1; i >= 0; i -= 3) {
+        while (pw > 0 && pw > (i >> 5) - 1) {
+          prepare(--pw);
+          fetch(pw - 1);
           __syncwarp();
         }
+        const uint32_t e0 = c.ring[i & 127], e1 = c.ring[(i - 1) & 127], e2 = c.ring[(i - 2) & 127];
+        uint32_t m0 = kAll, m1 = kAll, m2 = kAll;
+        if ((e0 | e1 | e2) & 511u) {
+          m0 = __reduce_min_sync(kAll, match_key(i, e0));
+          m1 = __reduce_min_sync(kAll, match_key(i - 1, e1));
+          m2 = __reduce_min_sync(kAll, match_key(i - 2, e2));
+        }
+        const uint32_t b0 = min(m0, ((((e0 >> 9) & 255u) + next) << 9) | 1u);
+        const uint32_t b1 = min(m1, ((((e1 >> 9) & 255u) + (b0 >> 9)) << 9) | 1u);
+        const uint32_t b2 = min(m2, ((((e2 >> 9) & 255u) + (b1 >> 9)) << 9) | 1u);
+        next = b2 >> 9;
+        const uint32_t v = lane == 0 ? b0 : lane == 1 ? b1 : b2;
+        if (lane < 3 && i >= int(lane)) {
+          c.cost[(uint32_t(i) - lane) & 511] = v >> 9;
+          m.len[uint32_t(i) - lane] = uint16_t(v & 511u);
+        }
+        __syncwarp();
       }
-      __syncthreads();
-      for (uint32_t i = tid; i < T; i += blockDim.x) tok_s[i] = 0;
-      __syncthreads();
-      if (tid == 0) {
-        uint32_t i = 0, nm = 0;
+      for (uint32_t w = lane; w < kFmWords; w += 32) m.em[w] = 0;
+      __syncwarp();
+      if (lane == 0) {
+        uint32_t i = 0, word = 0, bits = 0;  // the bits of the word being filled
         while (i < tl) {
-          const uint32_t c = choice[i];
-          if (c >= 3) {
-            tok_s[i] = 0x80000000u | (c << 16) | (F[i] & 0xFFFFu);
-            ++nm;
-            i += c;
-          } else {
-            ++i;
+          const uint32_t n = m.len[i];
+          if ((i >> 5) != word) {
+            m.em[word] = bits;
+            word = i >> 5;
+            bits = 0;
           }
+          bits |= (n >= 3 ? 1u : 0u) << (i & 31);
+          i += n;
         }
-        scan[63] = nm;
+        m.em[word] = bits;
       }
-      __syncthreads();
     }
-
-    // -- covered bytes (max-scan of match ends) and the histogram
-    const uint32_t nm = scan[63];
     __syncthreads();
-    tile_histogram(tok_s, tl, sd, ts - rs, hist, scan);
-    uint32_t* gh = reinterpret_cast<uint32_t*>(wk.scratch + t.hist);
-    for (uint32_t i = tid; i < 320; i += blockDim.x) gh[i] = hist[i];
-    uint32_t* gt = reinterpret_cast<uint32_t*>(wk.scratch + t.tok);
-    for (uint32_t i = tid; i < tl; i += blockDim.x) gt[i] = tok_s[i];
-    if (tid == 0) {
+  }
+
+  parse_tokens(m, F, tl, sb, ts, true);
+  uint32_t* gh = reinterpret_cast<uint32_t*>(wk.scratch + t.hist);
+  for (uint32_t i = tid; i < 320; i += kParseThreads) gh[i] = m.hist[i];
+  if (wid == 0) {
+    uint32_t nm = 0;
+    for (uint32_t w = lane; w < kFmWords; w += 32) nm += __popc(m.em[w]);
+    nm = __reduce_add_sync(kAll, nm);
+    if (lane == 0) {
       tp->fin_matches = nm;
       tp->fix_bits = 0;
       tp->splice_bit = 0;
     }
-    prev_rs = rs;
-    prev_nreg = nreg;
-    fence_proxy_async_smem();  // this tile's reads and writes of the staged bytes, before the next copy
-    __syncthreads();
   }
 }
 
@@ -1082,10 +1345,15 @@ int launch_lazy(const Work& wk, const LazyLists& L, cudaStream_t st, int sms, Ma
   static std::atomic<bool> attr_set[64];
   const int ds = device_slot();
   if (!attr_set[ds].load(std::memory_order_relaxed)) {
-    if (cudaFuncSetAttribute(k_lz, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLz)) == cudaSuccess)
+    constexpr auto kMaxSmem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (cudaFuncSetAttribute(k_link, kMaxSmem, int(sizeof(LinkSmem))) == cudaSuccess &&
+        cudaFuncSetAttribute(k_search, kMaxSmem, int(kSearchSmem)) == cudaSuccess)
       attr_set[ds].store(true, std::memory_order_relaxed);
   }
-  k_lz<<<L.n_runs, 1024, kSmemLz, st>>>(wk, L.runs, L.n_runs);
+  k_link<<<L.n_runs, 1024, sizeof(LinkSmem), st>>>(wk, L.runs, L.n_runs);
+  k_search<<<L.n_groups, kSearchThreads, kSearchSmem, st>>>(wk, L.groups, L.n_groups);
+  if (L.any_lazy) k_lparse<false><<<L.n_tiles, kParseThreads, 0, st>>>(wk, L.tiles, L.n_tiles);
+  if (L.any_opt) k_lparse<true><<<L.n_tiles, kParseThreads, 0, st>>>(wk, L.tiles, L.n_tiles);
   mk->mark(kPhLazyLz, st);
   k_huff<<<(L.n_segs + kHuffWarps - 1) / kHuffWarps, kHuffWarps * 32, 0, st>>>(wk, L.segs, L.n_segs);
   mk->mark(kPhLazyHuff, st);
@@ -1094,7 +1362,7 @@ int launch_lazy(const Work& wk, const LazyLists& L, cudaStream_t st, int sms, Ma
   if (blocks > need) blocks = need;
   k_enc<<<blocks, kEncWarps * 32, 0, st>>>(wk, L.tiles, L.n_tiles, L.counter);
   mk->mark(kPhLazyEnc, st);
-  return 3;
+  return 4 + (L.any_lazy ? 1 : 0) + (L.any_opt ? 1 : 0);
 }
 
 }  // namespace orotb
