@@ -296,7 +296,7 @@ bool Engine::plan(const std::vector<Job>& jobs) {
           tiles.push_back(tl);
         }
       } else if (lv >= 4) {
-        // independent 4 KiB tiles, each with its own token words and histogram
+        // independent 4 KiB tiles
         const uint32_t LT = kLazyTile;
         const uint32_t nt = len ? uint32_t((len + LT - 1) / LT) : 1;
         g.tile_count = nt;
@@ -322,11 +322,11 @@ bool Engine::plan(const std::vector<Job>& jobs) {
           tl.scratch = bits_at;
           bits_at += lazy_stream_bytes(tl.len);
           tl.tok = g.toks + uint64_t(tl.start) * 4;
-          tl.hist = scratch;
-          scratch += 320 * 4;
           lists[kLazyTiles].push_back(uint32_t(tiles.size()));
           tiles.push_back(tl);
         }
+        g.hist = scratch;
+        scratch += 320 * 4;
         g.codes = scratch;
         scratch += 320 * 4;
         g.hdr_off = scratch;
@@ -483,7 +483,6 @@ bool Engine::launch(cudaStream_t st) {
     L.n_tiles = uint32_t(lists[kLazyTiles].size());
     L.segs = list(kLazySegs);
     L.n_segs = uint32_t(lists[kLazySegs].size());
-    L.counter = counters + 2;
     L.any_lazy = any_lazy;
     L.any_opt = any_opt;
     launches += launch_lazy(w, L, st, sms, &marks);

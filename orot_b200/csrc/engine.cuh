@@ -68,6 +68,7 @@ struct Segment {
   uint32_t eob;        // EOB code | (code length << 16)
   uint64_t links;      // scratch byte offset of the links (u16 per position, 16-byte aligned)
   uint64_t toks;       // scratch byte offset of the token words (u32 per position)
+  uint64_t hist;       // scratch byte offset of the literal/length + distance histogram (320 bins)
   // filled by the planner kernel
   uint32_t block_type;
   uint32_t piece_off;  // first copy slot of this block, from the stream's piece_first
@@ -98,7 +99,6 @@ struct Tile {
   uint64_t cand;       // levels 1-3, index > 0: u16 per position, candidate distance
                        // that passed the first-byte check (0 = literal)
   uint64_t tok;        // levels 4+: token word per position (0 = not a match start)
-  uint64_t hist;       // levels 4+: 320-bin literal/length + distance histogram
   // speculative walk (entry = tile start)
   uint32_t spec_bits, spec_matches, spec_exit, spec_tokens;
   // resolved parse: piece A = fix-up bits [0, fix_bits) from the fix-up

@@ -53,7 +53,6 @@ struct LazyLists {
   uint32_t n_tiles;
   const uint32_t* segs;      // segments needing Huffman tables
   uint32_t n_segs;
-  uint32_t* counter;
   bool any_lazy, any_opt;    // tiles of levels 4-9 / 10-12 among them
 };
 

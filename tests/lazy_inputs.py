@@ -39,6 +39,16 @@ def two_chains(n: int, seed: int) -> bytes:
     return bytes(out[:n])
 
 
+def fibonacci(symbols: int) -> bytes:
+    """Shuffled bytes whose counts are the Fibonacci numbers: the deepest tree."""
+    counts = [1, 1]
+    while len(counts) < symbols:
+        counts.append(counts[-1] + counts[-2])
+    body = bytearray(b"".join(bytes([i * 7 & 255]) * c for i, c in enumerate(counts)))
+    random.Random(symbols).shuffle(body)
+    return bytes(body)
+
+
 def cases():
     """(name, data) in a fixed order; data is deterministic."""
     for kind in range(6):
@@ -48,6 +58,10 @@ def cases():
     for name, make in (("collide", colliding_words), ("chains", two_chains)):
         for n in (TILE + 5, 120001):
             yield f"{name}:{n}", make(n, n)
+    for n in (18, 22, 25):  # code lengths beyond 15 bits without a limit
+        yield f"fibonacci:{n}", fibonacci(n)
+    yield "every byte once", bytes(range(256))
+    yield "every byte, few often", bytes(range(256)) + bytes(random.Random(2).choices(b"abcd", k=30000))
     text = synth.gen(50000, synth.TEXT, 5)
     yield "text+zeros+text", text + bytes(40000) + text
     yield "rare tail", b"".join(bytes([i & 255, 1, 2, 3, 4, 5, 6, i >> 8]) for i in range(9000))
