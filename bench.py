@@ -468,8 +468,8 @@ def measure_serving(deflate, buf, total, count, rate, cap_count, seed=0):
 # kernel (the "candidates" phase is empty then).
 WARP_INST_PER_BYTE = {"candidates": 3.65, "parse": 12.07, "lazy_match": 77.4}
 PHASE_KERNEL = {"candidates": "k_cand", "parse": "k_cand_parse",  "lazy_match": "k_search", "lazy_encode": "k_enc", "lazy_huffman": "k_huff",
-                "hash_carry": "k_lastocc + k_carry_scan", "fixup": "k_fix1 + k_fix2", "join": "k_join",
-                "checksum": "k_ck_block + k_ck_fold", "plan": "k_plan + k_zero"}
+                "hash_carry": "k_lastocc + k_carry_scan", "fixup": "k_fix1 + k_fix2 + k_fix3", "join": "k_join",
+                "checksum": "k_ck_block + k_ck_fold", "plan": "k_plan"}
 
 
 def roofline_of(phases, nbytes, comp, sm_mhz, sms):

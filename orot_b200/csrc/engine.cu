@@ -269,7 +269,19 @@ bool Engine::plan(const std::vector<Job>& jobs) {
         const uint32_t nt = len ? uint32_t((len + T - 1) / T) : 1;
         g.tile_count = nt;
         const uint32_t seg_index = uint32_t(segs.size());
-        if (nt > 1) lists[hb == 12 ? kMulti12 : kMulti14].push_back(seg_index);
+        if (nt > 1) {
+          lists[hb == 12 ? kMulti12 : kMulti14].push_back(seg_index);
+          const uint32_t nc = (nt - 1 + kCarryChunk - 1) / kCarryChunk;  // of the tiles that publish a table
+          for (uint32_t c = 0; c < nc; ++c) {
+            lists[hb == 12 ? kChunk12 : kChunk14].push_back(seg_index);
+            lists[hb == 12 ? kChunk12 : kChunk14].push_back(c);
+          }
+          if (nc > 1) {
+            lists[hb == 12 ? kChunked12 : kChunked14].push_back(seg_index);
+            g.chunks = scratch;
+            scratch += uint64_t(nc) * H * 4;
+          }
+        }
         for (uint32_t t = 0; t < nt; ++t) {
           Tile tl{};
           tl.seg = seg_index;
@@ -285,7 +297,12 @@ bool Engine::plan(const std::vector<Job>& jobs) {
           scratch += align_up(uint64_t((tl.len + 31) / 32) * sizeof(WinRec), 256);
           tl.cand = scratch;
           scratch += align_up(uint64_t(tl.len) * 2 + 64, 256);
-          if (t > 0) tl.carry = tiles.back().slot;
+          tl.prefix = kNoTable;
+          if (t > 0) {
+            tl.carry = tiles.back().slot;
+            const uint32_t c = (t - 1) / kCarryChunk;
+            if (c > 0) tl.prefix = g.chunks + uint64_t(c) * H * 4;
+          }
           if (t + 1 < nt) {
             tl.slot = scratch;
             scratch += uint64_t(H) * 4;
@@ -334,7 +351,7 @@ bool Engine::plan(const std::vector<Job>& jobs) {
       }
       const uint32_t stored_pieces = std::max<uint32_t>(1, uint32_t((len + 65534) / 65535));
       g.piece_off = npieces - s.piece_first;
-      npieces += 1 + 2 * g.tile_count + 2 + 3 * stored_pieces;
+      npieces += seg_piece_slots(g.tile_count, stored_pieces);
       segs.push_back(g);
     }
     s.seg_count = uint32_t(segs.size()) - s.seg_first;
@@ -462,15 +479,21 @@ bool Engine::launch(cudaStream_t st) {
     L.n_lastocc = uint32_t(lists[g ? kLast14 : kLast12].size());
     L.multi = list(g ? kMulti14 : kMulti12);
     L.n_multi = uint32_t(lists[g ? kMulti14 : kMulti12].size());
+    L.chunks = list(g ? kChunk14 : kChunk12);
+    L.n_chunks = uint32_t(lists[g ? kChunk14 : kChunk12].size() / 2);
+    L.chunked = list(g ? kChunked14 : kChunked12);
+    L.n_chunked = uint32_t(lists[g ? kChunked14 : kChunked12].size());
     L.walk = list(g ? kWalk14 : kWalk12);
     L.n_walk = uint32_t(lists[g ? kWalk14 : kWalk12].size());
-    L.counter = counters + g;  // candidates: 0/1; fix-up round 1: 4/5 (+ 4); parse: 6/7 (+ 6); abort: 12/13 (+ 12)
+    // candidates: 0/1; fix-up rounds 1 and 3: 4/5 (+ 4), 8/9 (+ 8); parse: 6/7 (+ 6); abort: 12/13 (+ 12)
+    L.counter = counters + g;
     L.ready = reinterpret_cast<uint32_t*>(t + off_ready) + (g ? lists[kWalk12].size() : 0);
     if (L.n_walk) {
       launch_fast(w, L, hbs[g], st, sms, &marks);
-      // k_lastocc; k_carry_scan, k_fix1, k_fix2 for multi-tile segments;
-      // k_cand_parse (or k_cand and k_parse)
-      launches += (L.n_lastocc ? 1 : 0) + (L.n_multi ? 3 : 0) + (fast_launches_fused() ? 1 : 2);
+      // k_lastocc; k_carry_scan, k_fix1, k_fix2, k_fix3 for multi-tile
+      // segments, k_carry_prefix for those of several chunks; k_cand_parse (or
+      // k_cand and k_parse)
+      launches += (L.n_lastocc ? 1 : 0) + (L.n_multi ? 4 : 0) + (L.n_chunked ? 1 : 0) + (fast_launches_fused() ? 1 : 2);
     }
   }
   if (!lists[kLazyTiles].empty()) {
@@ -489,20 +512,18 @@ bool Engine::launch(cudaStream_t st) {
   }
   launch_plan(w, max_out_cap, st);
   marks.mark(kPhPlan, st);
-  launches += 4;  // k_plan_seg, k_plan_stream, k_plan_pieces, k_zero
+  launches += 3;  // k_plan_seg, k_plan_stream, k_plan_pieces
   launch_join(w, counters + 3, st, sms);
   marks.mark(kPhJoin, st);
   launches += w.npieces ? 1 : 0;
   bool framed = false;
   for (const Stream& s : streams) framed |= s.fmt != kFmtRaw;
   if (framed) {
-    launch_checksums(w, st);
+    launch_checksums(w, true, st);
     launches += (w.nck ? 1 : 0) + 1;
   }
   marks.mark(kPhCheck, st);
-  launch_frame(w, st);
-  marks.mark(kPhFrame, st);
-  launches += 1;
+  marks.mark(kPhFrame, st);  // (headers and trailers are written by k_ck_fold)
   CK(cudaGetLastError());
   return true;
 }

@@ -25,6 +25,11 @@ constexpr uint32_t kSegLast = 1u;        // BFINAL block of its stream
 constexpr uint32_t kSegWholeBuf = 2u;    // whole-buffer rule: all-literal parse -> stored
 constexpr uint32_t kSegFault = 8u;       // set by a kernel that could not finish the segment (its stream fails)
 
+constexpr uint64_t kNoTable = ~uint64_t(0);
+constexpr uint32_t kNoEntry = ~0u;         // Tile::fix_entry of a tile the fix-up has not parsed yet
+constexpr uint32_t kCarryChunk = 32;       // tiles of a segment whose hash tables are scanned by themselves
+constexpr uint32_t kStoredSplit = 16;      // copies a stored piece of at most 65535 bytes is cut into
+
 // Stream error codes written to Stream::error.
 constexpr uint32_t kErrNone = 0, kErrCapacity = 1, kErrInternal = 2;
 
@@ -69,6 +74,7 @@ struct Segment {
   uint64_t links;      // scratch byte offset of the links (u16 per position, 16-byte aligned)
   uint64_t toks;       // scratch byte offset of the token words (u32 per position)
   uint64_t hist;       // scratch byte offset of the literal/length + distance histogram (320 bins)
+  uint64_t chunks;     // levels 1-3: scratch byte offset of the hash tables of its chunks of kCarryChunk tiles
   // filled by the planner kernel
   uint32_t block_type;
   uint32_t piece_off;  // first copy slot of this block, from the stream's piece_first
@@ -94,7 +100,9 @@ struct Tile {
   uint32_t index;      // index within the segment
   uint64_t scratch;    // byte offset of this tile's bit buffers in the scratch arena
   uint64_t rec;        // byte offset of WinRec[] (tiles with index > 0)
-  uint64_t carry;      // byte offset of the carried-in hash table (index > 0)
+  uint64_t carry;      // byte offset of the carried-in hash table (index > 0): the chunk's tiles up to
+                       // the one before; tiles of earlier chunks are in `prefix`
+  uint64_t prefix;     // byte offset of the table of all earlier chunks, or kNoTable
   uint64_t slot;       // byte offset of this tile's published table (index < count-1)
   uint64_t cand;       // levels 1-3, index > 0: u16 per position, candidate distance
                        // that passed the first-byte check (0 = literal)
@@ -105,7 +113,7 @@ struct Tile {
   // buffer, piece B = speculative bits [splice_bit, spec_bits)
   uint32_t fix_bits, splice_bit, fin_matches, fin_exit;
   uint32_t fix_entry;  // parse entry the fix-up assumed
-  uint32_t pad1;
+  uint32_t run;        // 1: a parse from any entry is matches of 258 bytes up to the next tile
 };
 
 // A bit-range copy for the join kernel.  src == nullptr means "write the
@@ -118,6 +126,13 @@ struct Piece {
   uint32_t nbits;
   uint32_t value;
 };
+
+// Copy slots of a segment: one coded block (header, code table, two per tile,
+// end of block) or its stored pieces (header, length and kStoredSplit copies each).
+__host__ __device__ inline uint32_t seg_piece_slots(uint32_t tiles, uint32_t stored_pieces) {
+  const uint32_t coded = 3 + 2 * tiles, stored = (2 + kStoredSplit) * stored_pieces;
+  return coded > stored ? coded : stored;
+}
 
 // Checksum block: a range of one stream's input.
 struct CkBlock {

@@ -53,8 +53,8 @@ struct Job {
 };
 
 enum ListId {
-  kLast12, kMulti12, kWalk12,
-  kLast14, kMulti14, kWalk14,
+  kLast12, kMulti12, kChunk12, kChunked12, kWalk12,
+  kLast14, kMulti14, kChunk14, kChunked14, kWalk14,
   kLazyTiles, kLazySegs, kLazyRuns, kLazyGroups,
   kNumLists
 };

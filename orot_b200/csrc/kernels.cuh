@@ -37,6 +37,10 @@ struct FastLists {
   uint32_t n_lastocc;
   const uint32_t* multi;     // segments with more than one tile
   uint32_t n_multi;
+  const uint32_t* chunks;    // (segment, chunk) of every chunk of kCarryChunk tiles of theirs
+  uint32_t n_chunks;
+  const uint32_t* chunked;   // segments of more than one chunk
+  uint32_t n_chunked;
   const uint32_t* walk;      // tiles to walk
   uint32_t n_walk;
   uint32_t* counter;         // zeroed work counters
@@ -76,12 +80,12 @@ void launch_fast(const Work& wk, const FastLists& L, int hash_bits, cudaStream_t
 bool fast_launches_fused();
 int launch_lazy(const Work& wk, const LazyLists& L, cudaStream_t st, int sms, Marks* mk);
 void launch_plan(const Work& wk, uint64_t max_out, cudaStream_t st);  // max_out: largest stream bound
-void launch_checksums(const Work& wk, cudaStream_t st);
+// Checksums of every stream; `frame`: and its header and trailer (after launch_join).
+void launch_checksums(const Work& wk, bool frame, cudaStream_t st);
 void launch_ck_single(const CkBlock* ck, uint32_t nck, uint64_t total, uint32_t init, int adler, uint32_t* res,
                       const Work& wk, cudaStream_t st);
 CrcPowers host_crc_powers();
 void launch_join(const Work& wk, uint32_t* counter, cudaStream_t st, int sms);
-void launch_frame(const Work& wk, cudaStream_t st);
 bool upload_crc_tables();  // once per device; false on a device error
 
 // One DEFLATE stream to decode (raw data, framing stripped by the host).

@@ -6,15 +6,14 @@
 //               block, and the list of bit-range copies that assemble the
 //               stream; output size and capacity check (one warp per segment
 //               or stream, see below).
-//   k_zero      clears the words the streams will occupy.
 //   k_ck_block  CRC-32 (slicing-by-4) and Adler-32 partial sums of 64 KiB
 //               blocks, 256 bytes per thread, folded with the GF(2) shift /
 //               Adler weight identities.
 //   k_ck_fold   folds the blocks of each stream: runs of blocks per thread,
-//               then a tree over the runs (one CTA per stream).
+//               then a tree over the runs (one CTA per stream); writes the zlib
+//               / gzip header and trailer bytes.
 //   k_join      one warp per copy: funnel-shifted 32-bit words, plain stores
 //               inside a copy, atomicOr on the two boundary words it shares.
-//   k_frame     zlib / gzip header and trailer bytes.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <mutex>
@@ -43,7 +42,8 @@ __host__ __device__ inline uint32_t fmt_trailer_bytes(uint32_t fmt) { return fmt
 //                  capacity check, the closing sync point of an open part.
 //   k_plan_pieces  one warp per segment: its bit-range copies, at slots the
 //                  host reserved for the segment (Segment::piece_off); unused
-//                  slots are left empty (nbits 0).
+//                  slots are left empty (nbits 0).  More CTAs clear the words
+//                  the streams will occupy.
 
 // Bits a stored block of `len` bytes starting at bit c occupies: per piece of
 // at most 65535 bytes, 3 header bits, padding to a byte, LEN/NLEN and the
@@ -51,11 +51,6 @@ __host__ __device__ inline uint32_t fmt_trailer_bytes(uint32_t fmt) { return fmt
 __device__ __forceinline__ uint64_t stored_bits_at(uint64_t c, uint32_t len) {
   const uint64_t pieces = len ? (uint64_t(len) + 65534) / 65535 : 1;
   return (((c + 3 + 7) & ~uint64_t(7)) - c) + 32 + uint64_t(len) * 8 + (pieces - 1) * 40;
-}
-
-__device__ __forceinline__ uint32_t seg_piece_slots(const Segment& sg) {
-  const uint32_t stored_pieces = max(1u, (sg.len + 65534u) / 65535u);
-  return 1 + 2 * sg.tile_count + 2 + 3 * stored_pieces;
 }
 
 __global__ void k_plan_seg(Work wk) {
@@ -148,7 +143,25 @@ __global__ void k_plan_stream(Work wk) {
   wk.streams[si] = s;
 }
 
-__global__ void k_plan_pieces(Work wk) {
+// Clears the words stream si will occupy (the join ORs boundary words), part
+// `part` of `parts`, so that one large stream is cleared by many CTAs.
+__device__ __forceinline__ void clear_output(const Work& wk, uint32_t si, uint32_t part, uint32_t parts) {
+  const Stream& s = wk.streams[si];
+  if (s.error) return;
+  uint4* o = reinterpret_cast<uint4*>(wk.out + s.out_off);
+  const uint64_t n16 = (s.out_size + 15) / 16;
+  const uint64_t per = (n16 + parts - 1) / parts;
+  const uint64_t b = per * part, e = min(n16, b + per);
+  for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) o[i] = make_uint4(0, 0, 0, 0);
+}
+
+// The CTAs after those of the segments clear the streams' words.
+__global__ void k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
+  if (blockIdx.x >= seg_ctas) {
+    const uint32_t x = blockIdx.x - seg_ctas;
+    clear_output(wk, x / parts, x % parts, parts);
+    return;
+  }
   const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (g >= wk.nsegs) return;
   const Segment sg = wk.segs[g];
@@ -157,7 +170,7 @@ __global__ void k_plan_pieces(Work wk) {
   const uint32_t hdr = bare ? 0 : fmt_header_bytes(s.fmt);
   uint32_t* dst = reinterpret_cast<uint32_t*>(wk.out + s.out_off);
   Piece* pc = wk.pieces + s.piece_first + sg.piece_off;
-  const uint32_t slots = seg_piece_slots(sg);
+  const uint32_t slots = seg_piece_slots(sg.tile_count, max(1u, (sg.len + 65534u) / 65535u));
   const uint64_t c = uint64_t(hdr) * 8 + sg.bit_off;  // block start in the output slot
   const bool last = (sg.flags & kSegLast) != 0;
   for (uint32_t i = lane; i < slots; i += 32) pc[i].nbits = 0;
@@ -166,16 +179,27 @@ __global__ void k_plan_pieces(Work wk) {
   if (sg.block_type == kBlkStored) {
     const uint32_t P = max(1u, (sg.len + 65534u) / 65535u);
     const uint64_t c1 = ((c + 3 + 7) & ~uint64_t(7)) + 32 + 8ull * 65535;  // start of piece 1 (when P > 1)
-    for (uint32_t i = lane; i < P; i += 32) {
+    // per stored piece its header, its length and kStoredSplit copies of 4 KiB
+    // at most: one warp copies a Piece
+    constexpr uint32_t kPer = 2 + kStoredSplit;
+    for (uint32_t x = lane; x < P * kPer; x += 32) {
+      const uint32_t i = x / kPer, k = x % kPer;
       const uint64_t ci = i == 0 ? c : c1 + uint64_t(i - 1) * (40 + 8ull * 65535);
       const uint32_t off = i * 65535u, n = min(sg.len - off, 65535u);
       const bool fin = last && off + n == sg.len;
       const uint64_t lenpos = (ci + 3 + 7) & ~uint64_t(7);
-      const uint64_t a = sg.in_off + off;
-      pc[3 * i] = Piece{nullptr, dst, 0, ci, 3, fin ? 1u : 0u};
-      pc[3 * i + 1] = Piece{nullptr, dst, 0, lenpos, 32, n | ((~n & 0xFFFFu) << 16)};
-      pc[3 * i + 2] = Piece{reinterpret_cast<const uint32_t*>(wk.in + (a & ~uint64_t(3))), dst, (a & 3) * 8,
-                            lenpos + 32, n * 8, 0};
+      if (k == 0) {
+        pc[x] = Piece{nullptr, dst, 0, ci, 3, fin ? 1u : 0u};
+      } else if (k == 1) {
+        pc[x] = Piece{nullptr, dst, 0, lenpos, 32, n | ((~n & 0xFFFFu) << 16)};
+      } else {
+        constexpr uint32_t kPart = 65536 / kStoredSplit;
+        const uint32_t o = (k - 2) * kPart;
+        if (o >= n) continue;
+        const uint64_t a = sg.in_off + off + o;
+        pc[x] = Piece{reinterpret_cast<const uint32_t*>(wk.in + (a & ~uint64_t(3))), dst, (a & 3) * 8,
+                      lenpos + 32 + 8ull * o, min(kPart, n - o) * 8, 0};
+      }
     }
     return;
   }
@@ -219,22 +243,6 @@ __global__ void k_plan_pieces(Work wk) {
     const uint32_t eob = sg.eob;  // dynamic EOB: code | (len << 16)
     pc[2 + 2 * sg.tile_count] = Piece{nullptr, dst, 0, at, eob >> 16, eob & 0xFFFFu};
   }
-}
-
-// ---------------------------------------------------------------- k_zero
-// Clears the words every stream will occupy (the join ORs boundary words):
-// blockIdx.y splits a stream into gridDim.y parts, so one large stream is
-// cleared by many CTAs.
-__global__ void k_zero(Work wk) {
-  const uint32_t si = blockIdx.x;
-  if (si >= wk.nstreams) return;
-  const Stream s = wk.streams[si];
-  if (s.error) return;
-  uint4* o = reinterpret_cast<uint4*>(wk.out + s.out_off);
-  const uint64_t n16 = (s.out_size + 15) / 16;
-  const uint64_t per = (n16 + gridDim.y - 1) / gridDim.y;
-  const uint64_t b = per * blockIdx.y, e = min(n16, b + per);
-  for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) o[i] = make_uint4(0, 0, 0, 0);
 }
 
 // ---------------------------------------------------------------- checksums
@@ -374,8 +382,32 @@ __device__ CkPartial fold_blocks(const CkBlock* blk, uint32_t n, uint32_t what, 
   return sh[0];
 }
 
-// One CTA per stream.
-__global__ void __launch_bounds__(kFoldThreads) k_ck_fold(Work wk, CrcPowers pw) {
+// zlib / gzip header and trailer bytes of a stream (one thread).
+__device__ void write_frame(const Work& wk, const Stream& s, uint32_t check) {
+  if (s.error || (s.mode & kStreamBare)) return;
+  uint8_t* o = wk.out + s.out_off;
+  const uint64_t end = s.out_size;
+  if (s.fmt == kFmtZlib) {
+    // header 78 9C (zlib_wrapper.cpp:21-22), Adler-32 big-endian trailer
+    o[0] = 0x78; o[1] = 0x9C;
+    for (int i = 0; i < 4; ++i) o[end - 4 + i] = uint8_t(check >> (24 - 8 * i));
+  } else {
+    // 1F 8B 08 00 mtime=0 XFL OS=FF (gzip_wrapper.cpp:31-43); the parallel
+    // path always writes XFL 0 (parallel_compressor.cpp:96-98)
+    const uint8_t xfl = s.parallel ? 0 : (s.level >= 9 ? 2 : (s.level <= 2 ? 4 : 0));
+    const uint8_t h[10] = {0x1F, 0x8B, 8, 0, 0, 0, 0, 0, xfl, 0xFF};
+    for (int i = 0; i < 10; ++i) o[i] = h[i];
+    const uint32_t isz = uint32_t(s.in_len);
+    for (int i = 0; i < 4; ++i) {
+      o[end - 8 + i] = uint8_t(check >> (8 * i));
+      o[end - 4 + i] = uint8_t(isz >> (8 * i));
+    }
+  }
+}
+
+// One CTA per stream; with `frame` the stream's output (joined before) gets its
+// header and trailer.
+__global__ void __launch_bounds__(kFoldThreads) k_ck_fold(Work wk, CrcPowers pw, bool frame) {
   __shared__ CkPartial sh[kFoldThreads];
   const uint32_t si = blockIdx.x;
   if (si >= wk.nstreams) return;
@@ -394,6 +426,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_ck_fold(Work wk, CrcPowers pw)
     check = uint32_t(s2 << 16) | uint32_t(s1);
   }
   wk.streams[si].checksum = check;
+  if (frame) write_frame(wk, s, check);
 }
 
 // Single-stream checksum with an arbitrary initial value (deflate_crc32 /
@@ -438,48 +471,39 @@ __global__ void __launch_bounds__(256) k_join(Work wk, uint32_t* counter) {
     const uint64_t d0 = pc.dst_bit, d1 = pc.dst_bit + pc.nbits;
     const uint64_t w0 = d0 >> 5, w1 = (d1 - 1) >> 5;
     const int64_t delta = int64_t(pc.src_bit) - int64_t(d0);
-    for (uint64_t w = w0 + lane; w <= w1; w += 32) {
-      const int64_t sbit = int64_t(w) * 32 + delta;
-      const int64_t sw = sbit >> 5;  // floor
-      const uint32_t sh = uint32_t(sbit & 31);
-      const uint32_t lo = sw >= 0 ? __ldg(pc.src + sw) : 0u;
-      const uint32_t hi = __ldg(pc.src + sw + 1);
-      const uint32_t v = __funnelshift_r(lo, hi, sh);
-      const uint64_t x0 = w * 32;
+    // source word of destination word w0 (floor) and the shift; both sides
+    // advance word by word
+    const int64_t s0 = int64_t(w0) * 32 + delta;
+    const uint32_t* src = pc.src + (s0 >> 5);
+    const uint32_t sh = uint32_t(s0 & 31);
+    const uint32_t nw = uint32_t(w1 - w0);  // the last word
+    uint32_t* dw = dst + w0;
+    // the words inside, four per lane in flight
+    uint32_t k = lane == 0 ? 32u : lane;  // word 0 and word nw may be shared with other copies
+    for (; k + 96 < nw; k += 128) {
+      uint32_t lo[4], hi[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        lo[u] = __ldg(src + k + 32 * u);
+        hi[u] = __ldg(src + k + 32 * u + 1);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dw[k + 32 * u] = __funnelshift_r(lo[u], hi[u], sh);
+    }
+    for (; k < nw; k += 32) dw[k] = __funnelshift_r(__ldg(src + k), __ldg(src + k + 1), sh);
+    if (lane == 0 || (lane == 1 && nw)) {
+      const uint32_t e = lane ? nw : 0u;
+      const uint64_t x0 = (w0 + e) * 32;
       const uint32_t lb = uint32_t((d0 > x0 ? d0 : x0) - x0);
       const uint32_t hb = uint32_t((d1 < x0 + 32 ? d1 : x0 + 32) - x0);
+      const uint32_t lo = (s0 >> 5) + int64_t(e) >= 0 ? __ldg(src + e) : 0u;
+      const uint32_t v = __funnelshift_r(lo, __ldg(src + e + 1), sh);
       if (lb == 0 && hb == 32) {
-        dst[w] = v;
+        dw[e] = v;
       } else {
         const uint32_t m = (hb - lb == 32) ? kFullMask : (((1u << (hb - lb)) - 1) << lb);
-        atomicOr(dst + w, v & m);
+        atomicOr(dw + e, v & m);
       }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- k_frame
-__global__ void k_frame(Work wk) {
-  const uint32_t si = blockIdx.x * blockDim.x + threadIdx.x;
-  if (si >= wk.nstreams) return;
-  const Stream s = wk.streams[si];
-  if (s.error || s.fmt == kFmtRaw || (s.mode & kStreamBare)) return;
-  uint8_t* o = wk.out + s.out_off;
-  const uint64_t end = s.out_size;
-  if (s.fmt == kFmtZlib) {
-    // header 78 9C (zlib_wrapper.cpp:21-22), Adler-32 big-endian trailer
-    o[0] = 0x78; o[1] = 0x9C;
-    for (int i = 0; i < 4; ++i) o[end - 4 + i] = uint8_t(s.checksum >> (24 - 8 * i));
-  } else {
-    // 1F 8B 08 00 mtime=0 XFL OS=FF (gzip_wrapper.cpp:31-43); the parallel
-    // path always writes XFL 0 (parallel_compressor.cpp:96-98)
-    const uint8_t xfl = s.parallel ? 0 : (s.level >= 9 ? 2 : (s.level <= 2 ? 4 : 0));
-    const uint8_t h[10] = {0x1F, 0x8B, 8, 0, 0, 0, 0, 0, xfl, 0xFF};
-    for (int i = 0; i < 10; ++i) o[i] = h[i];
-    const uint32_t isz = uint32_t(s.in_len);
-    for (int i = 0; i < 4; ++i) {
-      o[end - 8 + i] = uint8_t(s.checksum >> (8 * i));
-      o[end - 4 + i] = uint8_t(isz >> (8 * i));
     }
   }
 }
@@ -528,16 +552,16 @@ void launch_plan(const Work& wk, uint64_t max_out, cudaStream_t st) {
   if (!wk.nstreams) return;
   if (wk.nsegs) k_plan_seg<<<(wk.nsegs + 7) / 8, 256, 0, st>>>(wk);
   k_plan_stream<<<(wk.nstreams + 7) / 8, 256, 0, st>>>(wk);
-  if (wk.nsegs) k_plan_pieces<<<(wk.nsegs + 7) / 8, 256, 0, st>>>(wk);
   // about 1 MiB of output per clearing CTA for the largest stream
   const uint32_t parts = uint32_t(std::min<uint64_t>(256, std::max<uint64_t>(1, max_out >> 20)));
-  k_zero<<<dim3(wk.nstreams, parts), 256, 0, st>>>(wk);
+  const uint32_t seg_ctas = (wk.nsegs + 7) / 8;
+  k_plan_pieces<<<seg_ctas + wk.nstreams * parts, 256, 0, st>>>(wk, seg_ctas, parts);
 }
 
-void launch_checksums(const Work& wk, cudaStream_t st) {
+void launch_checksums(const Work& wk, bool frame, cudaStream_t st) {
   const CrcPowers pw = host_crc_powers();
   if (wk.nck) k_ck_block<<<wk.nck, 256, 0, st>>>(wk, pw);
-  if (wk.nstreams) k_ck_fold<<<wk.nstreams, kFoldThreads, 0, st>>>(wk, pw);
+  if (wk.nstreams) k_ck_fold<<<wk.nstreams, kFoldThreads, 0, st>>>(wk, pw, frame);
 }
 
 void launch_ck_single(const CkBlock* ck, uint32_t nck, uint64_t total, uint32_t init, int adler, uint32_t* res,
@@ -553,11 +577,6 @@ void launch_join(const Work& wk, uint32_t* counter, cudaStream_t st, int sms) {
   const uint32_t need = (wk.npieces + 7) / 8;
   if (blocks > need) blocks = need;
   k_join<<<blocks, 256, 0, st>>>(wk, counter);
-}
-
-void launch_frame(const Work& wk, cudaStream_t st) {
-  if (!wk.nstreams) return;
-  k_frame<<<(wk.nstreams + 127) / 128, 128, 0, st>>>(wk);
 }
 
 }  // namespace orotb

@@ -146,7 +146,7 @@ deflate_result gzip_members_decompress(Engine& e, const uint8_t* in, size_t n, u
   w.nstreams = uint32_t(k);
   w.ck = d_ck;
   w.nck = uint32_t(ck.size());
-  launch_checksums(w, s);
+  launch_checksums(w, false, s);
   if (cudaMemcpyAsync(jobs.data(), d_jobs, k * sizeof(InflateJob), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaMemcpyAsync(st.data(), d_st, k * sizeof(Stream), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
