@@ -189,10 +189,25 @@ static const GeometryRow& geometry_row(uint64_t total_bytes, int sms) {
 
 const GeometryRow& Engine::geometry(uint64_t total_bytes) const { return geometry_row(total_bytes, sms); }
 
+// Passes of a few MiB are bound by the time one warp needs for a tile (about
+// 50 us for 1 KiB, two kernels of 16 or 28 parsers and 16 or 4 walkers per SM),
+// so they are cut finer than the table's smallest tile, down to 512 bytes
+// (shorter tiles cannot be crossed as parts of a long run, see run_tile):
+// about 1,024 tiles or more at 12 hash bits and 512 at 14, whose tables are four
+// times as large.  Mean over five kinds of data (us), 512 / 1024 / 2048 / 4096:
+//   12 bits:  4 KiB  86 / 102 / 140 / 194   512 KiB 181 / 185 / 224 / 312
+//             2 MiB 386 / 261 / 261 / 340     4 MiB 706 / 426 / 316 / 362
+//   14 bits: 32 KiB 133 / 146 / 183 / 259   512 KiB 276 / 209 / 232 / 319
+//             1 MiB 560 / 316 / 262 / 331     2 MiB 1002 / 599 / 368 / 362
 uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
   if (tile_override) return tile_override;
   const GeometryRow& g = geometry(total_bytes);
-  return hash_bits <= 12 ? g.tile12 : g.tile14;
+  const uint32_t most = hash_bits <= 12 ? g.tile12 : g.tile14;
+  const uint64_t scaled = total_bytes * 148u / uint64_t(std::max(sms, 1));
+  const uint64_t tiles = hash_bits <= 12 ? 2048 : 768;
+  uint32_t t = 512;
+  while (t < most && t * tiles <= scaled) t *= 2;
+  return t;
 }
 
 template <class T>
@@ -203,23 +218,41 @@ static uint64_t put_table(std::vector<uint8_t>& buf, const std::vector<T>& v) {
   return off;
 }
 
-// Tiles per search group: one CTA per SM searches a group, so the pass takes
-// (waves of groups) x (tiles per group, plus what staging a group and the
-// last long chains of its lanes cost, about a tile's time).
-uint32_t Engine::search_group() const {
-  if (lazy_run_override) return std::min(kSearchTiles, lazy_run_override);
-  uint32_t best = 1;
-  uint64_t best_cost = ~uint64_t(0);
-  for (uint32_t G = 1; G <= kSearchTiles; ++G) {
-    uint64_t groups = 0;
-    for (uint32_t si : lists[kLazySegs]) groups += (segs[si].tile_count + G - 1) / G;
-    const uint64_t cost = (groups + sms - 1) / sms * (G + 1);
-    if (cost <= best_cost) {
-      best_cost = cost;
-      best = G;
+// Tiles per CTA of the link and the search kernel (one CTA per SM): a pass takes
+// (waves of CTAs) x (tiles per CTA + `extra`), where `extra` is what a CTA costs
+// beside its tiles, in tiles.  The smallest count within 1/8 of the cheapest is
+// taken, since tiles differ and small groups even that out.  Measured (us):
+//   links, extra 1.6 (the window before a run enters its table): 3 MiB in runs
+//   of 2 / 4 / 6 / 8 tiles 94 / 96 / 83 / 105; 16 MiB in 4 / 16 / 32 399 / 390 / 380
+//   search, extra 0.4 to level 6 (staging): 3 MiB of mixed data in groups of 2 /
+//   4 / 6 188 / 247 / 337, 1 MiB of text in 1 / 2 / 4 193 / 167 / 245; above, 2
+//   (the last long chains): 32 MiB of text at level 9 in 2 / 4 / 8 5920 / 4891 / 4432
+uint32_t Engine::lazy_group(uint32_t most, float extra) const {
+  float cost[kLazyRun + 1] = {};
+  float least = 0;
+  for (uint32_t G = 1; G <= most; ++G) {
+    uint64_t ctas = 0;
+    for (uint32_t si : lists[kLazySegs]) ctas += (segs[si].tile_count + G - 1) / G;
+    cost[G] = float((ctas + sms - 1) / sms) * (float(G) + extra);
+    if (G == 1 || cost[G] < least) least = cost[G];
+  }
+  uint32_t G = 1;
+  while (cost[G] > least * 1.125f) ++G;
+  return G;
+}
+
+// The segments of a pass in groups of at most G tiles, as even as can be.
+void Engine::list_groups(int list, uint32_t G) {
+  for (uint32_t si : lists[kLazySegs]) {
+    const Segment& g = segs[si];
+    const uint32_t n = (g.tile_count + G - 1) / G;
+    for (uint32_t k = 0, t = 0; k < n; ++k) {
+      const uint32_t c = (g.tile_count - t + (n - k) - 1) / (n - k);
+      lists[list].push_back(g.tile_first + t);
+      lists[list].push_back(c);
+      t += c;
     }
   }
-  return best;
 }
 
 bool Engine::plan(const std::vector<Job>& jobs) {
@@ -397,33 +430,15 @@ bool Engine::plan(const std::vector<Job>& jobs) {
   off_segs = put_table(buf, segs);
   off_tiles = put_table(buf, tiles);
   off_ck = put_table(buf, cks);
-  // Links are built in runs of consecutive tiles of one segment (one CTA goes
-  // through a run after entering the 32 KiB before it in its table).  Short
-  // runs give small passes enough CTAs for every SM; long runs enter fewer
-  // windows.  The run length per level group and
-  // pass size is the autotuner's (geometry_table.h).
+  // Links are built and matches searched by CTAs that take several consecutive
+  // tiles of one segment.
   if (!lists[kLazySegs].empty()) {
-    const GeometryRow& geo = geometry(total);
-    for (uint32_t si : lists[kLazySegs]) {
-      const Segment& g = segs[si];
-      const int grp = g.level <= 6 ? 0 : g.level <= 9 ? 1 : 2;
-      const uint32_t R = std::min(kLazyRun, std::max(1u, lazy_run_override ? lazy_run_override : geo.lazy_run[grp]));
-      for (uint32_t t = 0; t < g.tile_count; t += R) {
-        lists[kLazyRuns].push_back(g.tile_first + t);
-        lists[kLazyRuns].push_back(std::min(R, g.tile_count - t));
-      }
-    }
-    const uint32_t G = search_group();
-    for (uint32_t si : lists[kLazySegs]) {
-      const Segment& g = segs[si];
-      const uint32_t n = (g.tile_count + G - 1) / G;  // groups of nearly equal size
-      for (uint32_t k = 0, t = 0; k < n; ++k) {
-        const uint32_t c = (g.tile_count - t + (n - k) - 1) / (n - k);
-        lists[kLazyGroups].push_back(g.tile_first + t);
-        lists[kLazyGroups].push_back(c);
-        t += c;
-      }
-    }
+    int top = 0;
+    for (uint32_t si : lists[kLazySegs]) top = std::max(top, segs[si].level);
+    const uint32_t cap = geometry(total).lazy_run[top <= 6 ? 0 : top <= 9 ? 1 : 2];
+    const uint32_t run = lazy_run_override, most = std::max(1u, std::min(kLazyRun, run ? run : cap));
+    list_groups(kLazyRuns, run ? most : lazy_group(most, 1.6f));
+    list_groups(kLazyGroups, run ? std::min(kSearchTiles, run) : lazy_group(std::min(kSearchTiles, most), top <= 6 ? 0.4f : 2.0f));
   }
   for (int i = 0; i < kNumLists; ++i) off_lists[i] = put_table(buf, lists[i]);
   off_counters = align_up(buf.size(), 256);

@@ -83,7 +83,8 @@ class Engine {
   void use_stream_ordered_arenas();
   uint32_t pick_tile(uint64_t total_bytes, int hash_bits) const;
   const GeometryRow& geometry(uint64_t total_bytes) const;
-  uint32_t search_group() const;
+  uint32_t lazy_group(uint32_t most, float extra) const;
+  void list_groups(int list, uint32_t G);
 
   int device = 0, sms = 148;
   bool ok = false;  // the stream and the device's constant tables are set up

@@ -7,8 +7,9 @@
 // bounds by their SM count).
 //   tile12, tile14  fast-level tile bytes at 12 hash bits (level 1) and
 //                   14 (levels 2-3): one warp walks one tile
-//   lazy_run[g]     tiles per CTA run at levels 4-6, 7-9 and 10-12: one CTA
-//                   slides its window over that many consecutive tiles
+//                   (passes of a few MiB are cut finer, Engine::pick_tile)
+//   lazy_run[g]     most tiles one CTA links or searches at levels 4-6, 7-9 and
+//                   10-12 (Engine::lazy_group picks the number)
 // Level 1-3 hash widths are fixed (parity with the reference); the output of
 // a pass does not depend on any value here.
 #pragma once
@@ -22,16 +23,16 @@ struct GeometryRow {
   uint32_t lazy_run[3];
 };
 
-constexpr const char* kGeometrySource = "orot_b200.tune on NVIDIA B200, 148 SMs, 2026-12-04";
+constexpr const char* kGeometrySource = "tile sweeps on NVIDIA B200, 148 SMs, 2026-12-05";
 constexpr GeometryRow kGeometry[] = {
-    {0ull, 4096, 8192, {1, 1, 1}},
-    {1ull << 20, 4096, 8192, {2, 2, 2}},
-    {4ull << 20, 4096, 8192, {8, 8, 1}},
-    {16ull << 20, 16384, 16384, {4, 4, 4}},
-    {64ull << 20, 16384, 16384, {16, 8, 4}},
-    {256ull << 20, 32768, 32768, {16, 16, 16}},
-    {1ull << 30, 32768, 65536, {32, 32, 16}},
-    {4ull << 30, 65536, 65536, {32, 32, 16}},
+    {0ull, 4096, 4096, {32, 32, 32}},
+    {8ull << 20, 4096, 8192, {32, 32, 32}},
+    {16ull << 20, 8192, 8192, {32, 32, 32}},
+    {32ull << 20, 8192, 16384, {32, 32, 32}},
+    {128ull << 20, 16384, 16384, {32, 32, 32}},
+    {256ull << 20, 16384, 32768, {32, 32, 32}},
+    {1ull << 30, 32768, 65536, {32, 32, 32}},
+    {4ull << 30, 65536, 65536, {32, 32, 32}},
 };
 
 }  // namespace orotb

@@ -8,7 +8,7 @@ report of every timing.
   level 1      tile bytes at 12 hash bits (one warp walks one tile)
   levels 2-3   tile bytes at 14 hash bits (timed at level 2)
   levels 4-6, 7-9, 10-12
-               tiles per CTA run (timed at levels 6, 9 and 12)
+               most tiles a CTA links or searches (timed at levels 6, 9 and 12)
 
 Workload per class: one buffer of the class size below 16 MiB, else
 buffers log-uniform in 1 KiB-4 MiB up to the class size, all from the mixed
@@ -31,10 +31,10 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 TABLE = os.path.join(HERE, "csrc", "geometry_table.h")
-CLASSES = [0, 1 << 20, 4 << 20, 16 << 20, 64 << 20, 256 << 20, 1 << 30, 4 << 30]
-CLASS_BYTES = [256 << 10, 1 << 20, 4 << 20, 16 << 20, 64 << 20, 256 << 20, 1 << 30, 4 << 30]
+CLASSES = [0, 8 << 20, 16 << 20, 32 << 20, 128 << 20, 256 << 20, 1 << 30, 4 << 30]
+CLASS_BYTES = [4 << 20, 8 << 20, 16 << 20, 48 << 20, 128 << 20, 256 << 20, 1 << 30, 4 << 30]
 TILES12 = [4096, 8192, 16384, 32768, 65536]
-TILES14 = [8192, 16384, 32768, 65536]
+TILES14 = [4096, 8192, 16384, 32768, 65536]
 RUNS = [1, 2, 4, 8, 16, 32]
 # largest class timed per level (larger classes take the last timed result)
 MAX_CLASS = {1: 4 << 30, 2: 4 << 30, 6: 1 << 30, 9: 1 << 30, 12: 256 << 20}
