@@ -79,6 +79,12 @@ struct deflate_gpu_batch {
   cudaStream_t graph_stream = nullptr;
   int launches = 0;
   bool ran = false;
+  std::mutex done_mu;
+  std::vector<Stream> done;  // the streams of the last run, once deflate_gpu_batch_sizes has waited for it
+  void forget() {
+    std::lock_guard<std::mutex> lk(done_mu);
+    done.clear();
+  }
   ~deflate_gpu_batch() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
@@ -86,6 +92,7 @@ struct deflate_gpu_batch {
 };
 
 static void drop_graph(deflate_gpu_batch* b) {
+  b->forget();
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   if (b->graph) cudaGraphDestroy(b->graph);
   b->gexec = nullptr;
@@ -210,6 +217,7 @@ int deflate_gpu_batch_run(deflate_gpu_batch* b, void* cuda_stream, int use_graph
   DeviceScope dev_scope(b->eng.device);
   Engine& e = b->eng;
   cudaStream_t st = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : e.stream;
+  b->forget();
   if (!use_graph) {
     if (!e.launch(st)) return -1;
     b->launches = e.launches;
@@ -254,6 +262,8 @@ int deflate_gpu_batch_sizes(deflate_gpu_batch* b, size_t* out_sizes) {
     return -1;
   }
   for (size_t i = 0; i < s.size(); ++i) out_sizes[i] = s[i].error ? 0 : s[i].out_size;
+  std::lock_guard<std::mutex> lk(b->done_mu);
+  b->done = std::move(s);
   return 0;
 }
 
@@ -334,9 +344,15 @@ size_t deflate_gpu_batch_output(deflate_gpu_batch* b, size_t i, void* dst, size_
   DeviceScope dev_scope(b->eng.device);
   Engine& e = b->eng;
   Stream s{};
-  if (cudaDeviceSynchronize() != cudaSuccess ||
-      cudaMemcpy(&s, static_cast<uint8_t*>(e.d_tables.p) + e.off_streams + i * sizeof(Stream), sizeof s,
-                 cudaMemcpyDeviceToHost) != cudaSuccess) {
+  bool known = false;
+  {
+    std::lock_guard<std::mutex> lk(b->done_mu);
+    known = i < b->done.size();  // sizes() has waited for the run and read its streams
+    if (known) s = b->done[i];
+  }
+  if (!known && (cudaDeviceSynchronize() != cudaSuccess ||
+                 cudaMemcpy(&s, static_cast<uint8_t*>(e.d_tables.p) + e.off_streams + i * sizeof(Stream), sizeof s,
+                            cudaMemcpyDeviceToHost) != cudaSuccess)) {
     set_error("D2H failed");
     return 0;
   }

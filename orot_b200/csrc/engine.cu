@@ -599,12 +599,55 @@ static size_t stage_piece(size_t n) {
   return n < kPieceStage ? n : std::max(kPieceMin, align_up((n + kStagePieces - 1) / kStagePieces, 4096));
 }
 
-// Pinned staging of a one-call entry point is sized at least this much, so
-// that the first calls do not each grow it (pinning memory is slow).
-constexpr size_t kStageMin = size_t(4) << 20;
 // Below this output bound, the result record and the whole output slot come
 // back in one device-to-host round trip (one wait instead of two).
 constexpr size_t kOneTripBound = size_t(1) << 20;
+
+bool Engine::upload(size_t dst_off, const void* src, size_t n) {
+  uint8_t* stage = static_cast<uint8_t*>(h_stage.p);
+  const size_t piece = stage_piece(n);
+  for (size_t o = 0; o < n; o += piece) {
+    const size_t len = std::min(piece, n - o);
+    host_copy(stage + o, static_cast<const uint8_t*>(src) + o, len);
+    if (cudaMemcpyAsync(static_cast<uint8_t*>(d_in.p) + dst_off + o, stage + o, len, cudaMemcpyHostToDevice, stream) !=
+        cudaSuccess) {
+      set_error("H2D failed");
+      return false;
+    }
+  }
+  return true;
+}
+
+bool Engine::download(void* dst, const uint8_t* d_src, size_t n) {
+  uint8_t* stage = static_cast<uint8_t*>(h_stage.p);
+  // staging that does not hold all of n is used as a ring of pieces
+  const size_t piece = h_stage.cap >= n ? stage_piece(n) : kPieceMin;
+  if (!made_stage_events) {
+    for (cudaEvent_t& ev : stage_ev) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    made_stage_events = true;
+  }
+  const size_t count = (n + piece - 1) / piece;
+  for (size_t k = 0; k < count + kStagePieces; ++k) {
+    if (k >= size_t(kStagePieces) && k - kStagePieces < count) {  // piece k - kStagePieces to the caller
+      const size_t d = k - kStagePieces, o = d * piece;
+      if (cudaEventSynchronize(stage_ev[d % kStagePieces]) != cudaSuccess) {
+        set_error("D2H failed");
+        return false;
+      }
+      host_copy(static_cast<uint8_t*>(dst) + o, stage + d % kStagePieces * piece, std::min(piece, n - o));
+    }
+    if (k < count) {
+      const size_t o = k * piece;
+      if (cudaMemcpyAsync(stage + k % kStagePieces * piece, d_src + o, std::min(piece, n - o), cudaMemcpyDeviceToHost,
+                          stream) != cudaSuccess ||
+          cudaEventRecord(stage_ev[k % kStagePieces], stream) != cudaSuccess) {
+        set_error("D2H failed");
+        return false;
+      }
+    }
+  }
+  return true;
+}
 
 size_t Engine::compress_host(const void* in, size_t n, void* out, size_t cap, int level, int fmt, bool parallel,
                              size_t block, uint32_t mode, Stream* result) {
@@ -612,20 +655,7 @@ size_t Engine::compress_host(const void* in, size_t n, void* out, size_t cap, in
   if (!ensure_io(align_up(n, 16), align_up(bound, 16))) return 0;
   if (!h_stage.ensure(std::max({n, bound + 64, kStageMin}))) return 0;
   uint8_t* stage = static_cast<uint8_t*>(h_stage.p);
-  const uint8_t* src = static_cast<const uint8_t*>(in);
-  if (n) {
-    // in pieces: the copy of piece k + 1 into staging overlaps the DMA of piece k
-    const size_t piece = stage_piece(n);
-    for (size_t o = 0; o < n; o += piece) {
-      const size_t len = std::min(piece, n - o);
-      host_copy(stage + o, src + o, len);
-      if (cudaMemcpyAsync(static_cast<uint8_t*>(d_in.p) + o, stage + o, len, cudaMemcpyHostToDevice, stream) !=
-          cudaSuccess) {
-        set_error("H2D failed");
-        return 0;
-      }
-    }
-  }
+  if (n && !upload(0, in, n)) return 0;
   std::vector<Job> jobs(1);
   jobs[0] = Job{0, n, 0, parallel ? std::min<uint64_t>(cap, bound) : bound, level, fmt, parallel, block, mode};
   if (!plan(jobs) || !launch(stream)) return 0;
@@ -639,37 +669,11 @@ size_t Engine::compress_host(const void* in, size_t n, void* out, size_t cap, in
   }
   if (result) *result = s;
   if (s.error || s.out_size == 0 || s.out_size > cap) return 0;
-  uint8_t* dst = static_cast<uint8_t*>(out);
   if (one_trip) {
-    std::memcpy(dst, stage + s.out_off, s.out_size);
+    std::memcpy(out, stage + s.out_off, s.out_size);
     return s.out_size;
   }
-  // in pieces: the copy out of piece k overlaps the DMA of piece k + 1
-  const size_t m = s.out_size;
-  const size_t piece = stage_piece(m);
-  if (!made_stage_events) {
-    for (cudaEvent_t& ev : stage_ev) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    made_stage_events = true;
-  }
-  int k = 0;
-  for (size_t o = 0; o < m; o += piece, ++k) {
-    const size_t len = std::min(piece, m - o);
-    if (cudaMemcpyAsync(stage + o, static_cast<uint8_t*>(d_out.p) + s.out_off + o, len, cudaMemcpyDeviceToHost,
-                        stream) != cudaSuccess ||
-        cudaEventRecord(stage_ev[k], stream) != cudaSuccess) {
-      set_error("D2H failed");
-      return 0;
-    }
-  }
-  k = 0;
-  for (size_t o = 0; o < m; o += piece, ++k) {
-    if (cudaEventSynchronize(stage_ev[k]) != cudaSuccess) {
-      set_error("D2H failed");
-      return 0;
-    }
-    host_copy(dst + o, stage + o, std::min(piece, m - o));
-  }
-  return s.out_size;
+  return download(out, static_cast<const uint8_t*>(d_out.p) + s.out_off, s.out_size) ? s.out_size : 0;
 }
 
 uint32_t Engine::checksum_host(uint32_t init, const void* data, size_t n, bool adler) {

@@ -74,6 +74,13 @@ class Engine {
   // kStreamOpen and `result` (optional) receives the stream's table entry.
   size_t compress_host(const void* in, size_t n, void* out, size_t cap, int level, int fmt, bool parallel, size_t block,
                        uint32_t mode = 0, Stream* result = nullptr);
+  // Caller memory to d_in.p + dst_off (input arena) and device memory to caller
+  // memory, through pinned staging (h_stage: n bytes; for download kStageRing are
+  // enough): in pieces, so that the host copy of one overlaps the DMA of
+  // another.  upload only queues its last copies on `stream`; download waits
+  // for everything queued there.
+  bool upload(size_t dst_off, const void* src, size_t n);
+  bool download(void* dst, const uint8_t* d_src, size_t n);
   uint32_t checksum_host(uint32_t init, const void* data, size_t n, bool adler);
   // Checksum of n bytes already on the device (d_data 16-byte aligned, with
   // readable padding after the last byte).
@@ -115,6 +122,11 @@ class Engine {
   bool made_stage_events = false;
   void phase_ms(float* ms) const;
 };
+
+// Pinned staging of a one-call entry point is sized at least this much, so
+// that the first calls do not each grow it (pinning memory is slow).
+constexpr size_t kStageMin = size_t(4) << 20;
+constexpr size_t kStageRing = size_t(32) << 20;
 
 std::mutex& global_mutex();
 

@@ -62,12 +62,17 @@ static deflate_result frame_range(const uint8_t* s, size_t n, int fmt, size_t* o
 deflate_result gzip_members_decompress(Engine& e, const uint8_t* in, size_t n, uint8_t* out, size_t cap,
                                        size_t* actual);
 
+// The first n decoded bytes to caller memory (the input's staging is free again).
+static bool fetch_output(Engine& e, uint8_t* out, size_t n) {
+  return e.h_stage.ensure(std::max(std::min(n, kStageRing), kStageMin)) && e.download(out, static_cast<const uint8_t*>(e.d_out.p), n);
+}
+
 // Decodes the raw DEFLATE bytes raw[0, len) on the device into d_out + out_off
 // (at most cap bytes).  Returns false on a device error; the job holds the
 // status, the bytes written and the input bytes the stream occupied.
 static bool decode_raw(Engine& e, const uint8_t* raw, size_t len, size_t out_off, size_t cap, InflateJob* job) {
   const size_t tbl = align_up(sizeof(InflateJob), 256) + 256;
-  if (!e.d_tables.ensure(tbl) || !e.h_stage.ensure(std::max<size_t>(len, 16))) return false;
+  if (!e.d_tables.ensure(tbl) || !e.h_stage.ensure(std::max<size_t>(len, kStageMin))) return false;
   uint8_t* dt = static_cast<uint8_t*>(e.d_tables.p);
   InflateJob* d_job = reinterpret_cast<InflateJob*>(dt);
   uint32_t* d_order = reinterpret_cast<uint32_t*>(dt + align_up(sizeof(InflateJob), 256));
@@ -77,9 +82,8 @@ static bool decode_raw(Engine& e, const uint8_t* raw, size_t len, size_t out_off
   job->out_off = out_off;
   job->out_cap = cap;
   const uint32_t zero = 0;
-  if (len) std::memcpy(e.h_stage.p, raw, len);
-  if ((len && cudaMemcpyAsync(e.d_in.p, e.h_stage.p, len, cudaMemcpyHostToDevice, e.stream) != cudaSuccess) ||
-      cudaMemcpyAsync(d_job, job, sizeof *job, cudaMemcpyHostToDevice, e.stream) != cudaSuccess ||
+  if (len && !e.upload(0, raw, len)) return false;
+  if (cudaMemcpyAsync(d_job, job, sizeof *job, cudaMemcpyHostToDevice, e.stream) != cudaSuccess ||
       cudaMemcpyAsync(d_order, &zero, 4, cudaMemcpyHostToDevice, e.stream) != cudaSuccess) {
     set_error("H2D failed");
     return false;
@@ -125,10 +129,7 @@ static deflate_result gzip_members_sequential(Engine& e, const uint8_t* in, size
     total += job.out_len;
     pos += off + job.in_used + 8;
   }
-  if (total && cudaMemcpy(out, e.d_out.p, total, cudaMemcpyDeviceToHost) != cudaSuccess) {
-    set_error("D2H failed");
-    return DEFLATE_MEM_ERROR;
-  }
+  if (total && !fetch_output(e, out, total)) return DEFLATE_MEM_ERROR;
   if (actual) *actual = total;
   return DEFLATE_OK;
 }
@@ -180,10 +181,7 @@ static deflate_result decompress_one(Engine& e, const uint8_t* in, size_t n, uin
       return gzip_members_sequential(e, in, n, out, cap, actual);
     return DEFLATE_DATA_ERROR;
   }
-  if (job.out_len && cudaMemcpy(out, e.d_out.p, job.out_len, cudaMemcpyDeviceToHost) != cudaSuccess) {
-    set_error("D2H failed");
-    return DEFLATE_MEM_ERROR;
-  }
+  if (job.out_len && !fetch_output(e, out, job.out_len)) return DEFLATE_MEM_ERROR;
   if (actual) *actual = job.out_len;
   return DEFLATE_OK;
 }

@@ -60,11 +60,15 @@ static std::vector<Member> find_members(const uint8_t* in, size_t n) {
     const size_t h = member_header(in + pos, n - pos);
     if (h == 0) break;
     size_t next = n;
-    for (size_t i = pos + h; i + 2 < n; ++i)
-      if (in[i] == 0x1F && in[i + 1] == 0x8B && i + 3 < n && in[i + 2] == 8 && member_header(in + i, n - i)) {
+    for (size_t i = pos + h; i + 3 < n; ++i) {
+      const void* hit = std::memchr(in + i, 0x1F, n - 3 - i);
+      if (!hit) break;
+      i = size_t(static_cast<const uint8_t*>(hit) - in);
+      if (in[i + 1] == 0x8B && in[i + 2] == 8 && member_header(in + i, n - i)) {
         next = i;
         break;
       }
+    }
     if (next < 8 || next - 8 < pos + h) break;
     const uint8_t* t = in + next - 8;
     Member m{pos, next, h, 0, size_t(uint32_t(t[4]) | (uint32_t(t[5]) << 8) | (uint32_t(t[6]) << 16) | (uint32_t(t[7]) << 24))};
@@ -88,7 +92,7 @@ deflate_result gzip_members_decompress(Engine& e, const uint8_t* in, size_t n, u
   }
   if (total > cap) return DEFLATE_MEM_ERROR;
   const size_t k = ms.size();
-  if (!e.ensure_io(align_up(n, 16) + 64, align_up(total, 16) + 64) || !e.h_stage.ensure(n)) return DEFLATE_MEM_ERROR;
+  if (!e.ensure_io(align_up(n, 16) + 64, align_up(total, 16) + 64) || !e.h_stage.ensure(std::max({n, std::min(total, kStageRing), kStageMin}))) return DEFLATE_MEM_ERROR;
   // decode jobs, largest first
   std::vector<InflateJob> jobs(k);
   std::vector<uint32_t> order(k);
@@ -128,10 +132,9 @@ deflate_result gzip_members_decompress(Engine& e, const uint8_t* in, size_t n, u
   Stream* d_st = reinterpret_cast<Stream*>(dt + o_st);
   CkBlock* d_ck = reinterpret_cast<CkBlock*>(dt + o_ck);
   uint32_t* d_cnt = reinterpret_cast<uint32_t*>(dt + o_cnt);
-  std::memcpy(e.h_stage.p, in, n);
   cudaStream_t s = e.stream;
-  if (cudaMemcpyAsync(e.d_in.p, e.h_stage.p, n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-      cudaMemcpyAsync(d_jobs, jobs.data(), k * sizeof(InflateJob), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+  if (!e.upload(0, in, n)) return DEFLATE_MEM_ERROR;
+  if (cudaMemcpyAsync(d_jobs, jobs.data(), k * sizeof(InflateJob), cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaMemcpyAsync(d_order, order.data(), k * 4, cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaMemcpyAsync(d_st, st.data(), k * sizeof(Stream), cudaMemcpyHostToDevice, s) != cudaSuccess ||
       (!ck.empty() && cudaMemcpyAsync(d_ck, ck.data(), ck.size() * sizeof(CkBlock), cudaMemcpyHostToDevice, s) != cudaSuccess)) {
@@ -158,10 +161,7 @@ deflate_result gzip_members_decompress(Engine& e, const uint8_t* in, size_t n, u
     const uint32_t crc = uint32_t(t[0]) | (uint32_t(t[1]) << 8) | (uint32_t(t[2]) << 16) | (uint32_t(t[3]) << 24);
     if (jobs[i].status != kInfOk || jobs[i].out_len != ms[i].out_size || st[i].checksum != crc) return DEFLATE_DATA_ERROR;
   }
-  if (total && cudaMemcpy(out, dec, total, cudaMemcpyDeviceToHost) != cudaSuccess) {
-    set_error("D2H failed");
-    return DEFLATE_MEM_ERROR;
-  }
+  if (total && !e.download(out, dec, total)) return DEFLATE_MEM_ERROR;
   if (actual) *actual = total;
   return DEFLATE_OK;
 }

@@ -153,8 +153,23 @@ def geometry_tile(pass_bytes: int, sms: int = 148, hash_bits: int = 12) -> int:
     return int(lib().orot_b200_geometry_tile(int(pass_bytes), int(sms), int(hash_bits)))
 
 
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype = ctypes.py_object
+_new_bytes.argtypes = [ctypes.c_char_p, ctypes.c_ssize_t]
+
+
+def _out(n: int) -> tuple[bytes, int]:
+    """A bytes object of at least n bytes that nothing has written yet, and the
+    address of its bytes: the library fills it before anyone sees it."""
+    b = _new_bytes(None, max(n, 2))  # (shorter ones may be shared)
+    return b, ctypes.cast(b, ctypes.c_void_p).value
+
+
 def _ptr(buf) -> tuple[int, int, object]:
-    """(address, length, keepalive) of a bytes-like or numpy buffer."""
+    """(address, length, keepalive) of a bytes-like or numpy buffer; the library
+    reads immutable ones in place."""
+    if type(buf) is bytes:
+        return ctypes.cast(buf, ctypes.c_void_p).value, len(buf), buf
     try:
         import numpy as np
         if isinstance(buf, np.ndarray):
@@ -179,12 +194,12 @@ def compress(data, level: int = Level.Default, format: Format = Format.Zlib) -> 
     L = lib()
     addr, n, keep = _ptr(data)
     bound = L.deflate_compress_bound(n, int(format))
-    out = ctypes.create_string_buffer(bound)
-    r = L.deflate_compress(addr if n else None, n, out, bound, int(level), int(format))
+    out, oaddr = _out(bound)
+    r = L.deflate_compress(addr if n else None, n, oaddr, bound, int(level), int(format))
     del keep
     if r == 0:
         raise Error(DEFLATE_BUF_ERROR, "deflate::compress: output buffer overflow " + last_error())
-    return out.raw[:r]
+    return out[:r]
 
 
 def decompress(data, format: Format = Format.Zlib, max_output: int = 256 << 20) -> bytes:
@@ -192,13 +207,13 @@ def decompress(data, format: Format = Format.Zlib, max_output: int = 256 << 20) 
     (include/orot/deflate.h:238-255); raises Error on failure."""
     L = lib()
     addr, n, keep = _ptr(data)
-    out = ctypes.create_string_buffer(max(max_output, 1))
+    out, oaddr = _out(max_output)
     actual = ctypes.c_size_t(0)
-    r = L.deflate_decompress(addr if n else None, n, out, max_output, ctypes.byref(actual), int(format))
+    r = L.deflate_decompress(addr if n else None, n, oaddr, max_output, ctypes.byref(actual), int(format))
     del keep
     if r != DEFLATE_OK:
         raise Error(r, "deflate::decompress failed " + last_error())
-    return out.raw[:actual.value]
+    return out[:actual.value]
 
 
 def compress_gzip_members(data, level: int = Level.Default, member_size: int = 1 << 20) -> bytes:
@@ -207,12 +222,12 @@ def compress_gzip_members(data, level: int = Level.Default, member_size: int = 1
     L = lib()
     addr, n, keep = _ptr(data)
     cap = L.deflate_gzip_members_bound(n, member_size)
-    out = ctypes.create_string_buffer(max(cap, 1))
-    r = L.deflate_gpu_compress_gzip_members(addr if n else None, n, int(level), member_size, out, cap)
+    out, oaddr = _out(cap)
+    r = L.deflate_gpu_compress_gzip_members(addr if n else None, n, int(level), member_size, oaddr, cap)
     del keep
     if r == 0:
         raise Error(DEFLATE_BUF_ERROR, "compress_gzip_members failed " + last_error())
-    return out.raw[:r]
+    return out[:r]
 
 
 NO_FLUSH, SYNC_FLUSH, FULL_FLUSH, FINISH = 0, 1, 2, 3
@@ -284,12 +299,12 @@ class ParallelCompressor:
         L = lib()
         addr, n, keep = _ptr(data)
         bound = L.deflate_compress_bound(n, int(Format.Gzip))
-        out = ctypes.create_string_buffer(bound)
-        r = L.deflate_parallel_compress(self._ctx, addr if n else None, n, out, bound)
+        out, oaddr = _out(bound)
+        r = L.deflate_parallel_compress(self._ctx, addr if n else None, n, oaddr, bound)
         del keep
         if r == 0:
             raise Error(DEFLATE_BUF_ERROR, "ParallelCompressor::compress: buffer overflow " + last_error())
-        return out.raw[:r]
+        return out[:r]
 
     def close(self) -> None:
         if self._ctx:
@@ -455,9 +470,9 @@ class DeviceBatch:
         return list(arr)
 
     def output(self, i: int, size: int) -> bytes:
-        buf = ctypes.create_string_buffer(max(size, 1))
-        r = lib().deflate_gpu_batch_output(self._b, i, buf, size)
-        return buf.raw[:r]
+        buf, addr = _out(size)
+        r = lib().deflate_gpu_batch_output(self._b, i, addr, size)
+        return buf[:r]
 
     def launches(self) -> int:
         return lib().deflate_gpu_batch_launches(self._b)
