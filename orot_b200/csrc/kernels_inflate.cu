@@ -40,7 +40,9 @@
 // the CTA is as large as can be and parts are short.  1 MiB streams of zlib
 // level 6 on a B200, against one warp per stream that decoded 64 bit offsets
 // at a time and followed the tokens one by one (whole deflate_decompress call,
-// ms): text 67.5 -> 2.1, integers (39 blocks) 4.2, 8-byte periods 1.1, zeros 1.0.
+// ms): text 67.5 -> 2.0, integers (39 blocks) 4.1, 8-byte periods 1.1, zeros 1.0.
+// One exit test per token and 16 consecutive bytes a thread when bytes are
+// coded took the text from 2.14 to 2.03.
 // 512 threads with parts of 480 bits take 2.7 on the text, 1024 threads with
 // parts of 480 bits 2.2.
 //
@@ -114,8 +116,8 @@ struct InfSmem {
   alignas(16) uint32_t map[kMapWords];  // token starts, by bit of the window
   union alignas(16) {
     uint32_t list[kBatch];  // bit positions of a batch's tokens
-    // a piece's bytes: at a token's first byte the literal, or kMatch |
-    // distance - 1; then kDone | byte, or the index of the byte copied
+    // a piece's bytes: at a token's first byte the literal, or its kMatch code;
+    // then the codes below
     uint16_t value[kPiece];
   };
   uint32_t bits[kPiece / 32];        // first bytes of tokens
@@ -127,9 +129,11 @@ struct InfSmem {
   uint8_t lens[320], raw[320];       // code lengths: literal/length at 0, distance at 288; as read
   uint32_t job, type, bad, hlit, hdist, used, stop;
 };
-constexpr uint32_t kMatch = 0x8000u, kDone = 0x8000u;
+// Codes of a piece's bytes: kMatch | distance - 1 at a match's start; then kDone |
+// byte, kBefore | bytes before the piece - 1, or an index (kHistory: in registers only).
+constexpr uint32_t kMatch = 0x8000u, kBefore = 0x8000u, kDone = 0x4000u, kHistory = 0x10000u;
 constexpr uint32_t kEndBlock = 1u << 30, kEndBad = 1u << 31, kEndFlags = kEndBlock | kEndBad;
-static_assert(kPiece <= 0x8000u, "indices leave the flag bit free");
+static_assert(kPiece <= kDone, "indices leave the flag bits free");
 static_assert(sizeof(InfSmem) <= 227 * 1024, "one CTA per SM");
 
 // Aligned input word j of a stream whose last bit is at absolute bit `endb`
@@ -425,31 +429,51 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
         const uint32_t limit = min(rem, (tid + 1) * kPartBits);  // tokens from here on are the next part's
         const bool active = tid < kParts && tid * kPartBits < rem;
         uint32_t begin = tid * kPartBits;  // where this part's first token starts, as far as known
+        // One test per token ends the inner loop; what it was is found behind it,
+        // so that a token is little more than its chain of lookups.
         auto decode_part = [&](auto again) {
           uint32_t pos = begin, word = tid * (kPartBits / 32), bits = 0, flag = 0;
           while (pos < limit) {
-            const uint32_t here = pos >> 5, bit = 1u << (pos & 31);
-            if (here != word) {  // a token has at most 48 bits: at most one word has no start
-              S.map[word] = bits;
-              if (here != word + 1) S.map[word + 1] = 0;
+            uint32_t e, d, nb, old = 0, next = pos;
+            bool out;
+            do {
+              pos = next;
+              const uint32_t here = pos >> 5, at = r0 + pos;
+              const uint32_t* sw = S.words + (at >> 5);
+              const uint32_t x0 = sw[0], x1 = sw[1], x2 = sw[2];
+              if constexpr (decltype(again)::value) old = S.map[here] >> (pos & 31);
+              const uint32_t w = __funnelshift_r(x0, x1, at & 31u), whi = __funnelshift_r(x1, x2, at & 31u);
+              e = S.lit[w & ((1u << kLitBits) - 1)];
+              // the map's words before this token's: at most one has no start (a token has at most 48 bits)
+              if (here != word) S.map[word] = bits;
+              if (here > word + 1) S.map[word + 1] = 0;
+              bits = here != word ? 0u : bits;
               word = here;
-              bits = 0;
+              const uint32_t tot = (e >> 6) & 31u;
+              d = S.dist[__funnelshift_r(w, whi, tot) & ((1u << kDistBits) - 1)];
+              const bool match = (e & 0x30u) == 0x10u;
+              nb = tot + (match ? (d >> 8) & 31u : 0u);
+              next = pos + nb;
+              // an end or invalid, a long code, the input's end, a start marked before
+              out = !e || (e & 0x20u) || (match && (!d || (d & 0x8000u))) || next > rem || (old & 1u);
+              if (!out) bits |= 1u << (pos & 31);
+            } while (!out && next < limit);
+            if (!out) {
+              pos = next;
+              break;
             }
-            if constexpr (decltype(again)::value) {
-              const uint32_t old = S.map[word];
-              if (old & bit) {  // from here on as before
-                S.map[word] = bits | (old & ~(bit - 1));
-                return;
-              }
+            if (old & 1u) {  // from here on as before
+              S.map[word] = bits | (S.map[word] & (kAll << (pos & 31)));
+              return;
             }
             uint32_t kind, len, dist;
-            const uint32_t next = pos + token_at(S, r0 + pos, kind, len, dist);
+            next = pos + token_at(S, r0 + pos, kind, len, dist);
             if (kind >= 2 || next > rem) {
               flag = kind == 2 && next <= rem ? kEndBlock : kEndBad;
               pos = next;
               break;
             }
-            bits |= bit;
+            bits |= 1u << (pos & 31);
             pos = next;
           }
           for (; word < (tid + 1) * (kPartBits / 32); ++word) {
@@ -575,33 +599,58 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
             }
             __syncthreads();
             uint8_t* ob = out + job.out_off + op + b0;
-            uint32_t open = 0;  // bytes of this thread (tid + k * kInfThreads) that are not known yet
-            uint32_t v[16];
+            // every thread codes 16 bytes in a row: a literal, an index of the
+            // piece, or how far before the piece the byte lies
+            {
+              const uint32_t j0 = tid * 16;
+              const uint32_t starts = (S.bits[tid >> 1] >> ((tid & 1) * 16)) & 0xFFFFu;
+              const uint32_t before = tid & 1 ? S.bits[tid >> 1] & 0xFFFFu : 0u;
+              uint32_t s = before ? j0 - 16 + 31 - __clz(before) : S.last[tid >> 1];
+              uint32_t e = S.value[s];
+              const uint4 c0 = reinterpret_cast<const uint4*>(S.value)[2 * tid], c1 = reinterpret_cast<const uint4*>(S.value)[2 * tid + 1];
+              const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+              __syncthreads();  // all codes are read
+              uint32_t v[8];
 #pragma unroll
-            for (uint32_t k = 0; k < 16; ++k) {
-              v[k] = kDone;
-              if (k * kInfThreads >= n) continue;
-              const uint32_t j = min(tid + k * kInfThreads, n - 1);  // (the last byte again past the end)
-              const uint32_t bm = S.bits[j >> 5] & (kAll >> (31 - (j & 31)));
-              const uint32_t s = bm ? (j & ~31u) + 31 - __clz(bm) : S.last[j >> 5];
-              const uint32_t e = S.value[s];
-              const uint32_t d = (e & 0x7FFFu) + 1;
-              // a match that overlaps itself repeats its first d bytes (the
-              // quotient is exact: it is below 258 and the half keeps it away
-              // from whole numbers)
-              uint32_t i = j - s;
-              if (__any_sync(kAll, i >= d)) i -= d * uint32_t(__fdividef(float(i) + 0.5f, float(d)));
-              const int src = int(s + i) - int(d);
-              const bool match = (e & kMatch) != 0;
-              v[k] = match && src < 0 ? kDone | ob[src] : match ? uint32_t(src) : kDone | (e & 255u);
+              for (uint32_t k = 0; k < 16; ++k) {
+                const uint32_t j = j0 + k;
+                if ((starts >> k) & 1u) {
+                  s = j;
+                  e = k & 1 ? cw[k / 2] >> 16 : cw[k / 2] & 0xFFFFu;
+                }
+                const uint32_t d = (e & 0x7FFFu) + 1;
+                uint32_t i = j - s;
+                // a match that overlaps itself repeats its first d bytes (the
+                // quotient is exact: it is below 258 and the half keeps it
+                // away from whole numbers)
+                if (i >= d && (e & kMatch)) i -= d * uint32_t(__fdividef(float(i) + 0.5f, float(d)));
+                const int src = int(s + i) - int(d);
+                const uint32_t x = !(e & kMatch) ? kDone | (e & 255u) : src >= 0 ? uint32_t(src) : kBefore | uint32_t(-1 - src);
+                v[k / 2] = k & 1 ? v[k / 2] | (x << 16) : x;
+              }
+              uint4* o4 = reinterpret_cast<uint4*>(S.value) + 2 * tid;
+              o4[0] = make_uint4(v[0], v[1], v[2], v[3]);
+              o4[1] = make_uint4(v[4], v[5], v[6], v[7]);
             }
             __syncthreads();
+            // bytes before the piece, neighbours by neighbouring threads
+            uint32_t open = 0;  // bytes of this thread (tid + k * kInfThreads) that are not known yet
 #pragma unroll
-            for (uint32_t k = 0; k < 16; ++k) {
-              const uint32_t j = tid + k * kInfThreads;
-              if (j < n) {
-                S.value[j] = uint16_t(v[k]);
-                if (!(v[k] & kDone)) open |= 1u << k;
+            for (uint32_t k0 = 0; k0 < 16; k0 += 8) {
+              uint32_t v[8];
+#pragma unroll
+              for (uint32_t k = 0; k < 8; ++k) {
+                const uint32_t j = tid + (k0 + k) * kInfThreads;
+                v[k] = j < n ? S.value[j] : kDone;
+              }
+#pragma unroll
+              for (uint32_t k = 0; k < 8; ++k)
+                if (v[k] & kBefore) v[k] = kHistory | ob[-1 - int(v[k] & 0x7FFFu)];
+#pragma unroll
+              for (uint32_t k = 0; k < 8; ++k) {
+                const uint32_t j = tid + (k0 + k) * kInfThreads;
+                if (v[k] & kHistory) S.value[j] = uint16_t(kDone | (v[k] & 255u));
+                else if (!(v[k] & kDone)) open |= 1u << (k0 + k);
               }
             }
             // -- copies: follow the indices until all are bytes, eight of a thread's at a time
