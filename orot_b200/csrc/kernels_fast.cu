@@ -10,25 +10,27 @@
 // parse.  That is what makes the path parallel:
 //
 //   k_lastocc     per tile, last position of every hash (shared atomics)
-//   k_carry_scan  per segment, exclusive prefix-max of those tables, in
+//   k_carry_scan  per segment, exclusive prefix of those tables, in
 //                 chunks of 32 tiles; k_carry_prefix over the chunks
 //   k_cand        one warp per tile, head[] in shared memory (18 walkers of
-//                 12.4 KB per SM at 12 hash bits): 32 positions per step;
-//                 hash, head lookup, insert by store and read-back (a
-//                 window with a repeated hash groups its lanes with
-//                 __match_any); the candidate distance of every position (2 bytes)
-//                 and the run period of every 32-position window.
+//                 12 KB per SM at 12 hash bits): 32 positions per step;
+//                 hash, head lookup, insert by store and read-back (what a
+//                 lane reads back names the lanes of its hash); the candidate
+//                 distance of every position (2 bytes) and the run period of
+//                 every 32-position window.
 //   k_parse       one warp per tile, no table (16 warps of 0.6 KB per CTA,
-//                 two CTAs per SM): capped match lengths per lane, greedy
-//                 parse resolved with ballots, fixed Huffman bits packed with
-//                 shared atomics and flushed as coalesced 128-byte stores.
-//                 The parse starts at the tile's first byte (speculation) and
-//                 one record per 32 positions remembers where it entered that
-//                 window; windows a match covers cost only that record.
-//   k_cand_parse  (the default) both passes in one persistent kernel: 16
-//                 walkers (4 at 14 hash bits) and the rest of 32 warps as
-//                 parsers per SM; a parser takes a tile once a walker has
-//                 published its candidates.
+//                 two CTAs per SM): match lengths up to 12 per lane, the greedy
+//                 parse by doubling along the lanes' paths, longer matches
+//                 measured by the whole warp when the parse reaches them;
+//                 fixed Huffman bits packed with shared atomics and flushed as
+//                 coalesced 128-byte stores.  The parse starts at the tile's
+//                 first byte (speculation) and one record per 32 positions
+//                 remembers where it entered that window; windows a match
+//                 covers cost only that record.
+//   k_cand_parse  (the default) both passes in one persistent kernel: 16 head
+//                 tables per SM (4 at 14 hash bits, each shared by three
+//                 warps) and the rest of 32 warps as parsers; a parser takes a
+//                 tile once its candidates are published.
 //   k_fix1/2/3    re-walk a tile from the true entry (where the previous
 //                 tile's parse ended; k_fix1 all tiles at once assuming the
 //                 previous speculation held, k_fix2 one warp per multi-tile
@@ -52,6 +54,16 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 __device__ __forceinline__ uint32_t hash_fast(uint32_t v, int hb) { return (v * 0x9E3779B1u) >> (32 - hb); }
 
 // ---------------------------------------------------------------- k_lastocc
+// Entry of a hash in the carried tables: the position mod 32768 with a valid
+// bit, and below it the first byte there; 0 if there is none (or only position
+// 0, which counts as none).  It is what head[] holds.  Of two entries the later
+// tile's stands, so no full position is needed; with full positions and no
+// byte a walker fetched the bytes one by one when it filled its table, and
+// these scattered loads took an eighth of k_cand_parse's time.
+__device__ __forceinline__ uint32_t carry_entry(uint32_t p, uint32_t byte) {
+  return p ? (((p & 0x7FFFu) | 0x8000u) << 8) | byte : 0u;
+}
+
 // Each thread hashes 16 consecutive positions from 5 loaded words; a position
 // followed by one with the same hash (runs) needs no atomic, since the later
 // position wins the max anyway.
@@ -86,20 +98,25 @@ __global__ void __launch_bounds__(256) k_lastocc(Work wk, const uint32_t* __rest
     for (int i = 0; i < 16; ++i) {
       const bool in = p0 + i >= t.start && p0 + i < lim;
       const bool next_in = i < 15 && p0 + i + 1 >= t.start && p0 + i + 1 < lim;
-      if (in && !(next_in && h[i] == h[i + 1])) atomicMax(&tbl[h[i]], p0 + i);
+      // position in the tile + 1, first byte
+      if (in && !(next_in && h[i] == h[i + 1]))
+        atomicMax(&tbl[h[i]], ((p0 + i - t.start + 1) << 8) | ((W[i >> 2] >> ((i & 3) * 8)) & 0xFFu));
     }
   }
   __syncthreads();
   uint32_t* slot = reinterpret_cast<uint32_t*>(wk.scratch + t.slot);
-  for (int i = threadIdx.x; i < H; i += blockDim.x) slot[i] = tbl[i];
+  for (int i = threadIdx.x; i < H; i += blockDim.x) {
+    const uint32_t e = tbl[i];
+    slot[i] = e ? carry_entry(t.start + (e >> 8) - 1, e & 0xFFu) : 0u;
+  }
 }
 
 // ---------------------------------------------------------------- k_carry_scan
-// Prefix-max over the tiles of a chunk of kCarryChunk tiles of a segment:
-// afterwards the slot of tile k holds max(last positions of the chunk's tiles
-// up to k), and the chunk's table the maximum of all of them.  k_carry_prefix
-// turns the chunks' tables into the maximum over all earlier chunks, so the
-// larger entry of a tile's slot and its chunk's table is the head[] state at
+// Last entries over the tiles of a chunk of kCarryChunk tiles of a segment:
+// afterwards the slot of tile k holds the last entry of the chunk's tiles up
+// to k, and the chunk's table the last of all of them.  k_carry_prefix turns
+// the chunks' tables into the last entry of all earlier chunks, so a tile's
+// slot, or where that has no entry its chunk's table, is the head[] state at
 // the start of tile k+1 (the walker takes it when it loads its table).
 //
 // One thread per hash went through all tiles of a segment: 4,096 threads and,
@@ -127,7 +144,7 @@ __global__ void __launch_bounds__(256) k_carry_scan(Work wk, const uint32_t* __r
       for (uint32_t j = 0; j < B; ++j) v[j] = slot[j] ? slot[j][h] : 0u;
 #pragma unroll
       for (uint32_t j = 0; j < B; ++j) {
-        run = max(run, v[j]);
+        run = v[j] ? v[j] : run;
         if (slot[j]) slot[j][h] = run;
       }
     }
@@ -153,7 +170,7 @@ __global__ void __launch_bounds__(256) k_carry_prefix(Work wk, const uint32_t* _
 #pragma unroll
       for (uint32_t j = 0; j < B; ++j) {
         if (c0 + j < nc) t[(c0 + j) * uint32_t(H)] = run;
-        run = max(run, v[j]);
+        run = v[j] ? v[j] : run;
       }
     }
   }
@@ -165,7 +182,6 @@ __global__ void __launch_bounds__(256) k_carry_prefix(Work wk, const uint32_t* _
 // window (so runs with a period up to 32 can be checked) and reaching 64
 // bytes past its start (the p side of every capped match length).
 constexpr uint32_t kRing = 128, kWbuf = 24;
-constexpr uint32_t kCapMax = 48;  // capped match length of lane 0 (48 - lane)
 
 struct WinState {
   uint32_t np, cursor, flushed, matches, tokens;
@@ -189,49 +205,48 @@ __device__ __forceinline__ uint32_t wload4(const uint32_t* wbuf, uint32_t off) {
   return __funnelshift_r(wbuf[off >> 2], wbuf[(off >> 2) + 1], (off & 3) * 8);
 }
 
-// Capped common-prefix length of the bytes at p (staged at wbuf offset po)
-// and at q (global), at most cap <= kCapMax.  The first 4 q-side words are
-// loaded in one batch (one memory latency covers matches up to ~12 bytes);
-// longer matches fetch one more word per step.  The loop runs while any lane
-// of the warp is still matching, so its trip count follows the longest match
-// in the window rather than the cap.  Every lane of the warp must call it.
-__device__ __forceinline__ uint32_t lcp_window(const SegBytes& sb, const uint32_t* wbuf, uint32_t po, uint32_t q,
-                                               uint32_t cap, bool active) {
-  constexpr int PRE = 4;
-  const uint32_t qa = q + sb.boff;
-  const uint32_t* qw = sb.w + (qa >> 2);
-  const uint32_t qs = (qa & 3) * 8;
-  const uint32_t* pw = wbuf + (po >> 2);  // p side: staged words, each loaded once
-  const uint32_t ps = (po & 3) * 8;
-  uint32_t v[PRE];
+// The first words of the bytes at q = p - d, where a match at p (d != 0) is
+// measured (up to 15 bytes past p; the arenas hold more beyond their data).
+// Two aligned 16-byte loads and a selection of words were 3% slower.
+__device__ __forceinline__ uint4 lcp_load(const SegBytes& sb, uint32_t p, uint32_t d) {
+  const uint32_t* q = sb.w + ((p - d + sb.boff) >> 2);
+  return d ? make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3)) : make_uint4(0, 0, 0, 0);
+}
+
+// Common-prefix length, up to kLcpNear, of the bytes at p (staged at wbuf
+// offset po) and at q (byte offset from sb.w), whose first words are `r`.
+constexpr uint32_t kLcpNear = 12;
+__device__ __forceinline__ uint32_t lcp_near(const uint32_t* wbuf, uint32_t po, uint32_t q, const uint4& r) {
+  const uint32_t* pw = wbuf + (po >> 2);  // words up to (po >> 2) + 3 <= 19 < kWbuf
+  const uint32_t ps = (po & 3) * 8, qs = (q & 3) * 8;
+  const uint32_t v[4] = {r.x, r.y, r.z, r.w};
+  uint32_t len = kLcpNear;
 #pragma unroll
-  for (int j = 0; j < PRE; ++j) v[j] = active && uint32_t(j) * 4 < cap + 4 ? __ldg(qw + j) : 0u;
-  uint32_t n = 0;
-  bool open = active && cap > 0;
-  uint32_t plo = pw[0];
-#pragma unroll
-  for (int j = 0; j < PRE - 1; ++j) {
-    if (!__any_sync(kFull, open)) break;
-    // staged words (po >> 2) + j + 1 <= 23 < kWbuf: in bounds for every lane
-    const uint32_t phi = pw[j + 1];
-    const uint32_t x = __funnelshift_r(plo, phi, ps) ^ __funnelshift_r(v[j], v[j + 1], qs);
-    plo = phi;
-    n += open ? (x ? (__ffs(x) - 1) >> 3 : 4u) : 0u;
-    open = open && !x && n < cap;
+  for (int j = 2; j >= 0; --j) {
+    const uint32_t x = __funnelshift_r(pw[j], pw[j + 1], ps) ^ __funnelshift_r(v[j], v[j + 1], qs);
+    if (x) len = 4 * j + ((__ffs(x) - 1) >> 3);
   }
-  uint32_t lo = v[PRE - 1];
-  for (uint32_t j = PRE - 1; __any_sync(kFull, open); ++j) {
-    if (open) {
-      const uint32_t hi = __ldg(qw + j + 1);
-      const uint32_t phi = pw[j + 1];
-      const uint32_t x = __funnelshift_r(plo, phi, ps) ^ __funnelshift_r(lo, hi, qs);
-      plo = phi;
-      lo = hi;
-      if (x) { n += (__ffs(x) - 1) >> 3; open = false; } else { n += 4; }
-      if (n >= cap) open = false;
-    }
+  return len;
+}
+
+// Length (at most maxm <= 258) of the match at p, d back, whose first kLcpNear
+// bytes are known to agree: eight bytes per lane, all at once.
+__device__ __forceinline__ uint32_t lcp_far(const SegBytes& sb, uint32_t p, uint32_t d, uint32_t maxm, uint32_t lane) {
+  static_assert(kLcpNear + 8 * 32 >= 258, "one round");
+  const uint32_t off = kLcpNear + 8 * lane;
+  uint32_t stop = kFull;
+  if (off < maxm) {
+    const uint32_t a = p + off + sb.boff, b = a - d;
+    const uint32_t *aw = sb.w + (a >> 2), *bw = sb.w + (b >> 2);
+    const uint32_t a0 = __ldg(aw), a1 = __ldg(aw + 1), a2 = __ldg(aw + 2);
+    const uint32_t b0 = __ldg(bw), b1 = __ldg(bw + 1), b2 = __ldg(bw + 2);
+    const uint32_t x0 = __funnelshift_r(a0, a1, (a & 3) * 8) ^ __funnelshift_r(b0, b1, (b & 3) * 8);
+    const uint32_t x1 = __funnelshift_r(a1, a2, (a & 3) * 8) ^ __funnelshift_r(b1, b2, (b & 3) * 8);
+    const uint32_t m = off + (x0 ? (__ffs(x0) - 1) >> 3 : x1 ? 4u + ((__ffs(x1) - 1) >> 3) : 8u);
+    if (m < off + 8 || m >= maxm) stop = min(m, maxm);
   }
-  return n < cap ? n : cap;
+  const uint32_t b = __ballot_sync(kFull, stop != kFull);
+  return __shfl_sync(kFull, stop, __ffs(b) - 1);
 }
 
 // Fixed-Huffman code tables for the parse kernels: literal b at [b], match
@@ -242,6 +257,7 @@ __device__ __forceinline__ uint32_t lcp_window(const SegBytes& sb, const uint32_
 // on its bits above the 7th): the 5-bit code reversed | extra-bit count << 8.
 constexpr uint32_t kDistTab = 256 + 259;
 constexpr uint32_t kCodeTab = kDistTab + 512;
+constexpr uint32_t kTabWords = (kCodeTab + 3) & ~3u;  // what follows the tables is 16-byte aligned
 __device__ __forceinline__ void fill_code_tab(uint32_t* tab) {
   for (uint32_t i = threadIdx.x; i < kCodeTab; i += blockDim.x) {
     uint32_t bits = 0, nb = 0;
@@ -299,58 +315,51 @@ __host__ __device__ constexpr uint32_t walker_words() { return ((1u << HB) * 3 +
 // `lane` holds position wpos+lane; `d` is its candidate distance (0 = none).
 __device__ __forceinline__ void parse_window(const SegBytes& sb, uint32_t n, uint32_t wpos, uint32_t lim,
                                              uint32_t lane, const uint32_t* wbuf, uint32_t woff, uint32_t d,
-                                             uint32_t* ring, uint32_t* out, WinState& st,
+                                             const uint4& v, uint32_t* ring, uint32_t* out, WinState& st,
                                              const uint32_t* ctab = nullptr) {
   const uint32_t p = wpos + lane;
-  uint32_t clen = 0;
-  bool exact = true;
+  uint32_t clen = 0;   // match length (0: literal), kLcpNear where `open`
+  bool open = false;   // at least that long
   const bool want = d && p >= st.np && lane < lim;
-  const uint32_t maxm = want ? min(258u, n - p) : 0u;
-  const uint32_t cap = want ? min(maxm, max(3u, kCapMax - lane)) : 0u;
   if (__any_sync(kFull, want)) {
-    clen = lcp_window(sb, wbuf, woff + lane, want ? p - d : p, cap, want);
+    const uint32_t near = lcp_near(wbuf, woff + lane, p - d + sb.boff, v);
     if (want) {
-      exact = clen < cap || cap == maxm;
+      const uint32_t maxm = n - p;
+      open = near == kLcpNear && maxm > kLcpNear;
+      clen = min(near, maxm);
       if (clen < 3) clen = 0;
-    } else {
-      clen = 0;
     }
   }
-  const uint32_t M = __ballot_sync(kFull, clen >= 3);
+  const uint32_t M = __ballot_sync(kFull, clen != 0);
   const uint32_t limmask = lim == 32 ? kFull : ((1u << lim) - 1);
   uint32_t cur = st.np - wpos, visited = 0;
-  int xl = -1;
-  while (cur < lim) {
-    const uint32_t nm = M & limmask & (kFull << cur);
-    if (!nm) { visited |= limmask & (kFull << cur); cur = lim; break; }
-    const uint32_t j = __ffs(nm) - 1;
-    visited |= (kFull << cur) & ((2u << j) - 1u);
-    const uint32_t lj = __shfl_sync(kFull, clen, j);
-    const bool ej = __shfl_sync(kFull, exact, j);
-    if (ej) { cur = j + lj; } else { xl = int(j); break; }
-  }
-  uint32_t full = 0;
-  if (xl >= 0) {
-    // warp-cooperative extension, 128 bytes per round
-    const uint32_t pj = wpos + xl;
-    const uint32_t dj = __shfl_sync(kFull, d, xl);
-    const uint32_t c0 = __shfl_sync(kFull, clen, xl);
-    const uint32_t maxm = min(258u, n - pj);
-    full = c0;
-    for (uint32_t base = c0; base < maxm; base += 128) {
-      const uint32_t off = base + 4 * lane;
-      uint32_t stop = kFull;
-      if (off < maxm) {
-        const uint32_t x = sb.load4(pj + off) ^ sb.load4(pj - dj + off);
-        const uint32_t m = x ? ((__ffs(x) - 1) >> 3) : 4u;
-        const uint32_t l4 = min(4u, maxm - off);
-        if (m < l4) stop = off + m;
-        else if (off + 4 >= maxm) stop = maxm;
-      }
-      const uint32_t b = __ballot_sync(kFull, stop != kFull);
-      if (b) { full = __shfl_sync(kFull, stop, __ffs(b) - 1); break; }
+  if (M) {
+    // The tokens are the lanes reached from lane `cur`: every lane collects
+    // the lanes of its path (its own path's first half and the second half of
+    // the lane reached) in five doublings.  A token that leaves the window or
+    // is longer than known leads to itself.
+    uint32_t to = lane + (clen ? clen : 1u), path = 1u << lane;
+    to = open || to >= 32 ? lane : to;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      path |= __shfl_sync(kFull, path, to);
+      to = __shfl_sync(kFull, to, to);
     }
-    cur = uint32_t(xl) + full;
+    path |= __shfl_sync(kFull, path, to);
+    const uint32_t longer = __ballot_sync(kFull, open);
+    do {
+      visited |= __shfl_sync(kFull, path, cur) & limmask;
+      const uint32_t j = 31 - __clz(visited);  // the last token
+      uint32_t len = __shfl_sync(kFull, clen, j);
+      if ((longer >> j) & 1u) {
+        len = lcp_far(sb, wpos + j, __shfl_sync(kFull, d, j), min(258u, n - wpos - j), lane);
+        if (lane == j) clen = len;
+      }
+      cur = j + (len ? len : 1u);
+    } while (cur < lim);
+  } else {
+    visited = limmask & (kFull << cur);
+    cur = lim;
   }
   const bool vis = (visited >> lane) & 1u;
   const bool ism = vis && ((M >> lane) & 1u);
@@ -358,7 +367,7 @@ __device__ __forceinline__ void parse_window(const SegBytes& sb, uint32_t n, uin
   if (ctab) {
     if (visited & M) {  // a match in the window: both codes, selected per lane
       uint32_t mc, mn;
-      tab_match(ctab, ism ? (int(lane) == xl ? full : clen) : 3u, ism ? d : 1u, mc, mn);
+      tab_match(ctab, ism ? (clen) : 3u, ism ? d : 1u, mc, mn);
       const uint32_t t = ctab[wload4(wbuf, woff + lane) & 0xFFu];
       code = !vis ? 0u : ism ? mc : (t & 0xFFFFu);
       nb = !vis ? 0u : ism ? mn : (t >> 16);
@@ -369,7 +378,7 @@ __device__ __forceinline__ void parse_window(const SegBytes& sb, uint32_t n, uin
     }
   } else if (vis) {
     if (ism) {
-      fixed_match(int(lane) == xl ? full : clen, d, code, nb);
+      fixed_match(clen, d, code, nb);
     } else {
       fixed_literal(wload4(wbuf, woff + lane) & 0xFFu, code, nb);
     }
@@ -419,23 +428,15 @@ __device__ __forceinline__ TileView tile_view(const Work& wk, const Tile& t, con
 // Speculative walk of one tile (parse entry = tile start): inserts every
 // position into head[], records the candidate distance of every position and
 // the parse entry (and run period) of every window, emits the fixed-Huffman
-// bits.  `carry` holds full segment positions (0 = empty).
+// bits.
 template <int HB>
-__device__ WinState walk_tile(const TileView& tv, const uint32_t* carry, uint32_t* smem_warp, uint32_t* ring,
+__device__ WinState walk_tile(const TileView& tv, uint32_t* smem_warp, uint32_t* ring,
                               uint32_t* wbuf, uint32_t* out, WinRec* rec, uint16_t* cand16) {
   constexpr int H = 1 << HB;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1;
   const HeadTab head{reinterpret_cast<uint16_t*>(smem_warp), reinterpret_cast<uint8_t*>(smem_warp) + 2 * H};
-  if (carry) {
-#pragma unroll 8
-    for (int i = lane; i < H; i += 32) {
-      const uint32_t pos = __ldg(carry + i);
-      head.put(i, pos, pos ? tv.sb.byte(pos) : 0u);
-    }
-  } else {
-    for (int i = lane; i < H; i += 32) head.put(i, 0, 0);
-  }
+  for (int i = lane; i < H; i += 32) head.put(i, 0, 0);
   for (uint32_t i = lane; i < kRing; i += 32) ring[i] = 0;
   __syncwarp();
   WinState st{tv.ts, 0, 0, 0, 0};
@@ -486,7 +487,10 @@ __device__ WinState walk_tile(const TileView& tv, const uint32_t* carry, uint32_
     }
     __syncwarp();
     const uint32_t lim = min(32u, tend - wpos);
-    if (st.np < wpos + lim) parse_window(tv.sb, tv.n, wpos, lim, lane, wbuf, woff, d, ring, out, st);
+    if (st.np < wpos + lim) {
+      const uint4 v = lcp_load(tv.sb, p, d);
+      parse_window(tv.sb, tv.n, wpos, lim, lane, wbuf, woff, d, v, ring, out, st);
+    }
   }
   flush_tail(ring, out, st, lane);
   return st;
@@ -549,7 +553,8 @@ __device__ FixOut fix_tile(const TileView& tv, uint32_t entry, const WinRec* rec
     const uint32_t pre = prefetch_window(tv.sb, wpos, lane);
     const uint32_t woff = stage_window(tv.sb, wpos, wbuf, lane, pre);
     const uint32_t d = lane < lim ? cand16[(w << 5) + lane] : 0u;
-    parse_window(tv.sb, tv.n, wpos, lim, lane, wbuf, woff, d, ring, out, st);
+    const uint4 v = lcp_load(tv.sb, wpos + lane, d);
+    parse_window(tv.sb, tv.n, wpos, lim, lane, wbuf, woff, d, v, ring, out, st);
   }
   flush_tail(ring, out, st, lane);
   r.bits = st.cursor;
@@ -565,95 +570,125 @@ __device__ FixOut fix_tile(const TileView& tv, uint32_t entry, const WinRec* rec
 // window, its run period (WinRec::run: D when all 32 positions have distance
 // D <= 32 and equal the bytes D earlier, with the first window after the run
 // in bits 8 and up; 0 for other windows).  Only this pass needs the head
-// table, so only it is limited to the walkers whose tables fit in shared
-// memory; the parse runs as a separate kernel with far more warps per SM.
-template <int HB>
-__device__ void cand_tile(const TileView& tv, const uint32_t* carry, const uint32_t* prefix, uint32_t* smem_warp,
-                          uint32_t* wbuf, WinRec* rec, uint16_t* cand16) {
-  constexpr int H = 1 << HB;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1;
-  const HeadTab head{reinterpret_cast<uint16_t*>(smem_warp), reinterpret_cast<uint8_t*>(smem_warp) + 2 * H};
+// table, so only it is limited to the tables that fit in shared memory.
+//
+// A table belongs to a team of warps that take windows in turn.  The order of
+// the windows matters only for the table (look up, store, read back): a warp
+// loads and hashes its window before its turn and turns candidates into
+// distances after it.  TEAM is 1 where tables for enough warps fit (12 hash
+// bits); at 14 bits four tables fill an SM, and one warp each issued 13% of
+// the time, waiting for its own results (96 MiB at level 3: 3.6 ms).
+
+// Fills a team's head[] from the carried tables (null: empty), four entries
+// per thread at a time.
+template <int HB, int TEAM>
+__device__ __forceinline__ void load_head(const uint32_t* carry, const uint32_t* prefix, uint32_t* table,
+                                          uint32_t member) {
+  constexpr uint32_t H = 1u << HB;
+  uint2* pos = reinterpret_cast<uint2*>(table);  // 4 entries
+  uint32_t* byte = table + H / 2;                // 4 entries
+  const uint32_t i0 = member * 32 + (threadIdx.x & 31);
   if (carry) {
     if (!prefix) prefix = carry;
-#pragma unroll 8
-    for (int i = lane; i < H; i += 32) {
-      const uint32_t pos = max(__ldg(carry + i), __ldg(prefix + i));
-      head.put(i, pos, pos ? tv.sb.byte(pos) : 0u);
+    const uint4 *ca = reinterpret_cast<const uint4*>(carry), *pa = reinterpret_cast<const uint4*>(prefix);
+#pragma unroll 4
+    for (uint32_t i = i0; i < H / 4; i += 32 * TEAM) {
+      const uint4 a = __ldg(ca + i), b = __ldg(pa + i);
+      const uint32_t e0 = a.x ? a.x : b.x, e1 = a.y ? a.y : b.y, e2 = a.z ? a.z : b.z, e3 = a.w ? a.w : b.w;
+      pos[i] = make_uint2(__byte_perm(e0, e1, 0x6521), __byte_perm(e2, e3, 0x6521));
+      byte[i] = __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
     }
   } else {
-    for (int i = lane; i < H; i += 32) head.put(i, 0, 0);
+    for (uint32_t i = i0; i < H / 4; i += 32 * TEAM) {
+      pos[i] = make_uint2(0, 0);
+      byte[i] = 0;
+    }
   }
-  __syncwarp();
+}
+
+// Barriers of team t (0 to 3): 4 t for all its warps, 4 t + 1 + j for the turn
+// of member j.  Barrier 0 is the CTA's before the teams start.
+__device__ __forceinline__ void bar_sync(uint32_t id, uint32_t threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t id, uint32_t threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+template <int TEAM>
+__device__ __forceinline__ void team_sync(uint32_t team) {
+  if constexpr (TEAM > 1) bar_sync(4 * team, 32 * TEAM);
+  else __syncwarp();
+}
+
+template <int HB, int TEAM>
+__device__ void cand_tile(const TileView& tv, const uint32_t* carry, const uint32_t* prefix, uint32_t* table,
+                          WinRec* rec, uint16_t* cand16, uint32_t team, uint32_t member, uint32_t* flag) {
+  constexpr int H = 1 << HB;
+  static_assert(TEAM <= 3, "four barriers per team");
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1;
+  uint16_t* hpos = reinterpret_cast<uint16_t*>(table);
+  uint8_t* hbyte = reinterpret_cast<uint8_t*>(table) + 2 * H;
+  if (TEAM > 1 && member == 0 && lane == 0) *flag = 0;
+  load_head<HB, TEAM>(carry, prefix, table, member);
   const uint32_t tend = tv.ts + tv.tl;
   const uint32_t nwin = (tv.tl + 31) >> 5;
-  uint32_t seg_D = 0, seg_start = 0;  // the run being recorded: its period and first window
-  uint32_t pre = prefetch_window(tv.sb, tv.ts, lane);
-  uint32_t prevD = 0;  // run period of the previous window (0 = not a run)
-  for (uint32_t w = 0; w < nwin; ++w) {
-    const uint32_t wpos = tv.ts + (w << 5);
-    const uint32_t woff = stage_window(tv.sb, wpos, wbuf, lane, pre);
-    if (w + 1 < nwin) pre = prefetch_window(tv.sb, wpos + 32, lane);
-    const uint32_t p = wpos + lane;
-    const bool ins = p < tend && p + 4 <= tv.n;
-    const uint32_t v4 = wload4(wbuf, woff + lane);
-    const uint32_t h = ins ? hash_fast(v4, HB) : 0u;
-    const uint32_t mine = p ? ((p & 0x7FFFu) | 0x8000u) : 0u;  // this position as a table entry
-    uint32_t d = 0, runD = 0;  // candidate distance (0 = none), run period of this window
-    uint32_t cpos = 0, cbyte = 0;  // the table's candidate: position mod 32768 | valid bit, first byte
-    bool done = false, have_c = false;
-    // A window that continues the previous window's run of period D (every
-    // position's 4 bytes equal those D earlier) has hashes repeating with
-    // period D.  When the last D lanes' hashes are distinct, every position's
-    // latest same-hash position is the one D earlier and the last D lanes
-    // hold the table's new entries, so the window is done without the
-    // same-hash search.  Period 1 needs no check.
-    if (prevD && __all_sync(kFull, p + 4 <= tend && wload4(wbuf, woff + lane - prevD) == v4)) {
-      const bool top = lane >= 32 - prevD;
-      if (prevD == 1) {
-        done = true;
-      } else {
-        cpos = head.pos[h];
-        cbyte = head.byte[h];
-        have_c = true;
+  const uint32_t ins_end = min(tend, tv.n >= 4 ? tv.n - 3 : 0u);  // positions that enter the table
+  // the two words around this lane's four bytes, kAhead of the team's turns ahead
+  constexpr int kAhead = 3;
+  uint32_t x0[kAhead], x1[kAhead];
+  auto fetch = [&](uint32_t w, uint32_t& a, uint32_t& b) {
+    const uint32_t p = tv.ts + (w << 5) + lane, q = p + tv.sb.boff;
+    a = p < ins_end ? __ldg(tv.sb.w + (q >> 2)) : 0u;
+    b = p < ins_end ? __ldg(tv.sb.w + (q >> 2) + 1) : 0u;
+  };
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) fetch(member + k * TEAM, x0[k], x1[k]);
+  const uint32_t sh = ((tv.ts + lane + tv.sb.boff) & 3u) * 8;  // the same in every window
+  uint32_t runs = 0;  // a run window was seen
+  team_sync<TEAM>(team);
+  for (uint32_t w0 = member; w0 < nwin; w0 += kAhead * TEAM) {
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint32_t w = w0 + k * TEAM;
+      if (w >= nwin) break;
+      const uint32_t wpos = tv.ts + (w << 5), p = wpos + lane;
+      const bool ins = p < ins_end;
+      const uint32_t v4 = __funnelshift_r(x0[k], x1[k], sh);
+      fetch(w + kAhead * TEAM, x0[k], x1[k]);
+      const uint32_t h = ins ? hash_fast(v4, HB) : 0u;
+      const uint32_t mine = p ? ((p & 0x7FFFu) | 0x8000u) : 0u;  // this position as a table entry
+      if constexpr (TEAM > 1) {
         __syncwarp();
-        if (top) head.pos[h] = uint16_t(mine);
-        __syncwarp();
-        done = !__any_sync(kFull, top && head.pos[h] != mine);
+        if (w) bar_sync(4 * team + 1 + member, 64);
       }
-      if (done) {
-        if (prevD == 1 && top) head.pos[h] = uint16_t(mine);
-        if (top) head.byte[h] = uint8_t(v4);
-        d = prevD;
-        runD = prevD;
-      }
-    }
-    if (!done) {
-      // the table's candidate (the latest position of the hash in earlier
-      // windows), read before any entry of this window is stored
-      if (!have_c) {
-        cpos = ins ? head.pos[h] : 0u;
-        cbyte = ins ? head.byte[h] : 0u;
-        __syncwarp();
-      }
+      // the table's candidate (position mod 32768 | valid bit, first byte): the
+      // latest position of the hash in earlier windows
+      uint32_t cpos = ins ? hpos[h] : 0u;
+      uint32_t cbyte = ins ? hbyte[h] : 0u;
+      __syncwarp();
       // Every lane stores its position and reads the entry back.  Positions
       // differ, so all read back their own exactly when no two lanes of the
-      // window share a hash; only then may the table's candidate stand for
-      // every lane and every lane's entry stay.  Otherwise (repeats within
-      // 32 bytes) the lanes of each hash are found with __match_any_sync,
-      // whose cost grows with the number of distinct hashes in the warp: the
-      // nearest earlier lane is the candidate and the last lane's entry
-      // stays.  After a run window (repeats all but certain) the probe is
-      // skipped.
-      bool clash = true, last = ins;
-      if (!prevD && !have_c) {
-        if (ins) head.pos[h] = uint16_t(mine);
-        __syncwarp();
-        clash = __any_sync(kFull, ins && head.pos[h] != mine);
-      }
-      if (clash) {
-        const uint32_t peers = __match_any_sync(kFull, ins ? h : kFull);
+      // window share a hash; then the table's candidate stands for every lane
+      // and every lane's entry stays.  Otherwise (repeats within 32 bytes) the
+      // lane whose entry was read back names the hash: lanes of one hash read
+      // the same one, so its five bits tell them apart from the others; the
+      // nearest earlier lane is the candidate and the last lane's entry stays.
+      if (ins) hpos[h] = uint16_t(mine);
+      __syncwarp();
+      const uint32_t got = ins ? hpos[h] : mine;
+      bool last = ins;
+      if (__any_sync(kFull, got != mine)) {
+        const uint32_t who = (got - wpos) & 31u;
+        uint32_t peers = __ballot_sync(kFull, ins);
+#pragma unroll
+        for (int b = 0; b < 5; ++b) {
+          const uint32_t bal = __ballot_sync(kFull, (who >> b) & 1u);
+          peers &= (who >> b) & 1u ? bal : ~bal;
+        }
         const uint32_t before = peers & lt;
+        last = ins && (peers >> lane) == 1u;
+        if (last) hpos[h] = uint16_t(mine);
         const uint32_t src = before ? 31 - __clz(before) : lane;
         const uint32_t vb = __shfl_sync(kFull, v4, src);
         if (ins && before) {
@@ -661,39 +696,55 @@ __device__ void cand_tile(const TileView& tv, const uint32_t* carry, const uint3
           cpos = c ? ((c & 0x7FFFu) | 0x8000u) : 0u;
           cbyte = vb & 0xFFu;
         }
-        last = ins && (peers >> lane) == 1u;
-        __syncwarp();
-        if (last) head.pos[h] = uint16_t(mine);
       }
-      if (last) head.byte[h] = uint8_t(v4);
+      if (last) hbyte[h] = uint8_t(v4);
+      __syncwarp();
+      if constexpr (TEAM > 1) {
+        if (w + 1 < nwin) bar_arrive(4 * team + 1 + (member + 1 == TEAM ? 0 : member + 1), 64);
+      }
       // candidate distance after the first-byte check at the candidate itself
+      uint32_t d = 0, run = 0;
       if (cpos & 0x8000u) {
         const uint32_t dist = (p - (cpos & 0x7FFFu)) & 0x7FFFu;
         if (dist != 0 && cbyte == (v4 & 0xFFu)) d = dist;
       }
+      if (p < tend) cand16[p - tv.ts] = uint16_t(d);
       // run window: every position has the same distance D <= 32 and its
       // four bytes equal the four bytes D earlier (checked only when every
       // lane has a distance of at most 32)
-      if (wpos >= 32 && __all_sync(kFull, d != 0 && d <= 32 && p + 4 <= tend)) {
+      if (wpos >= 32 && __all_sync(kFull, d - 1 < 32 && p + 4 <= tend)) {
         const uint32_t D = __shfl_sync(kFull, d, 0);
-        runD = __all_sync(kFull, d == D && wload4(wbuf, woff + lane - D) == v4) ? D : 0u;
+        if (__all_sync(kFull, d == D && tv.sb.load4(p - D) == v4)) run = D;
       }
+      if (lane == 0) rec[w].run = run;
+      runs |= run;
     }
-    if (p < tend) cand16[p - tv.ts] = uint16_t(d);
-    // consecutive run windows of one period form a run; when it ends, each of
-    // its windows records the period and the window after the run, so the
-    // fix-up crosses a run without scanning it
-    if (runD != seg_D) {
-      if (seg_D)
-        for (uint32_t k = seg_start + lane; k < w; k += 32) rec[k].run = seg_D | (w << 8);
-      seg_D = runD;
-      seg_start = w;
-    }
-    prevD = runD;
-    if (!runD && lane == 0) rec[w].run = 0;
   }
-  if (seg_D)
-    for (uint32_t k = seg_start + lane; k < nwin; k += 32) rec[k].run = seg_D | (nwin << 8);
+  // Consecutive run windows of one period form a run; each records the window
+  // after it, so that the fix-up crosses a run without scanning it.
+  __threadfence();  // this lane's candidates and records, before the flag
+  bool any = runs != 0;
+  if constexpr (TEAM > 1) {
+    if (any && lane == 0) *flag = 1;
+    team_sync<TEAM>(team);
+    if (member) return;
+    any = *flag != 0;
+  } else {
+    __syncwarp();
+  }
+  if (!any) return;
+  uint32_t next = 0, end = nwin;  // the run after a group's last window: its period and end
+  for (uint32_t g = (nwin + 31) / 32; g-- > 0;) {
+    const uint32_t w = g * 32 + lane;
+    const uint32_t D = w < nwin ? *reinterpret_cast<const volatile uint32_t*>(&rec[w].run) : 0u;
+    const uint32_t after = __shfl_down_sync(kFull, D, 1);
+    const uint32_t stop = __ballot_sync(kFull, D != (lane == 31 ? next : after)) & ~lt;
+    const uint32_t mine = stop ? g * 32 + __ffs(stop) : end;
+    if (D) rec[w].run = D | (mine << 8);
+    next = __shfl_sync(kFull, D, 0);
+    end = __shfl_sync(kFull, mine, 0);
+  }
+  __threadfence();
 }
 
 // The tables a tile's head[] starts from (null: none).
@@ -707,11 +758,10 @@ __device__ __forceinline__ const uint32_t* tile_prefix(const Work& wk, const Til
 template <int HB, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_cand(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                       uint32_t* __restrict__ counter) {
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   constexpr uint32_t HW = ((1u << HB) * 3 + 3) / 4;
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* head = sm + wid * (HW + kWbuf);
-  uint32_t* wbuf = head + HW;
+  uint32_t* head = sm + wid * HW;
   for (;;) {
     uint32_t i = 0;
     if (lane == 0) i = atomicAdd(counter, 1u);
@@ -720,8 +770,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_cand(Work wk, const uint32_t* __
     const Tile t = wk.tiles[list[i]];
     const Segment sg = wk.segs[t.seg];
     const TileView tv = tile_view(wk, t, sg);
-    cand_tile<HB>(tv, tile_carry(wk, t), tile_prefix(wk, t), head, wbuf, reinterpret_cast<WinRec*>(wk.scratch + t.rec),
-                  reinterpret_cast<uint16_t*>(wk.scratch + t.cand));
+    cand_tile<HB, 1>(tv, tile_carry(wk, t), tile_prefix(wk, t), head, reinterpret_cast<WinRec*>(wk.scratch + t.rec),
+                     reinterpret_cast<uint16_t*>(wk.scratch + t.cand), 0, 0, nullptr);
   }
 }
 
@@ -730,7 +780,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_cand(Work wk, const uint32_t* __
 // candidates: greedy parse, fixed-Huffman bits, and per window the parse
 // entry, bit offset and match count for the fix-up.  Windows that a match
 // covers entirely cost only that record.  Shared memory per warp is the bit
-// ring and the staged bytes, so many warps share an SM.  The candidates are
+// ring and the staged bytes, so many warps share an SM.  What a window needs
+// (its candidates, then the bytes they point at) is loaded one and two windows
+// ahead: loaded when needed, 16 MiB of text took 470 us in k_parse, now 347, and
+// 290 with long matches measured only where the parse meets them.  The candidates are
 // read at L2 (ld.global.cg): in the fused kernel they were written by other
 // SMs during the same launch.
 __device__ void parse_tile(const Work& wk, Tile* tp, uint32_t* ring, uint32_t* wbuf, const uint32_t* ctab) {
@@ -746,32 +799,49 @@ __device__ void parse_tile(const Work& wk, Tile* tp, uint32_t* ring, uint32_t* w
   WinState st{tv.ts, 0, 0, 0, 0};
   const uint32_t tend = tv.ts + tv.tl;
   const uint32_t nwin = (tv.tl + 31) >> 5;
-  // the next window's bytes and candidates are loaded one window ahead
-  uint32_t pre = prefetch_window(tv.sb, tv.ts, lane);
-  uint32_t dnext = lane < tv.tl ? __ldcg(c16 + lane) : 0u;
-  uint32_t pre_w = 0;
-  for (uint32_t w = 0; w < nwin; ++w) {
+  // Loaded ahead, since each depends on the one before: the candidates two
+  // windows, the bytes they point at and the window's own bytes one.
+  auto load_d = [&](uint32_t w) {
+    const uint32_t q = (w << 5) + lane;
+    return q < tv.tl ? uint32_t(__ldcg(c16 + q)) : 0u;
+  };
+  uint32_t w = 0, pre = prefetch_window(tv.sb, tv.ts, lane), d = load_d(0), d1 = load_d(1);
+  uint4 v = lcp_load(tv.sb, tv.ts + lane, d);
+  while (w < nwin) {
     const uint32_t wpos = tv.ts + (w << 5);
     const uint32_t lim = min(32u, tend - wpos);
     // parse state where the parse enters this window (lanes 0-2 write one field each)
-    const uint32_t f = lane == 0 ? st.np - tv.ts : lane == 1 ? st.cursor : st.matches;
+    uint32_t f = lane == 0 ? st.np - tv.ts : lane == 1 ? st.cursor : st.matches;
     if (lane < 3) reinterpret_cast<uint32_t*>(rec + w)[lane] = f;
-    if (st.np >= wpos + lim) continue;  // covered by a match
-    uint32_t woff, d;
-    if (pre_w == w) {
-      woff = stage_window(tv.sb, wpos, wbuf, lane, pre);
-      d = dnext;
-    } else {
-      woff = stage_window(tv.sb, wpos, wbuf, lane, prefetch_window(tv.sb, wpos, lane));
-      d = lane < lim ? __ldcg(c16 + (w << 5) + lane) : 0u;
-    }
+    const uint32_t woff = stage_window(tv.sb, wpos, wbuf, lane, pre);
+    uint32_t npre = 0, d2 = 0;
     if (w + 1 < nwin) {
-      pre = prefetch_window(tv.sb, wpos + 32, lane);
-      const uint32_t q = ((w + 1) << 5) + lane;
-      dnext = q < tv.tl ? __ldcg(c16 + q) : 0u;
-      pre_w = w + 1;
+      npre = prefetch_window(tv.sb, wpos + 32, lane);
+      d2 = load_d(w + 2);
     }
-    parse_window(tv.sb, tv.n, wpos, lim, lane, wbuf, woff, d, ring, out, st, ctab);
+    const uint4 nv = lcp_load(tv.sb, wpos + 32 + lane, d1);
+    parse_window(tv.sb, tv.n, wpos, lim, lane, wbuf, woff, d, v, ring, out, st, ctab);
+    ++w;
+    const uint32_t to = st.np >= tend ? nwin : (st.np - tv.ts) >> 5;  // the next window with a token
+    if (w < to) {
+      // windows that a match covers (at most 8) cost only their records
+      if (lane < to - w) {
+        rec[w + lane].entry = st.np - tv.ts;
+        rec[w + lane].bit = st.cursor;
+        rec[w + lane].matches = st.matches;
+      }
+      if (to == nwin) break;
+      w = to;
+      pre = prefetch_window(tv.sb, tv.ts + (w << 5), lane);
+      d = load_d(w);
+      d1 = load_d(w + 1);
+      v = lcp_load(tv.sb, tv.ts + (w << 5) + lane, d);
+    } else {
+      pre = npre;
+      d = d1;
+      d1 = d2;
+      v = nv;
+    }
   }
   flush_tail(ring, out, st, lane);
   if (lane == 0) {
@@ -808,17 +878,25 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_parse(Work wk, const uint32_t
 
 // ---------------------------------------------------------------- k_cand_parse
 // The candidate pass and the parse in one persistent kernel, one CTA of 32
-// warps per SM: the first CW warps are candidate walkers (head tables in
-// shared memory), the others parse, and a walker whose candidate work is
-// exhausted parses too.  Walkers take tiles in list order and publish each
+// warps per SM: CW teams of candidate walkers (a head table in shared memory
+// each), the others parse, and a walker whose candidate work is exhausted
+// parses too.  Walkers take tiles in list order and publish each
 // finished tile in `ready`; parsers take tiles in the same order and wait for
 // its flag.  The two kinds of warp have complementary limits (walkers:
 // shared-memory and warp-collective latency; parsers: instruction issue), so
 // an SM running both issues more than it does running either alone.  A walker
-// never waits, so every flag a parser waits for is set by a running warp; the
+// waits for its team only, so every flag a parser waits for is set by a running warp; the
 // wait is bounded all the same (kReadyWaitNs; the first parser that gives up
 // makes every later wait of the launch give up at once), and a parser that
 // gives up marks the tile's segment failed and leaves the tile as empty.
+//
+// Bound by instruction issue (60 to 77% of the issue slots, 110 instructions
+// per 32 positions to find candidates and 210 to parse them) and the L1's
+// look-ups of the matches' scattered bytes.  Launches on a B200, with
+// candidates' lanes grouped by __match_any, the carried bytes gathered, the
+// matches of a window followed one by one and their bytes loaded when needed,
+// against now: 16 MiB of text at level 1 649 -> 402 us, 96 MiB of mixed data
+// 1734 -> 1302, the same at level 3 3690 -> 1844.
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -849,38 +927,55 @@ __device__ __noinline__ bool wait_ready(const uint32_t* flag, uint32_t* abort) {
     }
   }
 }
+// Warps that share a head table.  At 14 hash bits 1 / 2 / 3 warps take 2646 /
+// 1965 / 1865 us for 96 MiB of mixed data.  At 12 bits 16 tables of one warp
+// leave as many parsers; 14 tables are 1 to 5% slower, 12 are 3 to 25%.
+template <int HB>
+__host__ __device__ constexpr int cand_team() { return HB <= 12 ? 1 : 3; }
 template <int HB>
 __host__ __device__ constexpr uint32_t cand_parse_words(int cw) {
-  return kCodeTab + uint32_t(cw) * (((1u << HB) * 3 + 3) / 4 + kWbuf) + uint32_t(32 - cw) * (kRing + kWbuf);
+  return kTabWords + 16 + uint32_t(cw) * (((1u << HB) * 3 + 3) / 4) + uint32_t(32 - cw * cand_team<HB>()) * (kRing + kWbuf);
 }
 template <int HB, int CW>
 __global__ void __launch_bounds__(1024, 1) k_cand_parse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                          uint32_t* __restrict__ counter, uint32_t* __restrict__ ready) {
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   constexpr uint32_t HW = ((1u << HB) * 3 + 3) / 4;
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int TEAM = cand_team<HB>();
+  constexpr uint32_t WALKERS = CW * TEAM;
   uint32_t* ctab = sm;
-  uint32_t* own = wid < CW ? sm + kCodeTab + wid * (HW + kWbuf)
-                           : sm + kCodeTab + CW * (HW + kWbuf) + (wid - CW) * (kRing + kWbuf);
+  uint32_t* taken = sm + kTabWords;  // the tile a team works on; from 8 on, whether it has run windows
+  uint32_t* tables = taken + 16;
+  uint32_t* own = wid < CW ? tables + wid * HW
+                  : wid < WALKERS ? tables + (wid % CW) * HW + (wid / CW) * (kRing + kWbuf)
+                                  : tables + CW * HW + (wid - WALKERS) * (kRing + kWbuf);
   fill_code_tab(ctab);
   __syncthreads();
-  if (wid < CW) {
+  if (wid < WALKERS) {
+    const uint32_t team = wid % CW, member = wid / CW;
     for (;;) {
       uint32_t i = 0;
-      if (lane == 0) i = atomicAdd(counter, 1u);
-      i = __shfl_sync(kFull, i, 0);
+      if constexpr (TEAM > 1) {
+        if (member == 0 && lane == 0) taken[team] = atomicAdd(counter, 1u);
+        team_sync<TEAM>(team);
+        i = taken[team];
+      } else {
+        if (lane == 0) i = atomicAdd(counter, 1u);
+        i = __shfl_sync(kFull, i, 0);
+      }
       if (i >= nlist) break;
       const Tile t = wk.tiles[list[i]];
       const Segment sg = wk.segs[t.seg];
       const TileView tv = tile_view(wk, t, sg);
-      cand_tile<HB>(tv, tile_carry(wk, t), tile_prefix(wk, t), own, own + HW,
-                    reinterpret_cast<WinRec*>(wk.scratch + t.rec), reinterpret_cast<uint16_t*>(wk.scratch + t.cand));
-      __threadfence();  // this lane's candidates and records, before the flag
+      cand_tile<HB, TEAM>(tv, tile_carry(wk, t), tile_prefix(wk, t), tables + team * HW,
+                          reinterpret_cast<WinRec*>(wk.scratch + t.rec),
+                          reinterpret_cast<uint16_t*>(wk.scratch + t.cand), team, member, taken + 8 + team);
       __syncwarp();
-      if (lane == 0) st_release_gpu(ready + i, 1u);
+      if (member == 0 && lane == 0) st_release_gpu(ready + i, 1u);
     }
   }
-  uint32_t* ring = own;  // a walker's head-table space holds a parser's ring and staged bytes
+  uint32_t* ring = own;  // a team's head-table space holds its warps' rings and staged bytes when it parses
   uint32_t* wbuf = own + kRing;
   for (;;) {
     uint32_t i = 0;
@@ -1102,14 +1197,13 @@ static bool fused_cand_parse() {
 template <int HB>
 static void launch_fast_t(const Work& wk, const FastLists& L, cudaStream_t st, int sms, Marks* mk) {
   constexpr int H = 1 << HB;
-  // Walkers per CTA: shared memory bounds them (12.9 KB each at 12 hash
-  // bits), and one CTA of 17 (219 KB) holds one more per SM than four CTAs
-  // of four, since every CTA also reserves 1 KB; 5% faster.  At 14 hash bits
-  // (49.7 KB each) four fit either way.
+  // Walkers per CTA: shared memory bounds them (12 KB each at 12 hash bits,
+  // 48 KB at 14), and one CTA per SM holds more than several that each reserve
+  // 1 KB.
   constexpr int WARPS = HB <= 12 ? 18 : 4;
   const size_t tbl_bytes = size_t(H) * 4;
   constexpr uint32_t HW = ((1u << HB) * 3 + 3) / 4;
-  const size_t csm = size_t(WARPS) * (HW + kWbuf) * 4;  // head table + staged bytes per walker
+  const size_t csm = size_t(WARPS) * HW * 4;  // a head table per walker
   // walker CTAs per SM, and the kernels' shared-memory limits, once per device
   static std::atomic<int> walk_per_sm[64];
   const int ds = device_slot();
@@ -1213,7 +1307,7 @@ template <int HB>
 __global__ void __launch_bounds__(256) k_noalloc(const uint8_t* __restrict__ in, uint32_t n, uint8_t* __restrict__ out,
                                                   int level_arg, int lv, int fmt, uint32_t* scratch,
                                                   unsigned long long* out_size) {
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   constexpr uint32_t HW = ((1u << HB) * 3 + 3) / 4;
   uint32_t* head = sm;
   uint32_t* ring = head + HW;
@@ -1244,7 +1338,7 @@ __global__ void __launch_bounds__(256) k_noalloc(const uint8_t* __restrict__ in,
   if (wid == 0) {
     if (lv >= 1) {
       const TileView tv{SegBytes{reinterpret_cast<const uint32_t*>(cin), 0}, n, 0, n};
-      const WinState r = walk_tile<HB>(tv, nullptr, head, ring, wbuf, bits, nullptr, nullptr);
+      const WinState r = walk_tile<HB>(tv, head, ring, wbuf, bits, nullptr, nullptr);
       if (lane == 0) { s_bits = r.cursor; s_matches = r.matches; }
     }
   } else {
