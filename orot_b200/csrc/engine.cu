@@ -190,15 +190,19 @@ static const GeometryRow& geometry_row(uint64_t total_bytes, int sms) {
 const GeometryRow& Engine::geometry(uint64_t total_bytes) const { return geometry_row(total_bytes, sms); }
 
 // Passes of a few MiB are bound by the time one warp needs for a tile (about
-// 50 us for 1 KiB, two kernels of 16 or 28 parsers and 16 or 4 walkers per SM),
-// so they are cut finer than the table's smallest tile, down to 512 bytes
-// (shorter tiles cannot be crossed as parts of a long run, see run_tile):
-// about 1,024 tiles or more at 12 hash bits and 512 at 14, whose tables are four
-// times as large.  Mean over five kinds of data (us), 512 / 1024 / 2048 / 4096:
-//   12 bits:  4 KiB  86 / 102 / 140 / 194   512 KiB 181 / 185 / 224 / 312
-//             2 MiB 386 / 261 / 261 / 340     4 MiB 706 / 426 / 316 / 362
-//   14 bits: 32 KiB 133 / 146 / 183 / 259   512 KiB 276 / 209 / 232 / 319
-//             1 MiB 560 / 316 / 262 / 331     2 MiB 1002 / 599 / 368 / 362
+// 25 us for 1 KiB, once to find candidates and once to parse; 16 tables and as
+// many parsers per SM, 4 and 20 at 14 hash bits), so they are cut finer than
+// the table's smallest tile, down to 512 bytes (shorter tiles cannot be crossed
+// as parts of a long run, see run_tile): about 1,024 tiles or more at 12 hash
+// bits and 512 at 14, whose tables are four times as large; 2,048 tiles of 2 KiB
+// at 12 bits before 4 KiB tiles pay.  Mean over five kinds of data (us),
+// 512 / 1024 / 2048 / 4096:
+//   12 bits:  4 KiB  74 /  87 / 110 / 157   512 KiB 123 / 129 / 156 / 227
+//             1 MiB 169 / 145 / 169 / 237     2 MiB 266 / 191 / 185 / 245
+//             4 MiB 506 / 299 / 231 / 266     8 MiB 924 / 562 / 367 / 314
+//   14 bits: 32 KiB  91 / 102 / 122 / 174   512 KiB 161 / 138 / 151 / 209
+//             1 MiB 314 / 183 / 173 / 218     2 MiB 542 / 335 / 226 / 240
+//             4 MiB 989 / 576 / 386 / 303
 uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
   if (tile_override) return tile_override;
   const GeometryRow& g = geometry(total_bytes);
@@ -206,7 +210,7 @@ uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
   const uint64_t scaled = total_bytes * 148u / uint64_t(std::max(sms, 1));
   const uint64_t tiles = hash_bits <= 12 ? 2048 : 768;
   uint32_t t = 512;
-  while (t < most && t * tiles <= scaled) t *= 2;
+  while (t < most && t * (hash_bits <= 12 && t == 2048 ? 2 * tiles : tiles) <= scaled) t *= 2;
   return t;
 }
 

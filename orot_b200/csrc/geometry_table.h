@@ -29,7 +29,7 @@ constexpr GeometryRow kGeometry[] = {
     {8ull << 20, 4096, 8192, {32, 32, 32}},
     {16ull << 20, 8192, 8192, {32, 32, 32}},
     {32ull << 20, 8192, 16384, {32, 32, 32}},
-    {128ull << 20, 16384, 16384, {32, 32, 32}},
+    {64ull << 20, 16384, 16384, {32, 32, 32}},
     {256ull << 20, 16384, 32768, {32, 32, 32}},
     {1ull << 30, 32768, 65536, {32, 32, 32}},
     {4ull << 30, 65536, 65536, {32, 32, 32}},

@@ -31,8 +31,8 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 TABLE = os.path.join(HERE, "csrc", "geometry_table.h")
-CLASSES = [0, 8 << 20, 16 << 20, 32 << 20, 128 << 20, 256 << 20, 1 << 30, 4 << 30]
-CLASS_BYTES = [4 << 20, 8 << 20, 16 << 20, 48 << 20, 128 << 20, 256 << 20, 1 << 30, 4 << 30]
+CLASSES = [0, 8 << 20, 16 << 20, 32 << 20, 64 << 20, 128 << 20, 256 << 20, 1 << 30, 4 << 30]
+CLASS_BYTES = [4 << 20, 8 << 20, 16 << 20, 48 << 20, 96 << 20, 128 << 20, 256 << 20, 1 << 30, 4 << 30]
 TILES12 = [4096, 8192, 16384, 32768, 65536]
 TILES14 = [4096, 8192, 16384, 32768, 65536]
 RUNS = [1, 2, 4, 8, 16, 32]
