@@ -33,14 +33,14 @@ __host__ __device__ inline uint32_t fmt_trailer_bytes(uint32_t fmt) { return fmt
 // Three kernels, so that a stream of thousands of segments (a pigz-style
 // stream) or a segment of thousands of tiles (a large whole buffer) is
 // planned in parallel:
-//   k_plan_seg     one warp per segment: token bits and matches summed over
+//   k_plan_seg     one warp or CTA per segment: token bits and matches summed over
 //                  its tiles, the block type, and the block's length when it
 //                  does not depend on its bit alignment (Huffman blocks).
 //   k_plan_stream  one warp per stream: block offsets in order (32 segments
-//                  loaded at a time, followed through shuffles; a stored
-//                  block's padding depends on where it starts), stream size,
+//                  at a time; a stored block's padding depends on where
+//                  it starts), stream size,
 //                  capacity check, the closing sync point of an open part.
-//   k_plan_pieces  one warp per segment: its bit-range copies, at slots the
+//   k_plan_pieces  one warp or CTA per segment: its bit-range copies, at slots the
 //                  host reserved for the segment (Segment::piece_off); unused
 //                  slots are left empty (nbits 0).  More CTAs clear the words
 //                  the streams will occupy.
@@ -53,23 +53,44 @@ __device__ __forceinline__ uint64_t stored_bits_at(uint64_t c, uint32_t len) {
   return (((c + 3 + 7) & ~uint64_t(7)) - c) + 32 + uint64_t(len) * 8 + (pieces - 1) * 40;
 }
 
-__global__ void k_plan_seg(Work wk) {
-  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+// Warps per segment of k_plan_seg and k_plan_pieces (WPS): 8, a CTA, where the
+// segments are too few to fill the chip by themselves, since a warp goes through
+// 32 tiles per memory latency (16 MiB in one segment of 2,048 tiles: 29 and 66 us,
+// with 8 warps 9 and 20); else 1.
+constexpr uint32_t kPlanCtaSegs = 1024;
+
+// Sum over the threads of a segment (32 * WPS of them).
+template <int WPS>
+__device__ __forceinline__ unsigned long long seg_sum(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
+  if constexpr (WPS > 1) {
+    __shared__ unsigned long long part[WPS];
+    __syncthreads();  // the sum before has been read
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0;
+#pragma unroll
+    for (int k = 0; k < WPS; ++k) v += part[k];
+  }
+  return v;
+}
+
+template <int WPS>
+__global__ void __launch_bounds__(256) k_plan_seg(Work wk) {
+  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / (32 * WPS), lane = threadIdx.x % (32 * WPS);
   if (g >= wk.nsegs) return;
   const Segment sg = wk.segs[g];
   unsigned long long tok = 0, matches = 0;
   if (sg.level > 0) {
-    for (uint32_t t = sg.tile_first + lane; t < sg.tile_first + sg.tile_count; t += 32) {
+    for (uint32_t t = sg.tile_first + lane; t < sg.tile_first + sg.tile_count; t += 32 * WPS) {
       const Tile& tl = wk.tiles[t];
       tok += uint64_t(tl.fix_bits) + (tl.spec_bits - tl.splice_bit);
       matches += tl.fin_matches;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    tok += __shfl_xor_sync(kFullMask, tok, o);
-    matches += __shfl_xor_sync(kFullMask, matches, o);
-  }
+  tok = seg_sum<WPS>(tok);
+  matches = seg_sum<WPS>(matches);
   if (lane) return;
   uint32_t type = kBlkStored;
   uint64_t bits = 0;
@@ -98,32 +119,53 @@ __global__ void k_plan_stream(Work wk) {
   const uint32_t hdr = bare ? 0 : fmt_header_bytes(s.fmt), trl = bare ? 0 : fmt_trailer_bytes(s.fmt);
   uint64_t c = 0;  // bits from the start of the raw DEFLATE stream
   bool fault = false;  // a kernel could not finish one of the stream's segments
-  for (uint32_t g0 = s.seg_first; g0 < s.seg_first + s.seg_count; g0 += 32) {
-    const uint32_t cnt = min(32u, s.seg_first + s.seg_count - g0);
-    uint32_t type = 0, len = 0, last = 0;
-    uint64_t bits = 0;
-    if (lane < cnt) {
-      const Segment& sg = wk.segs[g0 + lane];
-      type = sg.block_type;
-      len = sg.len;
-      last = sg.flags & kSegLast;
-      bits = sg.bits;
-      if (sg.flags & kSegFault) fault = true;
+  // 32 segments at once, the next 32 loaded ahead.  A coded block's length is
+  // known; a stored one's depends on the bit it starts at within a byte, and it
+  // ends on a byte.  So the bits since the last stored block give each block
+  // its phase, that its length, and those the offsets.  One segment after the
+  // other took 50 us for 512 segments, now 14.
+  struct Row {
+    uint32_t type, len, flags;
+    uint64_t bits;
+  };
+  const uint32_t g_end = s.seg_first + s.seg_count;
+  auto load = [&](uint32_t g) {
+    Row r{kBlkFixed, 0, 0, 0};
+    if (g < g_end) {
+      const Segment& sg = wk.segs[g];
+      r = Row{sg.block_type, sg.len, sg.flags, sg.bits};
     }
-    uint64_t my_off = 0, my_bits = 0;
-    for (uint32_t j = 0; j < cnt; ++j) {
-      const uint32_t tj = __shfl_sync(kFullMask, type, j), lj = __shfl_sync(kFullMask, len, j);
-      const uint32_t fj = __shfl_sync(kFullMask, last, j);
-      const uint64_t bj = __shfl_sync(kFullMask, bits, j);
-      const uint64_t start = c;
-      c += tj == kBlkStored ? stored_bits_at(c, lj) : bj;
-      if (fj) c = (c + 7) & ~uint64_t(7);
-      if (lane == j) { my_off = start; my_bits = c - start; }
+    return r;
+  };
+  Row next = load(s.seg_first + lane);
+  for (uint32_t g0 = s.seg_first; g0 < g_end; g0 += 32) {
+    const Row r = next;
+    next = load(g0 + 32 + lane);
+    if (r.flags & kSegFault) fault = true;
+    const bool stored = r.type == kBlkStored;
+    const uint32_t before = __ballot_sync(kFullMask, stored) & ((1u << lane) - 1);
+    uint32_t x = stored ? 0u : uint32_t(r.bits) & 7u;
+    const uint32_t own = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(kFullMask, x, o);
+      if (lane >= uint32_t(o)) x += v;
     }
-    if (lane < cnt) {
-      wk.segs[g0 + lane].bit_off = my_off;
-      wk.segs[g0 + lane].bits = my_bits;
+    const uint32_t since = __shfl_sync(kFullMask, x, before ? 31 - __clz(before) : 0);
+    const uint32_t phase = (before ? x - own - since : uint32_t(c) + x - own) & 7u;
+    uint64_t n = stored ? stored_bits_at(phase, r.len) : r.bits;
+    if (r.flags & kSegLast) n += (8 - (phase + uint32_t(n))) & 7u;
+    uint64_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t v = __shfl_up_sync(kFullMask, incl, o);
+      if (lane >= uint32_t(o)) incl += v;
     }
+    if (g0 + lane < g_end) {
+      wk.segs[g0 + lane].bit_off = c + incl - n;
+      wk.segs[g0 + lane].bits = n;
+    }
+    c += __shfl_sync(kFullMask, incl, 31);
   }
   fault = __any_sync(kFullMask, fault);
   if (lane) return;
@@ -156,13 +198,15 @@ __device__ __forceinline__ void clear_output(const Work& wk, uint32_t si, uint32
 }
 
 // The CTAs after those of the segments clear the streams' words.
-__global__ void k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
+template <int WPS>
+__global__ void __launch_bounds__(256) k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
   if (blockIdx.x >= seg_ctas) {
     const uint32_t x = blockIdx.x - seg_ctas;
     clear_output(wk, x / parts, x % parts, parts);
     return;
   }
-  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  constexpr uint32_t N = 32 * WPS;  // threads of a segment
+  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / N, lane = threadIdx.x % N;
   if (g >= wk.nsegs) return;
   const Segment sg = wk.segs[g];
   const Stream& s = wk.streams[sg.stream];
@@ -173,16 +217,20 @@ __global__ void k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
   const uint32_t slots = seg_piece_slots(sg.tile_count, max(1u, (sg.len + 65534u) / 65535u));
   const uint64_t c = uint64_t(hdr) * 8 + sg.bit_off;  // block start in the output slot
   const bool last = (sg.flags & kSegLast) != 0;
-  for (uint32_t i = lane; i < slots; i += 32) pc[i].nbits = 0;
-  __syncwarp();
+  // slots that stay empty: from `used` on, and the code table's of a fixed block
+  const bool coded = sg.block_type != kBlkStored;
+  const uint32_t used = s.error ? 0u : coded ? 2 + 2 * sg.tile_count + (sg.block_type == kBlkDynamic ? 1u : 0u)
+                                             : (2 + kStoredSplit) * max(1u, (sg.len + 65534u) / 65535u);
+  for (uint32_t i = used + lane; i < slots; i += N) pc[i].nbits = 0;
   if (s.error) return;
+  if (lane == 0 && sg.block_type == kBlkFixed) pc[1].nbits = 0;
   if (sg.block_type == kBlkStored) {
     const uint32_t P = max(1u, (sg.len + 65534u) / 65535u);
     const uint64_t c1 = ((c + 3 + 7) & ~uint64_t(7)) + 32 + 8ull * 65535;  // start of piece 1 (when P > 1)
     // per stored piece its header, its length and kStoredSplit copies of 4 KiB
     // at most: one warp copies a Piece
     constexpr uint32_t kPer = 2 + kStoredSplit;
-    for (uint32_t x = lane; x < P * kPer; x += 32) {
+    for (uint32_t x = lane; x < P * kPer; x += N) {
       const uint32_t i = x / kPer, k = x % kPer;
       const uint64_t ci = i == 0 ? c : c1 + uint64_t(i - 1) * (40 + 8ull * 65535);
       const uint32_t off = i * 65535u, n = min(sg.len - off, 65535u);
@@ -195,7 +243,10 @@ __global__ void k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
       } else {
         constexpr uint32_t kPart = 65536 / kStoredSplit;
         const uint32_t o = (k - 2) * kPart;
-        if (o >= n) continue;
+        if (o >= n) {
+          pc[x].nbits = 0;
+          continue;
+        }
         const uint64_t a = sg.in_off + off + o;
         pc[x] = Piece{reinterpret_cast<const uint32_t*>(wk.in + (a & ~uint64_t(3))), dst, (a & 3) * 8,
                       lenpos + 32 + 8ull * o, min(kPart, n - o) * 8, 0};
@@ -214,30 +265,53 @@ __global__ void k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
   }
   // two copies per tile (fix-up bits, then the speculative bits from the
   // splice point), at offsets from a prefix sum over the tiles
-  for (uint32_t t0 = 0; t0 < sg.tile_count; t0 += 32) {
-    const uint32_t t = t0 + lane;
-    uint32_t fb = 0, sb = 0, sp = 0;
-    const Tile* tl = nullptr;
+  struct Row {
+    uint32_t fb, sp, bits, len;
+    uint64_t words;
+  };
+  auto load = [&](uint32_t t) {
+    Row r{0, 0, 0, 0, 0};
     if (t < sg.tile_count) {
-      tl = wk.tiles + sg.tile_first + t;
-      fb = tl->fix_bits;
-      sp = tl->splice_bit;
-      sb = tl->spec_bits - sp;
+      const Tile& tl = wk.tiles[sg.tile_first + t];
+      r = Row{tl.fix_bits, tl.splice_bit, tl.spec_bits, tl.len, tl.scratch};
     }
+    return r;
+  };
+  Row next = load(lane);
+  for (uint32_t t0 = 0; t0 < sg.tile_count; t0 += N) {
+    const uint32_t t = t0 + lane;
+    const Row r = next;
+    next = load(t + N);
+    const uint32_t fb = r.fb, sp = r.sp, sb = r.bits - sp;
     unsigned long long incl = uint64_t(fb) + sb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned long long v = __shfl_up_sync(kFullMask, incl, o);
-      if (lane >= uint32_t(o)) incl += v;
+      if ((lane & 31) >= uint32_t(o)) incl += v;
+    }
+    unsigned long long total;  // of these tiles
+    if constexpr (WPS > 1) {
+      __shared__ unsigned long long part[WPS];
+      __syncthreads();  // the sums before have been read
+      if ((lane & 31) == 31) part[lane >> 5] = incl;
+      __syncthreads();
+      total = 0;
+#pragma unroll
+      for (int k = 0; k < WPS; ++k) {
+        if (uint32_t(k) < lane >> 5) incl += part[k];
+        total += part[k];
+      }
+    } else {
+      total = __shfl_sync(kFullMask, incl, 31);
     }
     const uint64_t mine = at + incl - (uint64_t(fb) + sb);
-    if (tl) {
-      const uint32_t* spec = reinterpret_cast<const uint32_t*>(wk.scratch + tl->scratch);
-      const uint32_t* fix = reinterpret_cast<const uint32_t*>(wk.scratch + tl->scratch + tile_stream_bytes(tl->len));
+    if (t < sg.tile_count) {
+      const uint32_t* spec = reinterpret_cast<const uint32_t*>(wk.scratch + r.words);
+      const uint32_t* fix = reinterpret_cast<const uint32_t*>(wk.scratch + r.words + tile_stream_bytes(r.len));
       pc[2 + 2 * t] = Piece{fix, dst, 0, mine, fb, 0};
       pc[3 + 2 * t] = Piece{spec, dst, sp, mine + fb, sb, 0};
     }
-    at += __shfl_sync(kFullMask, incl, 31);
+    at += total;
   }
   if (lane == 0 && sg.block_type == kBlkDynamic) {
     const uint32_t eob = sg.eob;  // dynamic EOB: code | (len << 16)
@@ -550,12 +624,16 @@ CrcPowers host_crc_powers() {
 
 void launch_plan(const Work& wk, uint64_t max_out, cudaStream_t st) {
   if (!wk.nstreams) return;
-  if (wk.nsegs) k_plan_seg<<<(wk.nsegs + 7) / 8, 256, 0, st>>>(wk);
+  const bool cta = wk.nsegs <= kPlanCtaSegs;  // a CTA per segment
+  const uint32_t seg_ctas = cta ? wk.nsegs : (wk.nsegs + 7) / 8;
+  if (wk.nsegs) (cta ? k_plan_seg<8> : k_plan_seg<1>)<<<seg_ctas, 256, 0, st>>>(wk);
   k_plan_stream<<<(wk.nstreams + 7) / 8, 256, 0, st>>>(wk);
-  // about 1 MiB of output per clearing CTA for the largest stream
-  const uint32_t parts = uint32_t(std::min<uint64_t>(256, std::max<uint64_t>(1, max_out >> 20)));
-  const uint32_t seg_ctas = (wk.nsegs + 7) / 8;
-  k_plan_pieces<<<seg_ctas + wk.nstreams * parts, 256, 0, st>>>(wk, seg_ctas, parts);
+  // clearing CTAs per stream: 64 KiB of the largest stream's output each for few
+  // streams (128 MiB in one: 32 us, at 1 MiB each; now 17), 1 MiB for many
+  const uint64_t few = std::max<uint64_t>(1, 2048 / wk.nstreams);
+  const uint64_t most = std::min<uint64_t>(256, std::max<uint64_t>(1, max_out >> 20));
+  const uint32_t parts = uint32_t(std::max(most, std::min(few, max_out >> 16)));
+  (cta ? k_plan_pieces<8> : k_plan_pieces<1>)<<<seg_ctas + wk.nstreams * parts, 256, 0, st>>>(wk, seg_ctas, parts);
 }
 
 void launch_checksums(const Work& wk, bool frame, cudaStream_t st) {
