@@ -634,10 +634,12 @@ __global__ void __launch_bounds__(kSearchThreads, 1) k_search(Work wk, const uin
 //
 // Lazy parse (reference rule, lz77.cpp:449-493, with n = tile end): a parse
 // step depends only on its start position (the head), so the heads are found
-// in parallel: (1) each lane of warp 0 parses one 1/32 of the tile from its
-// start; (2) lane 0 follows the true parse into every part until it meets a
-// head of that part's parse, after which the two are the same; (3) the
-// threads emit the matches of the heads.  Tiles with few match positions are parsed by one lane.
+// in parallel: (1) each thread parses one part of the tile from its start; (2)
+// it parses again from where the part before was left, until it meets a head of
+// its own parse, after which the two are the same, and so on until no part is
+// left elsewhere than before; (3) the threads emit the matches of the heads.
+// With 32 parts, stitched one after the other by one lane, a tile of text took
+// 40 us, now 31 with 128 threads and 15 with 512; 32 MiB of it 302 and 239.
 //
 // Optimal parse (levels 10-12): costs from the histogram of the lazy parse,
 // then a backward pass finds, for every position, the cheapest way to the
@@ -645,20 +647,19 @@ __global__ void __launch_bounds__(kSearchThreads, 1) k_search(Work wk, const uin
 // then the path from position 0 is read.
 //
 // The chains of one warp are bound by latency, so they run apart from the
-// search, 16 and 14 tiles per SM at once, where the search CTA had one parsing
-// warp and 31 waiting ones; the other three warps of a CTA help to read the
-// matches, mark the tokens and fill the histogram.
+// search, up to 16 tiles per SM at once, where the search CTA had one parsing
+// warp and 31 waiting ones.
 namespace {
 constexpr uint32_t kFmWords = T / 32;
 static_assert(T % 32 == 0, "tiles are whole windows of 32 positions");
-constexpr uint32_t kSerialParse = 128;  // at most this many match positions: serial parse
+template <int N>  // threads
 struct ParseMem {
   uint16_t len[T];         // match length found at each position (optimal: then the token length)
   uint32_t fm[kFmWords];   // positions with a match
   uint32_t hd[kFmWords];   // heads, then the first positions of the parse's matches
   uint32_t em[kFmWords];
   uint32_t hist[320];
-  uint32_t sx[32];         // where each part's parse leaves it
+  uint32_t sx[N];  // where each part's parse leaves it
 };
 struct OptMem {
   uint32_t cost[512];      // cost to the tile end, by position mod 512
@@ -666,9 +667,8 @@ struct OptMem {
   uint16_t scost[320];     // symbol costs, 1/16 bit: 0-255 literals, 257+ lengths, 288+ distances
   uint16_t lcost[260];     // cost of a match length 0..258 (code + extra bits)
 };
-constexpr int kParseThreads = 128;
-template <bool Opt> struct ParseSmem { ParseMem p; };
-template <> struct ParseSmem<true> { ParseMem p; OptMem o; };
+template <bool Opt, int N> struct ParseSmem { ParseMem<N> p; };
+template <int N> struct ParseSmem<true, N> { ParseMem<N> p; OptMem o; };
 
 // First position >= i where a match starts (a set bit of fm), or tl.
 __device__ __forceinline__ uint32_t next_head(const uint32_t* fm, uint32_t i, uint32_t tl) {
@@ -729,13 +729,14 @@ __device__ __forceinline__ uint16_t sym_cost(uint32_t count, uint32_t total) {
 // Histogram of the tokens whose first positions are the bits of m.em (lengths
 // in m.len, distances in F's low halves); every byte no match covers is a
 // literal.  With `write`, F's words become the tokens.  The warps of the CTA
-// take a quarter of the windows each; all threads call it.
-__device__ void parse_tokens(ParseMem& m, uint32_t* F, uint32_t tl, const SegBytes& sb, uint32_t ts, bool write) {
+// share the windows; all threads call it.
+template <int N>
+__device__ void parse_tokens(ParseMem<N>& m, uint32_t* F, uint32_t tl, const SegBytes& sb, uint32_t ts, bool write) {
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (uint32_t k = threadIdx.x; k < 320; k += kParseThreads) m.hist[k] = 0;
+  for (uint32_t k = threadIdx.x; k < 320; k += uint32_t(N)) m.hist[k] = 0;
   __syncthreads();
   const uint32_t nwin = (tl + 31) / 32;
-  const uint32_t per = (nwin + kParseThreads / 32 - 1) / (kParseThreads / 32);
+  const uint32_t per = (nwin + uint32_t(N) / 32 - 1) / (uint32_t(N) / 32);
   const uint32_t wa = min(nwin, wid * per), wb = min(nwin, wa + per);
   uint32_t cover = 0;  // end of the last match before the window (a match reaches 8 windows on at most)
   for (uint32_t w = wa; w > 0 && w + 9 > wa;) {
@@ -780,9 +781,9 @@ __device__ void parse_tokens(ParseMem& m, uint32_t* F, uint32_t tl, const SegByt
 }
 }  // namespace
 
-template <bool Opt>
-__global__ void __launch_bounds__(kParseThreads) k_lparse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
-  __shared__ ParseSmem<Opt> S;
+template <bool Opt, int N>
+__global__ void __launch_bounds__(N) k_lparse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  __shared__ ParseSmem<Opt, N> S;
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (blockIdx.x >= nlist) return;
   Tile* tp = wk.tiles + list[blockIdx.x];
@@ -790,14 +791,14 @@ __global__ void __launch_bounds__(kParseThreads) k_lparse(Work wk, const uint32_
   const Segment sg = wk.segs[t.seg];
   const LazyCfg cfg = c_lazy[sg.level];
   if ((cfg.opt != 0) != Opt) return;  // the other kernel's tile
-  ParseMem& m = S.p;
+  ParseMem<N>& m = S.p;
   uint32_t* F = reinterpret_cast<uint32_t*>(wk.scratch + t.tok);
   const uint32_t tl = t.len, ts = t.start;
   const uint64_t o = sg.in_off;
   const SegBytes sb{reinterpret_cast<const uint32_t*>(wk.in + (o & ~uint64_t(3))), uint32_t(o & 3)};
 
   // -- lengths and the match bitmap, a warp's loads of eight windows in flight
-  constexpr uint32_t kWarps = kParseThreads / 32;
+  constexpr uint32_t kWarps = uint32_t(N) / 32;
   for (uint32_t w0 = 0; w0 < kFmWords; w0 += 8 * kWarps) {
     uint32_t f[8];
 #pragma unroll
@@ -815,70 +816,46 @@ __global__ void __launch_bounds__(kParseThreads) k_lparse(Work wk, const uint32_
       }
     }
   }
-  for (uint32_t w = tid; w < kFmWords; w += kParseThreads) m.hd[w] = m.em[w] = 0;
+  for (uint32_t w = tid; w < kFmWords; w += uint32_t(N)) m.hd[w] = m.em[w] = 0;
   __syncthreads();
 
-  // -- heads of the lazy parse
-  uint32_t nf = 0;  // positions with a match: few -> one lane parses alone
-  if (wid == 0) {
-    for (uint32_t w = lane; w < kFmWords; w += 32) nf += __popc(m.fm[w]);
-    nf = __reduce_add_sync(kAll, nf);
-  }
-  if (wid == 0 && nf <= kSerialParse) {
-    if (lane == 0) {
-      uint32_t i = 0;
-      while ((i = next_head(m.fm, i, tl)) < tl) {
-        m.hd[i >> 5] |= 1u << (i & 31);
-        i = lazy_step(m.len, i, tl, cfg.lazy);
-        i += m.len[i];
-      }
-    }
-  } else if (wid == 0) {
-    const uint32_t part = (tl + 31) / 32;
-    const uint32_t a = min(lane * part, tl), b = min(a + part, tl);
-    uint32_t i = a;
-    while (i < b) {
-      i = next_head(m.fm, i, tl);
-      if (i >= b) break;
-      atomicOr(&m.hd[i >> 5], 1u << (i & 31));
-      i = lazy_step(m.len, i, tl, cfg.lazy);
-      i += m.len[i];
-    }
-    m.sx[lane] = i;
-    __syncwarp();
-    if (lane == 0) {
-      uint32_t e = m.sx[0];
-      for (uint32_t k = 1; k < 32; ++k) {
-        const uint32_t a2 = min(k * part, tl), b2 = min(a2 + part, tl);
-        if (a2 >= b2) break;
-        clear_bits(m.hd, a2, min(e, b2));
-        if (e >= b2) continue;
-        uint32_t i2 = e;
-        for (;;) {
-          const uint32_t h = next_head(m.fm, i2, tl);
-          if (h >= b2) {
-            e = h;
-            break;
-          }
-          if ((m.hd[h >> 5] >> (h & 31)) & 1u) {
-            e = m.sx[k];
-            break;
-          }
-          m.hd[h >> 5] |= 1u << (h & 31);
-          i2 = lazy_step(m.len, h, tl, cfg.lazy);
-          i2 += m.len[i2];
-          clear_bits(m.hd, h + 1, min(i2, b2));
-          if (i2 >= b2) {
-            e = i2;
-            break;
-          }
+  // -- heads of the lazy parse: thread k those from part k's first position on,
+  // then again from where part k - 1 was left, until no exit changes
+  {
+    const uint32_t part = ((tl + 32 * uint32_t(N) - 1) / (32 * uint32_t(N))) * 32;
+    const uint32_t a = min(tid * part, tl), b = min(a + part, tl);
+    uint32_t entry = a;
+    auto walk = [&](bool again) {
+      uint32_t i = entry;
+      if (again) clear_bits(m.hd, a, min(i, b));
+      for (;;) {
+        const uint32_t h = i < b ? next_head(m.fm, i, b) : b;
+        if (h >= b) {
+          m.sx[tid] = max(i, b);
+          return;
         }
+        const uint32_t bit = 1u << (h & 31);
+        if (again && (m.hd[h >> 5] & bit)) return;  // from here on as before
+        m.hd[h >> 5] |= bit;  // a part is whole words
+        i = lazy_step(m.len, h, tl, cfg.lazy);
+        i += m.len[i];
+        if (again) clear_bits(m.hd, h + 1, min(i, b));
+      }
+    };
+    walk(false);
+    for (;;) {
+      __syncthreads();
+      const uint32_t e = tid ? m.sx[tid - 1] : 0u;
+      const bool again = a < b && e != entry;
+      if (!__syncthreads_or(again)) break;
+      if (again) {
+        entry = e;
+        walk(true);
       }
     }
   }
-  __syncthreads();
   // -- the matches of the heads
-  for (uint32_t w = tid; w < kFmWords; w += kParseThreads) {
+  for (uint32_t w = tid; w < kFmWords; w += uint32_t(N)) {
     uint32_t bits = m.hd[w];
     while (bits) {
       const uint32_t i = lazy_step(m.len, w * 32 + __ffs(bits) - 1, tl, cfg.lazy);
@@ -983,7 +960,7 @@ __global__ void __launch_bounds__(kParseThreads) k_lparse(Work wk, const uint32_
 
   parse_tokens(m, F, tl, sb, ts, true);
   uint32_t* gh = reinterpret_cast<uint32_t*>(wk.scratch + sg.hist);  // the segment's, cleared by k_link
-  for (uint32_t i = tid; i < 320; i += kParseThreads)
+  for (uint32_t i = tid; i < 320; i += uint32_t(N))
     if (m.hist[i]) atomicAdd(&gh[i], m.hist[i]);
   if (wid == 0) {
     uint32_t nm = 0;
@@ -1394,12 +1371,15 @@ __global__ void __launch_bounds__(kHuffThreads) k_huff(Work wk, const uint32_t* 
 // codes into the tile's bits in shared memory, which are written out in order.
 // A position belongs to a token unless the nearest match before it reaches it.
 // One warp per tile, a window after the other with the token chain followed by
-// shuffles, took 137 us for a single tile, this 23 us; 64 MiB of mixed data
-// 0.44 ms and 0.39 (the packing is bound by issue, each pass once per window).
-constexpr int kEncThreads = 256;
-__global__ void __launch_bounds__(kEncThreads) k_enc(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
-  constexpr uint32_t kWarps = kEncThreads / 32;
-  __shared__ uint32_t code[320];
+// shuffles, took 137 us for a single tile, this 24, 16 with 512 threads; 64 MiB of mixed data
+// 0.44 ms and 0.38 (the packing is bound by issue, each pass once per window).
+template <int N>
+__global__ void __launch_bounds__(N) k_enc(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  constexpr uint32_t kWarps = N / 32;
+  // literal codes; per match length code and extra bits | their number << 24;
+  // per distance - 1 below 256, or 256 + its bits above the 7th, the code |
+  // its bits << 16 | extra bits << 20
+  __shared__ uint32_t code[256], lens[259], dists[512];
   __shared__ uint32_t buf[kLazyTile / 2 + 64];  // at most 16 bits per byte (lazy_stream_bytes)
   __shared__ uint32_t warp_bits[kWarps];
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1411,8 +1391,23 @@ __global__ void __launch_bounds__(kEncThreads) k_enc(Work wk, const uint32_t* __
     if (tid == 0) { tp->spec_bits = 0; tp->spec_exit = t.start + t.len; }
     return;
   }
-  for (uint32_t k = tid; k < 320; k += kEncThreads) code[k] = reinterpret_cast<const uint32_t*>(wk.scratch + sg.codes)[k];
-  for (uint32_t k = tid; k < kLazyTile / 2 + 64; k += kEncThreads) buf[k] = 0;
+  const uint32_t* codes = reinterpret_cast<const uint32_t*>(wk.scratch + sg.codes);
+  for (uint32_t k = tid; k < 1024; k += N) {
+    if (k < 256) {
+      code[k] = codes[k];
+    } else if (k < 512) {
+      uint32_t li, le, lv;
+      length_code(k - 253, li, le, lv);  // 3 to 258
+      const uint32_t c = codes[257 + li], n = c >> 16;
+      lens[k - 253] = (c & 0xFFFFu) | (lv << n) | ((n + le) << 24);
+    } else {
+      const uint32_t i = k - 512;
+      uint32_t dc, de, dv;
+      dist_code((i < 256 ? i : (i - 256) << 7) + 1, dc, de, dv);
+      dists[i] = codes[288 + dc] | (de << 20);
+    }
+  }
+  for (uint32_t k = tid; k < kLazyTile / 2 + 64; k += N) buf[k] = 0;
   const uint32_t* tok = reinterpret_cast<const uint32_t*>(wk.scratch + t.tok);
   const uint64_t o = sg.in_off;
   const SegBytes sb{reinterpret_cast<const uint32_t*>(wk.in + (o & ~uint64_t(3))), uint32_t(o & 3)};
@@ -1453,14 +1448,13 @@ __global__ void __launch_bounds__(kEncThreads) k_enc(Work wk, const uint32_t* __
         const uint32_t end = prior ? pend : cover;
         uint32_t a = 0, na = 0, b = 0, nb = 0;
         if (tk) {
-          uint32_t li, le, lv, dc, de, dv;
-          length_code(len, li, le, lv);
-          dist_code(tk & 0xFFFFu, dc, de, dv);
-          const uint32_t lc = code[257 + li], dcw = code[288 + dc];
-          a = (lc & 0xFFFFu) | (lv << (lc >> 16));
-          na = (lc >> 16) + le;
-          b = (dcw & 0xFFFFu) | (dv << (dcw >> 16));
-          nb = (dcw >> 16) + de;
+          const uint32_t dm1 = (tk & 0xFFFFu) - 1;
+          const uint32_t le = lens[len], de = dists[dm1 < 256 ? dm1 : 256 + (dm1 >> 7)];
+          const uint32_t dn = (de >> 16) & 15u, dx = de >> 20;
+          a = le & 0xFFFFFFu;
+          na = le >> 24;
+          b = (de & 0xFFFFu) | ((dm1 & ((1u << dx) - 1u)) << dn);
+          nb = dn + dx;
         } else if (i < t.len && end <= i) {
           const uint32_t c = code[by4[k]];
           a = c & 0xFFFFu;
@@ -1500,7 +1494,7 @@ __global__ void __launch_bounds__(kEncThreads) k_enc(Work wk, const uint32_t* __
   });
   __syncthreads();
   uint32_t* out = reinterpret_cast<uint32_t*>(wk.scratch + t.scratch);
-  for (uint32_t k = tid; k < (total + 31) / 32; k += kEncThreads) out[k] = buf[k];
+  for (uint32_t k = tid; k < (total + 31) / 32; k += N) out[k] = buf[k];
   if (tid == 0) {
     tp->spec_bits = total;
     tp->spec_exit = t.start + t.len;
@@ -1519,12 +1513,22 @@ int launch_lazy(const Work& wk, const LazyLists& L, cudaStream_t st, int sms, Ma
   }
   k_link<<<L.n_runs, 1024, sizeof(LinkSmem), st>>>(wk, L.runs, L.n_runs);
   k_search<<<L.n_groups, kSearchThreads, kSearchSmem, st>>>(wk, L.groups, L.n_groups);
-  if (L.any_lazy) k_lparse<false><<<L.n_tiles, kParseThreads, 0, st>>>(wk, L.tiles, L.n_tiles);
-  if (L.any_opt) k_lparse<true><<<L.n_tiles, kParseThreads, 0, st>>>(wk, L.tiles, L.n_tiles);
+  // Where all tiles' CTAs run at once, their latency counts and they are larger.
+  // k_lparse of 128 / 512 threads (us): one tile of text 31 / 15, 1 MiB 41 / 20,
+  // 2 MiB (508 tiles) 42 / 26, 3 MiB 50 / 61, 64 MiB 412 / 712; k_enc of 256 / 512:
+  // one tile 24 / 16, 1 MiB 27 / 22, 2 MiB 33 / 36, 64 MiB 382 / 483.
+  const bool few = L.n_tiles <= 4 * uint32_t(sms), few_enc = L.n_tiles <= 2 * uint32_t(sms);
+  if (L.any_lazy)
+    few ? k_lparse<false, 512><<<L.n_tiles, 512, 0, st>>>(wk, L.tiles, L.n_tiles)
+        : k_lparse<false, 128><<<L.n_tiles, 128, 0, st>>>(wk, L.tiles, L.n_tiles);
+  if (L.any_opt)
+    few ? k_lparse<true, 512><<<L.n_tiles, 512, 0, st>>>(wk, L.tiles, L.n_tiles)
+        : k_lparse<true, 128><<<L.n_tiles, 128, 0, st>>>(wk, L.tiles, L.n_tiles);
   mk->mark(kPhLazyLz, st);
   k_huff<<<L.n_segs, kHuffThreads, 0, st>>>(wk, L.segs, L.n_segs);
   mk->mark(kPhLazyHuff, st);
-  k_enc<<<L.n_tiles, kEncThreads, 0, st>>>(wk, L.tiles, L.n_tiles);
+  few_enc ? k_enc<512><<<L.n_tiles, 512, 0, st>>>(wk, L.tiles, L.n_tiles)
+          : k_enc<256><<<L.n_tiles, 256, 0, st>>>(wk, L.tiles, L.n_tiles);
   mk->mark(kPhLazyEnc, st);
   return 4 + (L.any_lazy ? 1 : 0) + (L.any_opt ? 1 : 0);
 }
