@@ -17,6 +17,31 @@ inline int device_slot() {
   return d;
 }
 
+// The kernels of a pass are launched so that one may start while the one before
+// ends (programmatic dependent launch): every kernel begins with begin_kernel(),
+// which lets the next one be launched as soon as all CTAs of this one run, and
+// waits until the kernels before have completed and their writes are visible.
+// No kernel touches memory before that.  A pass is 8 to 13 launches, whose gaps
+// were a seventh of a small call: 4 KiB at level 6 148 -> 126 us, 100 kB at level 1
+// 178 -> 158; passes of many MiB take the same.
+__device__ __forceinline__ void begin_kernel() {
+  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Device pointers of one compression pass.
 struct Work {
   const uint8_t* in;     // input arena (16-byte aligned, 64 bytes of padding)

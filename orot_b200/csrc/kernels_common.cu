@@ -78,6 +78,7 @@ __device__ __forceinline__ unsigned long long seg_sum(unsigned long long v) {
 
 template <int WPS>
 __global__ void __launch_bounds__(256) k_plan_seg(Work wk) {
+  begin_kernel();
   const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / (32 * WPS), lane = threadIdx.x % (32 * WPS);
   if (g >= wk.nsegs) return;
   const Segment sg = wk.segs[g];
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(256) k_plan_seg(Work wk) {
 }
 
 __global__ void k_plan_stream(Work wk) {
+  begin_kernel();
   const uint32_t si = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (si >= wk.nstreams) return;
   Stream s = wk.streams[si];
@@ -200,6 +202,7 @@ __device__ __forceinline__ void clear_output(const Work& wk, uint32_t si, uint32
 // The CTAs after those of the segments clear the streams' words.
 template <int WPS>
 __global__ void __launch_bounds__(256) k_plan_pieces(Work wk, uint32_t seg_ctas, uint32_t parts) {
+  begin_kernel();
   if (blockIdx.x >= seg_ctas) {
     const uint32_t x = blockIdx.x - seg_ctas;
     clear_output(wk, x / parts, x % parts, parts);
@@ -329,6 +332,7 @@ constexpr uint32_t kCkBlock = 65536u;
 constexpr uint32_t kCkSub = 256u;
 
 __global__ void __launch_bounds__(256) k_ck_block(Work wk, CrcPowers pw) {
+  begin_kernel();
   __shared__ uint32_t tb[4][256];
   __shared__ uint32_t sc[256], sa[256], sb2[256], sl[256];
   for (int i = threadIdx.x; i < 1024; i += blockDim.x) tb[i >> 8][i & 255] = c_crc_slice[i >> 8][i & 255];
@@ -482,6 +486,7 @@ __device__ void write_frame(const Work& wk, const Stream& s, uint32_t check) {
 // One CTA per stream; with `frame` the stream's output (joined before) gets its
 // header and trailer.
 __global__ void __launch_bounds__(kFoldThreads) k_ck_fold(Work wk, CrcPowers pw, bool frame) {
+  begin_kernel();
   __shared__ CkPartial sh[kFoldThreads];
   const uint32_t si = blockIdx.x;
   if (si >= wk.nstreams) return;
@@ -523,6 +528,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_ck_single(const CkBlock* ck, u
 
 // ---------------------------------------------------------------- k_join
 __global__ void __launch_bounds__(256) k_join(Work wk, uint32_t* counter) {
+  begin_kernel();
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t i = 0;
@@ -626,26 +632,26 @@ void launch_plan(const Work& wk, uint64_t max_out, cudaStream_t st) {
   if (!wk.nstreams) return;
   const bool cta = wk.nsegs <= kPlanCtaSegs;  // a CTA per segment
   const uint32_t seg_ctas = cta ? wk.nsegs : (wk.nsegs + 7) / 8;
-  if (wk.nsegs) (cta ? k_plan_seg<8> : k_plan_seg<1>)<<<seg_ctas, 256, 0, st>>>(wk);
-  k_plan_stream<<<(wk.nstreams + 7) / 8, 256, 0, st>>>(wk);
+  if (wk.nsegs) launch_after((cta ? k_plan_seg<8> : k_plan_seg<1>), seg_ctas, 256, 0, st, wk);
+  launch_after(k_plan_stream, (wk.nstreams + 7) / 8, 256, 0, st, wk);
   // clearing CTAs per stream: 64 KiB of the largest stream's output each for few
   // streams (128 MiB in one: 32 us, at 1 MiB each; now 17), 1 MiB for many
   const uint64_t few = std::max<uint64_t>(1, 2048 / wk.nstreams);
   const uint64_t most = std::min<uint64_t>(256, std::max<uint64_t>(1, max_out >> 20));
   const uint32_t parts = uint32_t(std::max(most, std::min(few, max_out >> 16)));
-  (cta ? k_plan_pieces<8> : k_plan_pieces<1>)<<<seg_ctas + wk.nstreams * parts, 256, 0, st>>>(wk, seg_ctas, parts);
+  launch_after((cta ? k_plan_pieces<8> : k_plan_pieces<1>), seg_ctas + wk.nstreams * parts, 256, 0, st, wk, seg_ctas, parts);
 }
 
 void launch_checksums(const Work& wk, bool frame, cudaStream_t st) {
   const CrcPowers pw = host_crc_powers();
-  if (wk.nck) k_ck_block<<<wk.nck, 256, 0, st>>>(wk, pw);
-  if (wk.nstreams) k_ck_fold<<<wk.nstreams, kFoldThreads, 0, st>>>(wk, pw, frame);
+  if (wk.nck) launch_after(k_ck_block, wk.nck, 256, 0, st, wk, pw);
+  if (wk.nstreams) launch_after(k_ck_fold, wk.nstreams, kFoldThreads, 0, st, wk, pw, frame);
 }
 
 void launch_ck_single(const CkBlock* ck, uint32_t nck, uint64_t total, uint32_t init, int adler, uint32_t* res,
                       const Work& wk, cudaStream_t st) {
   const CrcPowers pw = host_crc_powers();
-  if (nck) k_ck_block<<<nck, 256, 0, st>>>(wk, pw);
+  if (nck) launch_after(k_ck_block, nck, 256, 0, st, wk, pw);
   k_ck_single<<<1, kFoldThreads, 0, st>>>(ck, nck, total, init, adler, pw, res);
 }
 
@@ -654,7 +660,7 @@ void launch_join(const Work& wk, uint32_t* counter, cudaStream_t st, int sms) {
   uint32_t blocks = uint32_t(sms) * 8;
   const uint32_t need = (wk.npieces + 7) / 8;
   if (blocks > need) blocks = need;
-  k_join<<<blocks, 256, 0, st>>>(wk, counter);
+  launch_after(k_join, blocks, 256, 0, st, wk, counter);
 }
 
 }  // namespace orotb

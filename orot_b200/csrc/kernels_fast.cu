@@ -69,6 +69,7 @@ __device__ __forceinline__ uint32_t carry_entry(uint32_t p, uint32_t byte) {
 // position wins the max anyway.
 template <int HB>
 __global__ void __launch_bounds__(256) k_lastocc(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  begin_kernel();
   extern __shared__ uint32_t tbl[];
   constexpr int H = 1 << HB;
   if (blockIdx.x >= nlist) return;
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(256) k_lastocc(Work wk, const uint32_t* __rest
 // with k_lastocc, 0.93 ms for the 4,096 tiles of a 16 MiB buffer; now 0.07 ms.
 template <int HB>
 __global__ void __launch_bounds__(256) k_carry_scan(Work wk, const uint32_t* __restrict__ chunks, uint32_t nchunks) {
+  begin_kernel();
   constexpr int H = 1 << HB;
   const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= uint32_t(H)) return;
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(256) k_carry_scan(Work wk, const uint32_t* __r
 
 template <int HB>
 __global__ void __launch_bounds__(256) k_carry_prefix(Work wk, const uint32_t* __restrict__ seglist, uint32_t nseg) {
+  begin_kernel();
   constexpr int H = 1 << HB;
   const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= uint32_t(H)) return;
@@ -758,6 +761,7 @@ __device__ __forceinline__ const uint32_t* tile_prefix(const Work& wk, const Til
 template <int HB, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_cand(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                       uint32_t* __restrict__ counter) {
+  begin_kernel();
   extern __shared__ __align__(16) uint32_t sm[];
   constexpr uint32_t HW = ((1u << HB) * 3 + 3) / 4;
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -860,6 +864,7 @@ __device__ void parse_tile(const Work& wk, Tile* tp, uint32_t* ring, uint32_t* w
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 2) k_parse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                           uint32_t* __restrict__ counter) {
+  begin_kernel();
   __shared__ uint32_t sm[WARPS][kRing + kWbuf];
   __shared__ uint32_t ctab[kCodeTab];
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -939,6 +944,7 @@ __host__ __device__ constexpr uint32_t cand_parse_words(int cw) {
 template <int HB, int CW>
 __global__ void __launch_bounds__(1024, 1) k_cand_parse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                          uint32_t* __restrict__ counter, uint32_t* __restrict__ ready) {
+  begin_kernel();
   extern __shared__ __align__(16) uint32_t sm[];
   constexpr uint32_t HW = ((1u << HB) * 3 + 3) / 4;
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1080,6 +1086,7 @@ __device__ __forceinline__ uint32_t run_exit(uint32_t entry, uint32_t end) {
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_fix1(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                       uint32_t* __restrict__ counter) {
+  begin_kernel();
   __shared__ uint32_t sm[WARPS][kRing + kWbuf];
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
@@ -1116,6 +1123,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_fix1(Work wk, const uint32_t* __
 // takes 19; 24,576 tiles of mixed data with runs 858 -> 288.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_fix2(Work wk, const uint32_t* __restrict__ seglist) {
+  begin_kernel();
   constexpr uint32_t G = WARPS * 32;
   __shared__ uint32_t sm[kRing + kWbuf];
   __shared__ uint32_t s_ent[G], s_ext[G], s_run[G], s_end[G], s_exit;
@@ -1189,6 +1197,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_fix2(Work wk, const uint32_t* __
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_fix3(Work wk, const uint32_t* __restrict__ list, uint32_t nlist,
                                                       uint32_t* __restrict__ counter) {
+  begin_kernel();
   __shared__ uint32_t sm[WARPS][kRing + kWbuf];
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
@@ -1235,12 +1244,12 @@ static void launch_fast_t(const Work& wk, const FastLists& L, cudaStream_t st, i
     if (per_sm < 1) per_sm = 1;
     walk_per_sm[ds].store(per_sm, std::memory_order_relaxed);
   }
-  if (L.n_lastocc) k_lastocc<HB><<<L.n_lastocc, 256, tbl_bytes, st>>>(wk, L.lastocc, L.n_lastocc);
+  if (L.n_lastocc) launch_after(k_lastocc<HB>, L.n_lastocc, 256, tbl_bytes, st, wk, L.lastocc, L.n_lastocc);
   if (L.n_multi) {
     dim3 g((H + 255) / 256, L.n_chunks < 65535u ? L.n_chunks : 65535u);
-    k_carry_scan<HB><<<g, 256, 0, st>>>(wk, L.chunks, L.n_chunks);
+    launch_after(k_carry_scan<HB>, g, 256, 0, st, wk, L.chunks, L.n_chunks);
     g.y = L.n_chunked < 65535u ? L.n_chunked : 65535u;
-    if (L.n_chunked) k_carry_prefix<HB><<<g, 256, 0, st>>>(wk, L.chunked, L.n_chunked);
+    if (L.n_chunked) launch_after(k_carry_prefix<HB>, g, 256, 0, st, wk, L.chunked, L.n_chunked);
   }
   mk->mark(kPhPre, st);
   if (L.n_walk && L.ready && fused_cand_parse()) {
@@ -1256,12 +1265,12 @@ static void launch_fast_t(const Work& wk, const FastLists& L, cudaStream_t st, i
     const uint32_t need = (L.n_walk + CW - 1) / CW;
     if (blocks > need) blocks = need;
     mk->mark(kPhCand, st);
-    k_cand_parse<HB, CW><<<blocks, 1024, fsm, st>>>(wk, L.walk, L.n_walk, L.counter, L.ready);
+    launch_after(k_cand_parse<HB, CW>, blocks, 1024, fsm, st, wk, L.walk, L.n_walk, L.counter, L.ready);
   } else if (L.n_walk) {
     uint32_t blocks = uint32_t(per_sm) * uint32_t(sms);
     const uint32_t need = (L.n_walk + WARPS - 1) / WARPS;
     if (blocks > need) blocks = need;
-    k_cand<HB, WARPS><<<blocks, WARPS * 32, csm, st>>>(wk, L.walk, L.n_walk, L.counter);
+    launch_after(k_cand<HB, WARPS>, blocks, WARPS * 32, csm, st, wk, L.walk, L.n_walk, L.counter);
     mk->mark(kPhCand, st);
     constexpr int PW = 16;
     static std::atomic<int> parse_per_sm[64];
@@ -1274,7 +1283,7 @@ static void launch_fast_t(const Work& wk, const FastLists& L, cudaStream_t st, i
     uint32_t pblocks = uint32_t(sms) * uint32_t(pps);
     const uint32_t pneed = (L.n_walk + PW - 1) / PW;
     if (pblocks > pneed) pblocks = pneed;
-    k_parse<PW><<<pblocks, PW * 32, 0, st>>>(wk, L.walk, L.n_walk, L.counter + 6);
+    launch_after(k_parse<PW>, pblocks, PW * 32, 0, st, wk, L.walk, L.n_walk, L.counter + 6);
   }
   mk->mark(kPhWalk, st);
   if (L.n_multi) {
@@ -1282,9 +1291,9 @@ static void launch_fast_t(const Work& wk, const FastLists& L, cudaStream_t st, i
     uint32_t blocks = uint32_t(sms) * 8;
     const uint32_t need = (L.n_walk + FW - 1) / FW;
     if (blocks > need) blocks = need;
-    k_fix1<FW><<<blocks, FW * 32, 0, st>>>(wk, L.walk, L.n_walk, L.counter + 4);
-    k_fix2<FW><<<L.n_multi, FW * 32, 0, st>>>(wk, L.multi);
-    k_fix3<FW><<<blocks, FW * 32, 0, st>>>(wk, L.walk, L.n_walk, L.counter + 8);
+    launch_after(k_fix1<FW>, blocks, FW * 32, 0, st, wk, L.walk, L.n_walk, L.counter + 4);
+    launch_after(k_fix2<FW>, L.n_multi, FW * 32, 0, st, wk, L.multi);
+    launch_after(k_fix3<FW>, blocks, FW * 32, 0, st, wk, L.walk, L.n_walk, L.counter + 8);
   }
   mk->mark(kPhFix, st);
 }

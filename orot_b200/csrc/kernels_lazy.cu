@@ -192,6 +192,7 @@ __device__ __forceinline__ void ring_stage(LinkSmem& S, const uint8_t* in, uint6
 }  // namespace
 
 __global__ void __launch_bounds__(1024, 1) k_link(Work wk, const uint32_t* __restrict__ runs, uint32_t nruns) {
+  begin_kernel();
   extern __shared__ __align__(128) uint8_t link_sm[];
   LinkSmem& S = *reinterpret_cast<LinkSmem*>(link_sm);
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -451,6 +452,7 @@ __device__ __forceinline__ bool none_longer(const uint16_t* link, uint32_t r, ui
 
 __global__ void __launch_bounds__(kSearchThreads, 1) k_search(Work wk, const uint32_t* __restrict__ runs,
                                                               uint32_t nruns) {
+  begin_kernel();
   extern __shared__ __align__(128) uint8_t search_sm[];
   const uint32_t* sdata = reinterpret_cast<const uint32_t*>(search_sm);
   const uint16_t* link = reinterpret_cast<const uint16_t*>(search_sm + kDataBytes);
@@ -783,6 +785,7 @@ __device__ void parse_tokens(ParseMem<N>& m, uint32_t* F, uint32_t tl, const Seg
 
 template <bool Opt, int N>
 __global__ void __launch_bounds__(N) k_lparse(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  begin_kernel();
   __shared__ ParseSmem<Opt, N> S;
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (blockIdx.x >= nlist) return;
@@ -1149,6 +1152,7 @@ __constant__ uint8_t c_cl_order[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 
 }  // namespace
 
 __global__ void __launch_bounds__(kHuffThreads) k_huff(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  begin_kernel();
   __shared__ HuffSmem S;
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (blockIdx.x >= nlist) return;
@@ -1375,6 +1379,7 @@ __global__ void __launch_bounds__(kHuffThreads) k_huff(Work wk, const uint32_t* 
 // 0.44 ms and 0.38 (the packing is bound by issue, each pass once per window).
 template <int N>
 __global__ void __launch_bounds__(N) k_enc(Work wk, const uint32_t* __restrict__ list, uint32_t nlist) {
+  begin_kernel();
   constexpr uint32_t kWarps = N / 32;
   // literal codes; per match length code and extra bits | their number << 24;
   // per distance - 1 below 256, or 256 + its bits above the 7th, the code |
@@ -1511,24 +1516,24 @@ int launch_lazy(const Work& wk, const LazyLists& L, cudaStream_t st, int sms, Ma
         cudaFuncSetAttribute(k_search, kMaxSmem, int(kSearchSmem)) == cudaSuccess)
       attr_set[ds].store(true, std::memory_order_relaxed);
   }
-  k_link<<<L.n_runs, 1024, sizeof(LinkSmem), st>>>(wk, L.runs, L.n_runs);
-  k_search<<<L.n_groups, kSearchThreads, kSearchSmem, st>>>(wk, L.groups, L.n_groups);
+  launch_after(k_link, L.n_runs, 1024, sizeof(LinkSmem), st, wk, L.runs, L.n_runs);
+  launch_after(k_search, L.n_groups, kSearchThreads, kSearchSmem, st, wk, L.groups, L.n_groups);
   // Where all tiles' CTAs run at once, their latency counts and they are larger.
   // k_lparse of 128 / 512 threads (us): one tile of text 31 / 15, 1 MiB 41 / 20,
   // 2 MiB (508 tiles) 42 / 26, 3 MiB 50 / 61, 64 MiB 412 / 712; k_enc of 256 / 512:
   // one tile 24 / 16, 1 MiB 27 / 22, 2 MiB 33 / 36, 64 MiB 382 / 483.
   const bool few = L.n_tiles <= 4 * uint32_t(sms), few_enc = L.n_tiles <= 2 * uint32_t(sms);
   if (L.any_lazy)
-    few ? k_lparse<false, 512><<<L.n_tiles, 512, 0, st>>>(wk, L.tiles, L.n_tiles)
-        : k_lparse<false, 128><<<L.n_tiles, 128, 0, st>>>(wk, L.tiles, L.n_tiles);
+    few ? launch_after(k_lparse<false, 512>, L.n_tiles, 512, 0, st, wk, L.tiles, L.n_tiles)
+        : launch_after(k_lparse<false, 128>, L.n_tiles, 128, 0, st, wk, L.tiles, L.n_tiles);
   if (L.any_opt)
-    few ? k_lparse<true, 512><<<L.n_tiles, 512, 0, st>>>(wk, L.tiles, L.n_tiles)
-        : k_lparse<true, 128><<<L.n_tiles, 128, 0, st>>>(wk, L.tiles, L.n_tiles);
+    few ? launch_after(k_lparse<true, 512>, L.n_tiles, 512, 0, st, wk, L.tiles, L.n_tiles)
+        : launch_after(k_lparse<true, 128>, L.n_tiles, 128, 0, st, wk, L.tiles, L.n_tiles);
   mk->mark(kPhLazyLz, st);
-  k_huff<<<L.n_segs, kHuffThreads, 0, st>>>(wk, L.segs, L.n_segs);
+  launch_after(k_huff, L.n_segs, kHuffThreads, 0, st, wk, L.segs, L.n_segs);
   mk->mark(kPhLazyHuff, st);
-  few_enc ? k_enc<512><<<L.n_tiles, 512, 0, st>>>(wk, L.tiles, L.n_tiles)
-          : k_enc<256><<<L.n_tiles, 256, 0, st>>>(wk, L.tiles, L.n_tiles);
+  few_enc ? launch_after(k_enc<512>, L.n_tiles, 512, 0, st, wk, L.tiles, L.n_tiles)
+          : launch_after(k_enc<256>, L.n_tiles, 256, 0, st, wk, L.tiles, L.n_tiles);
   mk->mark(kPhLazyEnc, st);
   return 4 + (L.any_lazy ? 1 : 0) + (L.any_opt ? 1 : 0);
 }
