@@ -32,7 +32,8 @@
 // rule of RFC 1951 3.2.2 (codes of one length are consecutive integers and
 // shorter codes precede longer ones): left-aligned, a code is below the end of
 // its length's range and of no shorter one's.
-// The code lengths of a dynamic block are read by one thread.
+// The code lengths of a dynamic block are read by one warp, 32 bit offsets at a
+// time (one thread took 16 to 32 thousand cycles a block).
 //
 // Bound by latency: the dependent steps of a token (two table lookups in shared
 // memory, shifts) times the tokens of a part times the rounds of
@@ -40,9 +41,10 @@
 // the CTA is as large as can be and parts are short.  1 MiB streams of zlib
 // level 6 on a B200, against one warp per stream that decoded 64 bit offsets
 // at a time and followed the tokens one by one (whole deflate_decompress call,
-// ms): text 67.5 -> 2.0, integers (39 blocks) 4.1, 8-byte periods 1.1, zeros 1.0.
+// ms): text 67.5 -> 1.9, integers (39 blocks) 3.8, 8-byte periods 1.0, zeros 1.0.
 // One exit test per token and 16 consecutive bytes a thread when bytes are
-// coded took the text from 2.14 to 2.03.
+// coded took the text from 2.14 to 2.03, indices reduced only where a match
+// overlaps itself to 1.97, code lengths read by a warp to 1.94.
 // 512 threads with parts of 480 bits take 2.7 on the text, 1024 threads with
 // parts of 480 bits 2.2.
 //
@@ -116,8 +118,7 @@ struct InfSmem {
   alignas(16) uint32_t map[kMapWords];  // token starts, by bit of the window
   union alignas(16) {
     uint32_t list[kBatch];  // bit positions of a batch's tokens
-    // a piece's bytes: at a token's first byte the literal, or its kMatch code;
-    // then the codes below
+    // a piece's bytes: at a token's first byte its code, then the codes below
     uint16_t value[kPiece];
   };
   uint32_t bits[kPiece / 32];        // first bytes of tokens
@@ -127,10 +128,10 @@ struct InfSmem {
   Canon lc, dc;
   uint32_t groups[10][16];           // build: codes of each length per 32 symbols
   uint8_t lens[320], raw[320];       // code lengths: literal/length at 0, distance at 288; as read
-  uint32_t job, type, bad, hlit, hdist, used, stop;
+  uint32_t job, type, bad, used, stop;
 };
-// Codes of a piece's bytes: kMatch | distance - 1 at a match's start; then kDone |
-// byte, kBefore | bytes before the piece - 1, or an index (kHistory: in registers only).
+// Codes of a piece's bytes: at a token's start kDone | literal or kMatch |
+// distance - 1; then kDone | byte, kBefore | bytes before the piece - 1, or an index (kHistory: in registers only).
 constexpr uint32_t kMatch = 0x8000u, kBefore = 0x8000u, kDone = 0x4000u, kHistory = 0x10000u;
 constexpr uint32_t kEndBlock = 1u << 30, kEndBad = 1u << 31, kEndFlags = kEndBlock | kEndBad;
 static_assert(kPiece <= kDone, "indices leave the flag bits free");
@@ -145,34 +146,6 @@ __device__ __forceinline__ uint32_t word_at(const uint32_t* a, uint64_t j, uint6
   if (endb - b0 < 32) v &= (1u << uint32_t(endb - b0)) - 1u;
   return v;
 }
-
-// LSB-first reader over the staged words.
-struct Bits {
-  const uint32_t* w;
-  uint64_t buf;
-  uint32_t cnt;
-  __device__ __forceinline__ Bits(const uint32_t* words, uint32_t bit) : w(words + (bit >> 5)) {
-    const uint32_t sh = bit & 31u;
-    buf = ((uint64_t(w[1]) << 32) | w[0]) >> sh;
-    cnt = 64 - sh;
-    w += 2;
-  }
-  __device__ __forceinline__ void refill() {  // at least 33 bits
-    if (cnt <= 32) {
-      buf |= uint64_t(*w++) << cnt;
-      cnt += 32;
-    }
-  }
-  __device__ __forceinline__ void skip(uint32_t n) {
-    buf >>= n;
-    cnt -= n;
-  }
-  __device__ __forceinline__ uint32_t take(uint32_t n) {  // n < 32, refilled
-    const uint32_t v = uint32_t(buf) & ((1u << n) - 1u);
-    skip(n);
-    return v;
-  }
-};
 
 // Table entry of the code at the low bits of `w`, one of more than `nbits` (at
 // least 11) bits or not assigned (then 0).
@@ -292,54 +265,68 @@ __device__ bool build_code(InfSmem& S, Canon& c, const uint8_t* lens, uint32_t n
 }
 
 // Reads a dynamic block's code lengths, from bit `at` of the staged words (all
-// threads; thread 0 decodes).  Returns false for an invalid header; S.used is
+// threads; the first warp decodes).  Returns false for an invalid header; S.used is
 // the bit after it.
 __device__ bool read_lengths(InfSmem& S, uint32_t at) {
-  const uint32_t tid = threadIdx.x;
-  if (tid < 19) S.lens[tid] = 0;
-  __syncthreads();
-  if (tid == 0) {
-    Bits b(S.words, at);
-    S.hlit = b.take(5) + 257;
-    S.hdist = b.take(5) + 1;
-    const uint32_t hclen = b.take(4) + 4;
-    at += 14 + 3 * hclen;
-    for (uint32_t i = 0; i < hclen; ++i) {
-      b.refill();
-      S.lens[c_cl_order[i]] = uint8_t(b.take(3));
-    }
-  }
-  __syncthreads();
-  const uint32_t hlit = S.hlit, hdist = S.hdist;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  auto bits_at = [&](uint32_t o) { return __funnelshift_r(S.words[o >> 5], S.words[(o >> 5) + 1], o & 31u); };
+  const uint32_t h = bits_at(at);
+  const uint32_t hlit = (h & 31u) + 257, hdist = ((h >> 5) & 31u) + 1, hclen = ((h >> 10) & 15u) + 4;
+  at += 14;
   if (hlit > 286 || hdist > 30) return false;
+  if (tid < 320) S.raw[tid] = 0;
+  if (tid < 19) S.lens[c_cl_order[tid]] = tid < hclen ? uint8_t(bits_at(at + 3 * tid) & 7u) : uint8_t(0);
+  at += 3 * hclen;
+  __syncthreads();
   if (!build_code(S, S.lc, S.lens, 19, S.lit, kClBits, kTabCl)) return false;
-  if (tid == 0) {
-    Bits b(S.words, at);
-    uint32_t i = 0, err = 0, prev = 0;
-    const uint32_t n = hlit + hdist;
+  if (tid < 32) {
+    const uint32_t n = hlit + hdist, lt = (1u << lane) - 1;
+    uint32_t i = 0, prev = 0, err = 0;
     while (i < n) {
-      b.refill();
-      const uint32_t e = S.lit[uint32_t(b.buf) & ((1u << kClBits) - 1)];  // every assigned code has at most 7 bits
-      if (!e) { err = 1; break; }
+      // lane: the symbol at bit at + lane, its bits and how many lengths it gives
+      const uint32_t w = bits_at(at + lane);
+      const uint32_t e = S.lit[w & ((1u << kClBits) - 1)];  // every assigned code has at most 7 bits
       const uint32_t cb = e & 15u, sym = e >> 16;
-      b.skip(cb);
-      at += cb;
-      if (sym < 16) {
-        prev = sym;
-        S.raw[i++] = uint8_t(sym);
-        continue;
+      const uint32_t xb = sym < 16 ? 0u : sym == 16 ? 2u : sym == 17 ? 3u : 7u;
+      const uint32_t rep = sym < 16 ? 1u : (sym == 18 ? 11u : 3u) + ((w >> cb) & ((1u << xb) - 1u));
+      const uint32_t nb = cb + xb;
+      // the symbols are the lanes reached from lane 0; one that is not a code
+      // or leads out leads to itself
+      uint32_t to = e && lane + nb < 32 ? lane + nb : lane, path = 1u << lane;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        path |= __shfl_sync(kAll, path, to);
+        to = __shfl_sync(kAll, to, to);
       }
-      const uint32_t xb = sym == 16 ? 2u : sym == 17 ? 3u : 7u;
-      const uint32_t rep = (sym == 18 ? 11u : 3u) + b.take(xb);
-      at += xb;
-      if (sym == 16 ? i == 0 : false) { err = 1; break; }
-      if (i + rep > n) { err = 1; break; }
-      if (sym != 16) prev = 0;
-      for (uint32_t k = 0; k < rep; ++k) S.raw[i + k] = uint8_t(prev);
-      i += rep;
+      path |= __shfl_sync(kAll, path, to);
+      const bool mine = (__shfl_sync(kAll, path, 0) >> lane) & 1u;
+      uint32_t incl = mine ? rep : 0u;
+#pragma unroll
+      for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t t = __shfl_up_sync(kAll, incl, k);
+        if (lane >= uint32_t(k)) incl += t;
+      }
+      const uint32_t first = i + incl - rep;  // index of the symbol's first length
+      const bool real = mine && first < n;
+      if (__any_sync(kAll, real && (!e || first + rep > n || (sym == 16 && first == 0)))) {
+        err = 1;
+        break;
+      }
+      const uint32_t set = __ballot_sync(kAll, real && sym != 16) & lt;  // symbols that give a value
+      uint32_t v = sym < 16 ? sym : 0u;
+      const uint32_t pv = __shfl_sync(kAll, v, set ? 31 - __clz(set) : 0);
+      if (sym == 16) v = set ? pv : prev;
+      if (real && v)  // the lengths are cleared
+        for (uint32_t k = 0; k < rep; ++k) S.raw[first + k] = uint8_t(v);
+      const uint32_t last = 31 - __clz(__ballot_sync(kAll, real));
+      prev = __shfl_sync(kAll, v, last);
+      i = __shfl_sync(kAll, first + rep, last);
+      at += __shfl_sync(kAll, lane + nb, last);
     }
-    S.bad = err;
-    S.used = at;
+    if (lane == 0) {
+      S.bad = err;
+      S.used = at;
+    }
   }
   __syncthreads();
   if (S.bad) return false;
@@ -574,7 +561,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
                 const uint32_t len = (tok[q] >> 16) & 0x1FFu;
                 if (at < b0 + n && at + len > b0) {  // a match cut by a piece's start goes on from there
                   const uint32_t j = max(at, b0) - b0;
-                  S.value[j] = uint16_t((tok[q] & 0x7FFFu) | (tok[q] >> 31) << 15);
+                  S.value[j] = uint16_t(tok[q] >> 31 ? kMatch | (tok[q] & 0x7FFFu) : kDone | (tok[q] & 0xFFu));
                   atomicOr(&S.bits[j >> 5], 1u << (j & 31));
                 }
                 at += len;
@@ -618,14 +605,15 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
                   s = j;
                   e = k & 1 ? cw[k / 2] >> 16 : cw[k / 2] & 0xFFFFu;
                 }
-                const uint32_t d = (e & 0x7FFFu) + 1;
-                uint32_t i = j - s;
+                int src = int(j) - 1 - int(e & 0x7FFFu);
                 // a match that overlaps itself repeats its first d bytes (the
                 // quotient is exact: it is below 258 and the half keeps it
                 // away from whole numbers)
-                if (i >= d && (e & kMatch)) i -= d * uint32_t(__fdividef(float(i) + 0.5f, float(d)));
-                const int src = int(s + i) - int(d);
-                const uint32_t x = !(e & kMatch) ? kDone | (e & 255u) : src >= 0 ? uint32_t(src) : kBefore | uint32_t(-1 - src);
+                if ((e & kMatch) && src >= int(s)) {
+                  const uint32_t i = j - s, d = (e & 0x7FFFu) + 1;
+                  src -= int(d * uint32_t(__fdividef(float(i) + 0.5f, float(d))));
+                }
+                const uint32_t x = !(e & kMatch) ? e : src >= 0 ? uint32_t(src) : kBefore | uint32_t(~src);
                 v[k / 2] = k & 1 ? v[k / 2] | (x << 16) : x;
               }
               uint4* o4 = reinterpret_cast<uint4*>(S.value) + 2 * tid;
