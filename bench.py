@@ -83,7 +83,7 @@ HBM_FALLBACK_GBS = 6650.0
 # this workload; every term of that traffic is per byte or per tile, so it is
 # scaled by the input size for the full launch (profiles/k_cand_parse_L1_mixed_300MB.md).
 DRAM_BYTES_PER_INPUT_BYTE = {"candidates": (759.450e6 + 703.093e6) / 301540590,
-                             "parse": (2088.913e6 + 1095.331e6) / 301540590}
+                             "parse": (2052.324e6 + 1119.271e6) / 301540590}
 
 
 def parse():
@@ -466,8 +466,8 @@ def measure_serving(deflate, buf, total, count, rate, cap_count, seed=0):
 # input byte, for the issue-rate roofline (4 warp instructions per SM cycle).
 # The "parse" phase is k_cand_parse, the candidate pass and the parse in one
 # kernel (the "candidates" phase is empty then).
-WARP_INST_PER_BYTE = {"candidates": 3.65, "parse": 12.07, "lazy_match": 77.4}
-PHASE_KERNEL = {"candidates": "k_cand", "parse": "k_cand_parse",  "lazy_match": "k_search", "lazy_encode": "k_enc", "lazy_huffman": "k_huff",
+WARP_INST_PER_BYTE = {"candidates": 3.36, "parse": 10.6, "lazy_match": 48.0}
+PHASE_KERNEL = {"candidates": "k_cand", "parse": "k_cand_parse",  "lazy_match": "k_link + k_search + k_lparse", "lazy_encode": "k_enc", "lazy_huffman": "k_huff",
                 "hash_carry": "k_lastocc + k_carry_scan", "fixup": "k_fix1 + k_fix2 + k_fix3", "join": "k_join",
                 "checksum": "k_ck_block + k_ck_fold", "plan": "k_plan"}
 

@@ -236,7 +236,7 @@ size_t deflate_gpu_compress_gzip_members(const void* in, size_t in_size, int lev
                                          size_t out_capacity);
 
 /* On-device verification of the last run of a batch (no counterpart in the
- * reference): every stream is decoded on the GPU (one warp per stream),
+ * reference): every stream is decoded on the GPU (one CTA per stream),
  * compared byte for byte with its input, and its framing and trailer are
  * checked.  ok[i] = 1 for a stream that round-trips.  Returns the number of
  * streams that failed, or -1. */

@@ -125,7 +125,7 @@ struct InflateJob {
   uint32_t pad;
 };
 constexpr int32_t kInfOk = 0, kInfData = 1, kInfOutput = 2, kInfInput = 3, kInfMismatch = 4;
-// Decodes jobs[order[0..n)] (one warp per stream; the input and output
+// Decodes jobs[order[0..n)] (one CTA per stream; the input and output
 // buffers carry at least 8 bytes of padding); `counter` is a device word.
 void launch_inflate(const uint8_t* in, uint8_t* out, InflateJob* jobs, const uint32_t* order, uint32_t njobs,
                     uint32_t* counter, int sms, cudaStream_t st);
