@@ -41,10 +41,11 @@
 // the CTA is as large as can be and parts are short.  1 MiB streams of zlib
 // level 6 on a B200, against one warp per stream that decoded 64 bit offsets
 // at a time and followed the tokens one by one (whole deflate_decompress call,
-// ms): text 67.5 -> 1.9, integers (39 blocks) 3.8, 8-byte periods 1.0, zeros 1.0.
+// ms): text 67.5 -> 1.9, integers (39 blocks) 3.7, 8-byte periods 1.0, zeros 0.9.
 // One exit test per token and 16 consecutive bytes a thread when bytes are
 // coded took the text from 2.14 to 2.03, indices reduced only where a match
-// overlaps itself to 1.97, code lengths read by a warp to 1.94.
+// overlaps itself to 1.97, code lengths read by a warp to 1.94, tables filled by
+// comparing with the ends of the lengths' ranges (held in registers) to 1.92.
 // 512 threads with parts of 480 bits take 2.7 on the text, 1024 threads with
 // parts of 480 bits 2.2.
 //
@@ -247,18 +248,17 @@ __device__ bool build_code(InfSmem& S, Canon& c, const uint8_t* lens, uint32_t n
     c.sym[c.offs[len] + r] = uint16_t(tid);
   }
   __syncthreads();
-  // every index finds its code: codes are sent most significant bit first
+  // every index finds its code: codes are sent most significant bit first, and
+  // a code is below the end of its length's range and of no shorter one's
+  uint32_t end[kLitBits];
+#pragma unroll
+  for (uint32_t l = 0; l < kLitBits; ++l) end[l] = l < nbits ? c.end[l + 1] : 0u;
   for (uint32_t i = tid; i < (1u << nbits); i += kInfThreads) {
-    uint32_t e = 0, code = 0;
-    for (uint32_t l = 1; l <= nbits; ++l) {
-      code = (code << 1) | ((i >> (l - 1)) & 1u);
-      const uint32_t k = code - c.first[l];
-      if (k < c.count[l]) {
-        e = make_entry(tab, c.sym[c.offs[l] + k], l);
-        break;
-      }
-    }
-    table[i] = e;
+    const uint32_t code = __brev(i) >> 17;
+    uint32_t l = 1;
+#pragma unroll
+    for (uint32_t k = 0; k < kLitBits; ++k) l += k < nbits && code >= end[k] ? 1u : 0u;
+    table[i] = l <= nbits ? make_entry(tab, c.sym[(code >> (15 - l)) - c.first[l] + c.offs[l]], l) : 0u;
   }
   __syncthreads();
   return true;
