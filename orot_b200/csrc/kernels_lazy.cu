@@ -152,7 +152,9 @@ __device__ __forceinline__ uint32_t same_bits(uint32_t h, uint32_t among) {
 //
 // This replaces the ordered pass of one warp over all chunks of a tile inside
 // the search kernel: 30% of that kernel on mixed data, with 31 warps idle.
-// Bound by instruction issue (the ballots) and four barriers per round.
+// Bound by instruction issue (the ballots) and four barriers per round.  64 MiB
+// of mixed data in 128 KiB blocks 1249 us with ten ballots per 32 entries of a
+// list, 1124 with a lane number read back from the table.
 namespace {
 constexpr uint32_t kLkRound = 4096;             // positions per round: 128 chunks
 constexpr uint32_t kLkChunks = kLkRound / 32;
@@ -326,13 +328,22 @@ __global__ void __launch_bounds__(1024, 1) k_link(Work wk, const uint32_t* __res
         const uint32_t x = q0 + (e & 0xFFFu), xl = q0 + (e >> 12);
         const uint32_t v = rb.load4(x);
         const uint32_t h = hash15(v) & 1023u;
-        const uint32_t peers = same_bits<10>(h, __ballot_sync(kAll, valid));
-        const uint32_t before = valid ? peers & lt : 0u;
-        const uint32_t pl = __shfl_sync(kAll, xl, before ? 31 - __clz(before) : lane);
-        uint32_t p = pl + 1;  // previous position + 1
-        if (valid && !before) p = tb[h];
+        // What the table holds, then a lane number in its place: entries of one
+        // hash read back the same one, whose bits tell them apart.
+        uint32_t p = valid ? tb[h] : 0u;  // previous position + 1
         __syncwarp();
-        if (valid && (peers >> lane) == 1u) tb[h] = xl + 1;
+        if (valid) tb[h] = lane;
+        __syncwarp();
+        const uint32_t who = valid ? tb[h] : lane;
+        bool last = valid;
+        if (__any_sync(kAll, who != lane)) {
+          const uint32_t peers = same_bits<5>(who, __ballot_sync(kAll, valid));
+          const uint32_t before = valid ? peers & lt : 0u;
+          const uint32_t pl = __shfl_sync(kAll, xl, before ? 31 - __clz(before) : lane);
+          if (before) p = pl + 1;
+          last = valid && (peers >> lane) == 1u;
+        }
+        if (last) tb[h] = xl + 1;
         __syncwarp();
         if (valid && p && x + 1 - p <= kMaxDist)
           S.out[e & 0xFFFu] = uint16_t((x + 1 - p) | (rb.load4(p - 1) == v ? 0u : kLinkDiff));
