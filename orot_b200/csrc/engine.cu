@@ -189,29 +189,36 @@ static const GeometryRow& geometry_row(uint64_t total_bytes, int sms) {
 
 const GeometryRow& Engine::geometry(uint64_t total_bytes) const { return geometry_row(total_bytes, sms); }
 
-// Passes of a few MiB are bound by the time one warp needs for a tile (about
-// 25 us for 1 KiB, once to find candidates and once to parse; 16 tables and as
-// many parsers per SM, 4 and 20 at 14 hash bits), so they are cut finer than
-// the table's smallest tile, down to 512 bytes (shorter tiles cannot be crossed
-// as parts of a long run, see run_tile): about 1,024 tiles or more at 12 hash
-// bits and 512 at 14, whose tables are four times as large; 2,048 tiles of 2 KiB
-// at 12 bits before 4 KiB tiles pay.  Mean over five kinds of data (us),
-// 512 / 1024 / 2048 / 4096:
+// Tile bytes of a pass: the table's, but passes of a few MiB are bound by the
+// time one warp needs for a tile (about 25 us for 1 KiB, once to find candidates
+// and once to parse; 16 tables and as many parsers per SM, 4 and 20 at 14 hash
+// bits), so they are cut finer than the table's smallest tile, down to 512 bytes
+// (shorter tiles cannot be crossed as parts of a long run, see run_tile).  A tile
+// is doubled while the pass still has as many of it as pay: 2,048 at 12 hash
+// bits and 4,096 of the 2 KiB ones, 768 at 14, whose tables are four times as
+// large.  Mean over five kinds of data (us), 512 / 1024 / 2048 / 4096:
 //   12 bits:  4 KiB  74 /  87 / 110 / 157   512 KiB 123 / 129 / 156 / 227
 //             1 MiB 169 / 145 / 169 / 237     2 MiB 266 / 191 / 185 / 245
 //             4 MiB 506 / 299 / 231 / 266     8 MiB 924 / 562 / 367 / 314
 //   14 bits: 32 KiB  91 / 102 / 122 / 174   512 KiB 161 / 138 / 151 / 209
 //             1 MiB 314 / 183 / 173 / 218     2 MiB 542 / 335 / 226 / 240
 //             4 MiB 989 / 576 / 386 / 303
-uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
-  if (tile_override) return tile_override;
-  const GeometryRow& g = geometry(total_bytes);
+// An empty pass has nothing to cut.
+static uint32_t plan_tile(uint64_t total_bytes, int sms, int hash_bits) {
+  const GeometryRow& g = geometry_row(total_bytes, sms);
   const uint32_t most = hash_bits <= 12 ? g.tile12 : g.tile14;
+  if (!total_bytes) return most;
   const uint64_t scaled = total_bytes * 148u / uint64_t(std::max(sms, 1));
-  const uint64_t tiles = hash_bits <= 12 ? 2048 : 768;
   uint32_t t = 512;
-  while (t < most && t * (hash_bits <= 12 && t == 2048 ? 2 * tiles : tiles) <= scaled) t *= 2;
+  while (t < most) {
+    const uint64_t tiles = (scaled + t - 1) / t;
+    if (tiles < (hash_bits > 12 ? 768u : t == 2048 ? 4096u : 2048u)) break;
+    t *= 2;
+  }
   return t;
+}
+uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
+  return tile_override ? tile_override : plan_tile(total_bytes, sms, hash_bits);
 }
 
 template <class T>
@@ -847,8 +854,7 @@ const char* orot_b200_last_error(void) { return g_err.c_str(); }
 const char* orot_b200_geometry_source(void) { return kGeometrySource; }
 
 uint32_t orot_b200_geometry_tile(uint64_t pass_bytes, int sms, int hash_bits) {
-  const GeometryRow& g = geometry_row(pass_bytes, sms);
-  return hash_bits <= 12 ? g.tile12 : g.tile14;
+  return plan_tile(pass_bytes, sms, hash_bits);
 }
 
 }  // extern "C"
