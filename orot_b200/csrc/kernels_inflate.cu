@@ -9,12 +9,15 @@
 //            one per thread.  Every thread decodes its part from a guessed
 //            start (the part's first bit) to the first token that starts
 //            beyond it, marking the token starts in a bitmap.  Huffman codes
-//            synchronise themselves: after a few tokens a wrong start leads to
-//            the same token starts as the right one.  Then each thread compares
-//            its start with the end its left neighbour found and, if they
-//            differ, decodes again until it meets a token start it had marked,
-//            until no thread's start changes; the first part's start is right,
-//            so then all are.
+//            mostly synchronise themselves: after a few tokens a wrong start
+//            leads to the same token starts as the right one.  Then each thread
+//            compares its start with the end its left neighbour found and, if
+//            they differ, decodes again until it meets a token start it had
+//            marked, until no thread's start changes; the first part's start is
+//            right, so then all are.  Where all codes have one length that does
+//            not divide a part, a wrong start stays wrong and the right one moves
+//            on by a part a round (1 MiB of literals in codes of 7 bits: 16 ms,
+//            in codes of 8 bits 0.4).
 //   tokens   The bitmap's tokens are dealt out evenly and decoded independently
 //            (kBatch at a time); output offsets come from a scan of their
 //            lengths.
@@ -48,6 +51,11 @@
 // comparing with the ends of the lengths' ranges (held in registers) to 1.92.
 // 512 threads with parts of 480 bits take 2.7 on the text, 1024 threads with
 // parts of 480 bits 2.2.
+// A stream of short blocks pays for each block, not for what lies behind it:
+// words stay staged, the fixed code's tables stay, and the first window of a
+// block is about twice the block before (1 MiB of text in blocks of 100 bytes
+// each behind a flush: 717 ms with whole windows staged and decoded, now 360;
+// with the fixed code 437 and 189; one warp per stream took 489 and 324).
 //
 // The kernel does not read the zlib / gzip framing; the host strips it and
 // checks the trailer against a checksum of the output (src/formats/*:
@@ -69,6 +77,10 @@ constexpr int kInfThreads = 1024;      // one CTA per SM
 constexpr uint32_t kParts = kInfThreads, kPartBits = 9 * 32;
 constexpr uint32_t kMapWords = kParts * kPartBits / 32;
 constexpr uint32_t kWindowWords = kMapWords + 6;  // with the bits a last token reaches past the window
+constexpr uint32_t kOverBits = 48 + 96;           // a token, and what is loaded for the one behind it
+constexpr uint32_t kHeaderBits = 4608 + 96;       // a dynamic block's header (3 + 14 + 19 * 3 + 316 * 14), and the same
+static_assert(kParts * kPartBits + kOverBits + 31 <= kWindowWords * 32 && kHeaderBits + 31 <= kWindowWords * 32,
+              "a window fits from any bit of its first word");
 constexpr uint32_t kBatch = 8 * kInfThreads;      // tokens decoded at once
 constexpr uint32_t kPiece = 16 * kInfThreads;      // output bytes expanded at once
 constexpr int kLitBits = 12, kDistBits = 11, kClBits = 7;  // table index bits
@@ -345,6 +357,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
   extern __shared__ __align__(16) uint8_t inf_smem[];
   InfSmem& S = *reinterpret_cast<InfSmem*>(inf_smem);
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  bool fixed_tables = false;  // the tables are those of the fixed code
   for (;;) {
     __syncthreads();
     if (tid == 0) S.job = atomicAdd(counter, 1u);
@@ -362,18 +375,25 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
     uint64_t op = 0;  // output position
     int32_t status = kInfOk;
     bool last = false;
-    // stages the words from bit P on; returns the bit of P in the first one
-    auto stage = [&]() -> uint32_t {
+    uint64_t sq = uint64_t(1) << 63;  // the first staged word (none)
+    uint32_t first_parts = kParts;  // parts in the first window of a block
+    // stages the words from bit P on unless `bits` from there are staged;
+    // returns the bit of P in the staged words
+    auto stage = [&](uint32_t bits) -> uint32_t {
       const uint64_t q = (s0 + P) >> 5;
+      const uint32_t r = uint32_t((s0 + P) & 31u);
       __syncthreads();  // the words staged before are no longer read
+      if (q - sq < kWindowWords && uint32_t(q - sq) * 32 + r + bits <= kWindowWords * 32)
+        return uint32_t(q - sq) * 32 + r;
+      sq = q;
       for (uint32_t k = tid; k < kWindowWords; k += kInfThreads) S.words[k] = word_at(aw, q + k, endb);
       __syncthreads();
-      return uint32_t((s0 + P) & 31u);
+      return r;
     };
     while (!last && status == kInfOk) {
       if (s0 + P + 3 > endb) { status = kInfInput; break; }
-      const uint32_t r = stage();
-      const uint32_t hdr = (S.words[0] >> r) | (r > 29 ? S.words[1] << (32 - r) : 0u);
+      const uint32_t r = stage(kHeaderBits);
+      const uint32_t hdr = __funnelshift_r(S.words[r >> 5], S.words[(r >> 5) + 1], r & 31u);
       last = hdr & 1u;
       const uint32_t type = (hdr >> 1) & 3u;
       if (type == 3) { status = kInfData; break; }
@@ -393,28 +413,36 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
       }
       uint32_t used = r + 3;
       if (type == 1) {
-        if (tid < 320) S.lens[tid] = tid < 144 ? 8 : tid < 256 ? 9 : tid < 280 ? 7 : tid < 288 ? 8 : 5;
-        __syncthreads();
+        if (!fixed_tables) {
+          if (tid < 320) S.lens[tid] = tid < 144 ? 8 : tid < 256 ? 9 : tid < 280 ? 7 : tid < 288 ? 8 : 5;
+          __syncthreads();
+        }
       } else {
+        fixed_tables = false;
         if (!read_lengths(S, used)) { status = kInfData; break; }
         used = S.used;
       }
-      if (!build_code(S, S.lc, S.lens, 288, S.lit, kLitBits, kTabLit) ||
-          !build_code(S, S.dc, S.lens + 288, 30, S.dist, kDistBits, kTabDist)) {
+      if (!fixed_tables && (!build_code(S, S.lc, S.lens, 288, S.lit, kLitBits, kTabLit) ||
+                            !build_code(S, S.dc, S.lens + 288, 30, S.dist, kDistBits, kTabDist))) {
         status = kInfData;
         break;
       }
+      fixed_tables = type == 1;
       P += used - r;
+      // What lies behind the block is decoded for nothing, so the window of a
+      // block behind a short one starts at about twice that one's size.
+      const uint64_t block_at = P;
+      uint32_t parts = first_parts;
 
       bool block_end = false;
       while (!block_end) {
         if (s0 + P >= endb) { status = kInfInput; break; }
-        const uint32_t r0 = stage();
+        const uint32_t r0 = stage(parts * kPartBits + kOverBits);
         const uint64_t left = endb - (s0 + P);
         const uint32_t rem = left > (1u << 20) ? 1u << 20 : uint32_t(left);  // bits left, more than a window if capped
         // -- synchronisation
         const uint32_t limit = min(rem, (tid + 1) * kPartBits);  // tokens from here on are the next part's
-        const bool active = tid < kParts && tid * kPartBits < rem;
+        const bool active = tid < parts && tid * kPartBits < rem;
         uint32_t begin = tid * kPartBits;  // where this part's first token starts, as far as known
         // One test per token ends the inner loop; what it was is found behind it,
         // so that a token is little more than its chain of lookups.
@@ -482,7 +510,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
           }
         }
         // -- the parts up to the first that met an end count
-        if (tid == 0) S.stop = min(kParts, (rem + kPartBits - 1) / kPartBits) - 1;
+        if (tid == 0) S.stop = min(parts, (rem + kPartBits - 1) / kPartBits) - 1;
         __syncthreads();
         if (active && (S.end[tid] & kEndFlags)) atomicMin(&S.stop, tid);
         __syncthreads();
@@ -494,6 +522,8 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
         }
         block_end = (stop_end & kEndBlock) != 0;
         P += stop_end & ~kEndFlags;
+        parts = kParts;
+        if (block_end) first_parts = uint32_t(min(uint64_t(kParts), (P - block_at) / (kPartBits / 2) + 4));
 
         // -- tokens, a batch at a time
         constexpr uint32_t kPartWords = kPartBits / 32;
