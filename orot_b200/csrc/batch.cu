@@ -321,7 +321,9 @@ int deflate_gpu_batch_verify(deflate_gpu_batch* b, int* ok) {
     return -1;
   }
   uint8_t* dec = static_cast<uint8_t*>(b->d_verify.p);
-  launch_inflate(static_cast<const uint8_t*>(e.d_out.p), dec, d_jobs, d_order, uint32_t(order.size()), d_cnt, e.sms, st);
+  const uint32_t nj = uint32_t(order.size());
+  launch_inflate(static_cast<const uint8_t*>(e.d_out.p), dec, d_jobs, d_order, nj,
+                 large_streams(jobs.data(), order.data(), nj, e.sms), d_cnt, e.sms, st);
   launch_inflate_compare(dec, static_cast<const uint8_t*>(e.d_in.p), d_jobs, d_roff, d_rlen, uint32_t(n), st);
   launch_frame_check(static_cast<const uint8_t*>(e.d_out.p),
                      reinterpret_cast<const Stream*>(static_cast<uint8_t*>(e.d_tables.p) + e.off_streams), d_jobs,

@@ -76,7 +76,7 @@ static bool decode_raw(Engine& e, const uint8_t* raw, size_t len, size_t out_off
   uint8_t* dt = static_cast<uint8_t*>(e.d_tables.p);
   InflateJob* d_job = reinterpret_cast<InflateJob*>(dt);
   uint32_t* d_order = reinterpret_cast<uint32_t*>(dt + align_up(sizeof(InflateJob), 256));
-  uint32_t* d_counter = d_order + 1;
+  uint32_t* d_counters = d_order + 1;
   *job = InflateJob{};
   job->in_len = len;
   job->out_off = out_off;
@@ -88,8 +88,8 @@ static bool decode_raw(Engine& e, const uint8_t* raw, size_t len, size_t out_off
     set_error("H2D failed");
     return false;
   }
-  launch_inflate(static_cast<const uint8_t*>(e.d_in.p), static_cast<uint8_t*>(e.d_out.p), d_job, d_order, 1,
-                 d_counter, e.sms, e.stream);
+  launch_inflate(static_cast<const uint8_t*>(e.d_in.p), static_cast<uint8_t*>(e.d_out.p), d_job, d_order, 1, 1,
+                 d_counters, e.sms, e.stream);
   if (cudaMemcpyAsync(job, d_job, sizeof *job, cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
       cudaStreamSynchronize(e.stream) != cudaSuccess) {
     set_error(std::string("device error: ") + cudaGetErrorString(cudaGetLastError()));

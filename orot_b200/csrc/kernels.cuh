@@ -125,10 +125,30 @@ struct InflateJob {
   uint32_t pad;
 };
 constexpr int32_t kInfOk = 0, kInfData = 1, kInfOutput = 2, kInfInput = 3, kInfMismatch = 4;
-// Decodes jobs[order[0..n)] (one CTA per stream; the input and output
-// buffers carry at least 8 bytes of padding); `counter` is a device word.
+// How many of the streams order[0..n) (by decreasing in_len) are decoded by large
+// CTAs, one per SM; the others by small ones, eight per SM, which pay where a
+// large one would wait for the same dozens of steps whatever the stream's length: for
+// short streams, the longer the more rounds of large CTAs they would take, and
+// most of the streams, since the small CTAs start after the large ones.
+// deflate_gpu_batch_verify of zlib level-6-like text (us), all large / small / with
+// the one warp per stream that went before: 300 of 100 to 200 bytes 186 / 134 / 167,
+// 10,000 of them 4300 / 2080 / 2090, 10,000 of 1 to 4 KiB 5200 / 2580 / 3400, 450 of 1
+// to 4 KiB 338 / 329 / 507, 1,000 of 32 to 64 KiB 1560 / 1560 / 5340.
+inline uint32_t large_streams(const InflateJob* jobs, const uint32_t* order, uint32_t n, int sms) {
+  auto shorter = [&](uint64_t len) {
+    uint32_t k = 0;
+    while (k < n && jobs[order[n - 1 - k]].in_len < len) ++k;
+    return k;
+  };
+  const uint64_t rounds = shorter(4096) / uint32_t(sms);
+  const uint32_t small = shorter(rounds < 16 ? 256 * rounds : 4096);
+  return small > uint32_t(sms) && small > n / 2 ? n - small : n;
+}
+// Decodes jobs[order[0..n)] (one CTA per stream, a large one for the first nlarge;
+// the input and output buffers carry at least 8 bytes of padding); `counters` are
+// two device words.
 void launch_inflate(const uint8_t* in, uint8_t* out, InflateJob* jobs, const uint32_t* order, uint32_t njobs,
-                    uint32_t* counter, int sms, cudaStream_t st);
+                    uint32_t nlarge, uint32_t* counters, int sms, cudaStream_t st);
 // Marks kInfMismatch on streams whose framing or trailer is wrong (job i is stream i).
 void launch_frame_check(const uint8_t* out, const Stream* streams, InflateJob* jobs, uint32_t n, cudaStream_t st);
 // Marks kInfMismatch on jobs whose decoded bytes differ from ref[ref_off[j], + ref_len[j]).

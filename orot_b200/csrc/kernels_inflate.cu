@@ -3,7 +3,8 @@
 // Decoding a DEFLATE stream is sequential by its definition: a code's length
 // is known only after the code before it is decoded, and a match copies bytes
 // that earlier tokens produced.  One CTA decodes one stream (CTAs take streams
-// from a counter, largest first), and both chains are broken up inside it:
+// from a counter, largest first; many short streams go to small CTAs), and both
+// chains are broken up inside it:
 //
 //   synchronisation  A window of the stream is cut into parts of kPartBits,
 //            one per thread.  Every thread decodes its part from a guessed
@@ -30,8 +31,8 @@
 //            until all are bytes: as many rounds as the logarithm of the
 //            longest chain of matches that copy from matches.
 //
-// Tables are looked up by 12 bits (literal/length) and 11 (distance); their entries carry all a token needs (code
-// bits, base value, extra bits).  Longer codes are resolved by the canonical
+// Tables are looked up by 12 bits (literal/length) and 11 (distance), 10 and 8 in small CTAs; their
+// entries carry all a token needs (code bits, base value, extra bits).  Longer codes are resolved by the canonical
 // rule of RFC 1951 3.2.2 (codes of one length are consecutive integers and
 // shorter codes precede longer ones): left-aligned, a code is below the end of
 // its length's range and of no shorter one's.
@@ -71,19 +72,28 @@ namespace orotb {
 namespace {
 
 constexpr uint32_t kAll = 0xFFFFFFFFu;
-constexpr int kInfThreads = 1024;      // one CTA per SM
-// Parts of the stream per window, decoded by a thread each.  An odd number of
-// words: threads at the same place of their parts read different banks.
-constexpr uint32_t kParts = kInfThreads, kPartBits = 9 * 32;
-constexpr uint32_t kMapWords = kParts * kPartBits / 32;
-constexpr uint32_t kWindowWords = kMapWords + 6;  // with the bits a last token reaches past the window
+// A CTA of N threads, with tables looked up by LIT and DIST bits.
+template <int N, int LIT, int DIST>
+struct Inf {
+  static constexpr uint32_t kThreads = N;
+  // Parts of the stream per window, decoded by a thread each.  An odd number of
+  // words: threads at the same place of their parts read different banks.
+  static constexpr uint32_t kParts = N, kPartBits = 9 * 32;
+  static constexpr uint32_t kMapWords = kParts * kPartBits / 32;
+  static constexpr uint32_t kWindowWords = kMapWords + 6;  // with the bits a last token reaches past the window
+  static constexpr uint32_t kBatch = 8 * N;                // tokens decoded at once
+  static constexpr uint32_t kPiece = 16 * N;               // output bytes expanded at once
+  static constexpr int kLitBits = LIT, kDistBits = DIST;   // table index bits
+};
+using InfLarge = Inf<1024, 12, 11>;  // one CTA per SM
+// For many short streams (large_streams): 22 KB, eight CTAs per SM by their
+// registers.  10,000 streams of 100 bytes / of 1 to 4 KiB verified, with 128
+// threads and 10 + 8 bits 2.08 / 2.58 ms, 11 + 9 bits 2.13 / 2.63, 256 threads 2.28 /
+// 2.76, 64 threads and 9 + 8 bits 2.03 / 2.60 (and 35% slower on streams of 64 KiB).
+using InfSmall = Inf<128, 10, 8>;
 constexpr uint32_t kOverBits = 48 + 96;           // a token, and what is loaded for the one behind it
 constexpr uint32_t kHeaderBits = 4608 + 96;       // a dynamic block's header (3 + 14 + 19 * 3 + 316 * 14), and the same
-static_assert(kParts * kPartBits + kOverBits + 31 <= kWindowWords * 32 && kHeaderBits + 31 <= kWindowWords * 32,
-              "a window fits from any bit of its first word");
-constexpr uint32_t kBatch = 8 * kInfThreads;      // tokens decoded at once
-constexpr uint32_t kPiece = 16 * kInfThreads;      // output bytes expanded at once
-constexpr int kLitBits = 12, kDistBits = 11, kClBits = 7;  // table index bits
+constexpr int kClBits = 7;                        // table index bits of the code-length code
 
 // order of the code-length code lengths in a dynamic block header (3.2.7)
 __constant__ uint8_t c_cl_order[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
@@ -125,30 +135,33 @@ struct Canon {
   uint16_t sym[288];
 };
 
+template <class C>
 struct InfSmem {
-  uint32_t lit[1 << kLitBits], dist[1 << kDistBits];  // the lit table holds the code-length code first
-  uint32_t words[kWindowWords];        // the stream from the window's first word
-  alignas(16) uint32_t map[kMapWords];  // token starts, by bit of the window
+  uint32_t lit[1 << C::kLitBits], dist[1 << C::kDistBits];  // the lit table holds the code-length code first
+  uint32_t words[C::kWindowWords];         // the stream from the window's first word
+  alignas(16) uint32_t map[C::kMapWords];  // token starts, by bit of the window
   union alignas(16) {
-    uint32_t list[kBatch];  // bit positions of a batch's tokens
+    uint32_t list[C::kBatch];  // bit positions of a batch's tokens
     // a piece's bytes: at a token's first byte its code, then the codes below
-    uint16_t value[kPiece];
+    uint16_t value[C::kPiece];
   };
-  uint32_t bits[kPiece / 32];        // first bytes of tokens
-  uint16_t last[kPiece / 32];        // the last first byte before each bitmap word
-  uint32_t end[kParts];              // where a part's last token ends, from the window's first bit | flags
-  uint32_t scan[kInfThreads / 32];
+  uint32_t bits[C::kPiece / 32];     // first bytes of tokens
+  uint16_t last[C::kPiece / 32];     // the last first byte before each bitmap word
+  uint32_t end[C::kParts];           // where a part's last token ends, from the window's first bit | flags
+  uint32_t scan[C::kThreads / 32];
   Canon lc, dc;
   uint32_t groups[10][16];           // build: codes of each length per 32 symbols
   uint8_t lens[320], raw[320];       // code lengths: literal/length at 0, distance at 288; as read
   uint32_t job, type, bad, used, stop;
+  static_assert(C::kParts * C::kPartBits + kOverBits + 31 <= C::kWindowWords * 32 && kHeaderBits + 31 <= C::kWindowWords * 32,
+                "a window fits from any bit of its first word");
 };
 // Codes of a piece's bytes: at a token's start kDone | literal or kMatch |
 // distance - 1; then kDone | byte, kBefore | bytes before the piece - 1, or an index (kHistory: in registers only).
 constexpr uint32_t kMatch = 0x8000u, kBefore = 0x8000u, kDone = 0x4000u, kHistory = 0x10000u;
 constexpr uint32_t kEndBlock = 1u << 30, kEndBad = 1u << 31, kEndFlags = kEndBlock | kEndBad;
-static_assert(kPiece <= kDone, "indices leave the flag bits free");
-static_assert(sizeof(InfSmem) <= 227 * 1024, "one CTA per SM");
+static_assert(InfLarge::kPiece <= kDone, "indices leave the flag bits free");
+static_assert(sizeof(InfSmem<InfLarge>) <= 227 * 1024, "one CTA per SM");
 
 // Aligned input word j of a stream whose last bit is at absolute bit `endb`
 // (bits at or past it read as zero).
@@ -160,8 +173,8 @@ __device__ __forceinline__ uint32_t word_at(const uint32_t* a, uint64_t j, uint6
   return v;
 }
 
-// Table entry of the code at the low bits of `w`, one of more than `nbits` (at
-// least 11) bits or not assigned (then 0).
+// Table entry of the code at the low bits of `w`, one of more than `nbits` bits
+// or not assigned (then 0).
 __device__ __forceinline__ uint32_t long_code(const Canon& c, uint32_t w, uint32_t nbits, uint32_t tab) {
   const uint32_t code = __brev(w) >> 17;  // 15 bits, first bit on top
   for (uint32_t l = nbits + 1; l < 16; ++l)
@@ -173,8 +186,10 @@ __device__ __forceinline__ uint32_t long_code(const Canon& c, uint32_t w, uint32
 // end of block, 3 invalid), with the literal or length in `len` and the
 // distance in `dist`; returns its bits.  Both lookups are made for every kind,
 // so that lanes with literals and with matches stay together.
-__device__ __forceinline__ uint32_t token_at(const InfSmem& S, uint32_t at, uint32_t& kind, uint32_t& len,
+template <class C>
+__device__ __forceinline__ uint32_t token_at(const InfSmem<C>& S, uint32_t at, uint32_t& kind, uint32_t& len,
                                              uint32_t& dist) {
+  constexpr int kLitBits = C::kLitBits, kDistBits = C::kDistBits;
   const uint32_t* sw = S.words + (at >> 5);
   const uint32_t x0 = sw[0], x1 = sw[1], x2 = sw[2];
   const uint32_t w = __funnelshift_r(x0, x1, at & 31u), whi = __funnelshift_r(x1, x2, at & 31u);
@@ -196,7 +211,8 @@ __device__ __forceinline__ uint32_t token_at(const InfSmem& S, uint32_t at, uint
 
 // Exclusive scan over the CTA of `v`; the sum over all threads in `total`.
 // Every thread calls it; the CTA has passed a barrier since the last call.
-__device__ __forceinline__ uint32_t cta_scan(InfSmem& S, uint32_t v, uint32_t& total) {
+template <class C>
+__device__ __forceinline__ uint32_t cta_scan(InfSmem<C>& S, uint32_t v, uint32_t& total) {
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t incl = v;
 #pragma unroll
@@ -206,7 +222,7 @@ __device__ __forceinline__ uint32_t cta_scan(InfSmem& S, uint32_t v, uint32_t& t
   }
   if (lane == 31) S.scan[wid] = incl;
   __syncthreads();
-  const uint32_t w = lane < kInfThreads / 32 ? S.scan[lane] : 0u;
+  const uint32_t w = lane < C::kThreads / 32 ? S.scan[lane] : 0u;
   const uint32_t below = __reduce_add_sync(kAll, lane < wid ? w : 0u);
   total = __reduce_add_sync(kAll, w);
   return below + incl - v;
@@ -216,20 +232,27 @@ __device__ __forceinline__ uint32_t cta_scan(InfSmem& S, uint32_t v, uint32_t& t
 // code lengths lens[0..n), n <= 320 (all threads).  Returns false for an
 // over-subscribed set of lengths; an incomplete set is accepted (a code that
 // is not assigned is reported when it is read).
-__device__ bool build_code(InfSmem& S, Canon& c, const uint8_t* lens, uint32_t n, uint32_t* table, uint32_t nbits,
+template <class C>
+__device__ bool build_code(InfSmem<C>& S, Canon& c, const uint8_t* lens, uint32_t n, uint32_t* table, uint32_t nbits,
                            uint32_t tab) {
-  const uint32_t tid = threadIdx.x, lane = tid & 31, g = tid >> 5;
-  const uint32_t len = tid < n ? lens[tid] : 0u;
-  if (tid < 160) S.groups[tid >> 4][tid & 15] = 0;
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  constexpr uint32_t N = C::kThreads, K = (320 + N - 1) / N;  // symbols of a thread
+  uint32_t len[K], before[K];
+  for (uint32_t i = tid; i < 160; i += N) S.groups[i >> 4][i & 15] = 0;
   __syncthreads();
-  uint32_t peers = kAll;  // lanes of the same length
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t bal = __ballot_sync(kAll, (len >> k) & 1u);
-    peers &= (len >> k) & 1u ? bal : ~bal;
+  for (uint32_t j = 0; j < K; ++j) {
+    const uint32_t s = tid + j * N;
+    len[j] = s < n ? lens[s] : 0u;
+    uint32_t peers = kAll;  // lanes of the same length
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t bal = __ballot_sync(kAll, (len[j] >> k) & 1u);
+      peers &= (len[j] >> k) & 1u ? bal : ~bal;
+    }
+    before[j] = __popc(peers & ((1u << lane) - 1));
+    if (len[j] && !before[j]) S.groups[s >> 5][len[j]] = __popc(peers);
   }
-  const uint32_t before = __popc(peers & ((1u << lane) - 1));
-  if (len && !before) S.groups[g][len] = __popc(peers);
   __syncthreads();
   if (tid < 16) {
     uint32_t sum = 0;
@@ -254,18 +277,22 @@ __device__ bool build_code(InfSmem& S, Canon& c, const uint8_t* lens, uint32_t n
   }
   __syncthreads();
   if (S.bad) return false;
-  if (len) {
-    uint32_t r = before;
-    for (uint32_t k = 0; k < g; ++k) r += S.groups[k][len];
-    c.sym[c.offs[len] + r] = uint16_t(tid);
+#pragma unroll
+  for (uint32_t j = 0; j < K; ++j) {
+    if (!len[j]) continue;
+    const uint32_t s = tid + j * N;
+    uint32_t r = before[j];
+    for (uint32_t k = 0; k < s >> 5; ++k) r += S.groups[k][len[j]];
+    c.sym[c.offs[len[j]] + r] = uint16_t(s);
   }
   __syncthreads();
   // every index finds its code: codes are sent most significant bit first, and
   // a code is below the end of its length's range and of no shorter one's
+  constexpr uint32_t kLitBits = C::kLitBits;
   uint32_t end[kLitBits];
 #pragma unroll
   for (uint32_t l = 0; l < kLitBits; ++l) end[l] = l < nbits ? c.end[l + 1] : 0u;
-  for (uint32_t i = tid; i < (1u << nbits); i += kInfThreads) {
+  for (uint32_t i = tid; i < (1u << nbits); i += N) {
     const uint32_t code = __brev(i) >> 17;
     uint32_t l = 1;
 #pragma unroll
@@ -279,14 +306,16 @@ __device__ bool build_code(InfSmem& S, Canon& c, const uint8_t* lens, uint32_t n
 // Reads a dynamic block's code lengths, from bit `at` of the staged words (all
 // threads; the first warp decodes).  Returns false for an invalid header; S.used is
 // the bit after it.
-__device__ bool read_lengths(InfSmem& S, uint32_t at) {
+template <class C>
+__device__ bool read_lengths(InfSmem<C>& S, uint32_t at) {
   const uint32_t tid = threadIdx.x, lane = tid & 31;
+  constexpr uint32_t N = C::kThreads;
   auto bits_at = [&](uint32_t o) { return __funnelshift_r(S.words[o >> 5], S.words[(o >> 5) + 1], o & 31u); };
   const uint32_t h = bits_at(at);
   const uint32_t hlit = (h & 31u) + 257, hdist = ((h >> 5) & 31u) + 1, hclen = ((h >> 10) & 15u) + 4;
   at += 14;
   if (hlit > 286 || hdist > 30) return false;
-  if (tid < 320) S.raw[tid] = 0;
+  for (uint32_t i = tid; i < 320; i += N) S.raw[i] = 0;
   if (tid < 19) S.lens[c_cl_order[tid]] = tid < hclen ? uint8_t(bits_at(at + 3 * tid) & 7u) : uint8_t(0);
   at += 3 * hclen;
   __syncthreads();
@@ -342,8 +371,8 @@ __device__ bool read_lengths(InfSmem& S, uint32_t at) {
   }
   __syncthreads();
   if (S.bad) return false;
-  if (tid < 288) S.lens[tid] = tid < hlit ? S.raw[tid] : 0;
-  else if (tid < 320) S.lens[tid] = tid - 288 < hdist ? S.raw[hlit + tid - 288] : 0;
+  for (uint32_t i = tid; i < 320; i += N)
+    S.lens[i] = i < 288 ? (i < hlit ? S.raw[i] : 0) : i - 288 < hdist ? S.raw[hlit + i - 288] : 0;
   __syncthreads();
   return S.lens[256] != 0;  // a block needs an end-of-block code
 }
@@ -351,11 +380,15 @@ __device__ bool read_lengths(InfSmem& S, uint32_t at) {
 }  // namespace
 
 // status: kInfOk, kInfData (corrupt), kInfOutput (output full), kInfInput (input exhausted)
-__global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __restrict__ in, uint8_t* out,
+template <class C>
+__global__ void __launch_bounds__(C::kThreads, 1024 / C::kThreads) k_inflate(const uint8_t* __restrict__ in, uint8_t* out,
                                                             InflateJob* jobs, const uint32_t* __restrict__ order,
                                                             uint32_t njobs, uint32_t* counter) {
   extern __shared__ __align__(16) uint8_t inf_smem[];
-  InfSmem& S = *reinterpret_cast<InfSmem*>(inf_smem);
+  InfSmem<C>& S = *reinterpret_cast<InfSmem<C>*>(inf_smem);
+  constexpr uint32_t N = C::kThreads, kParts = C::kParts, kPartBits = C::kPartBits, kWindowWords = C::kWindowWords;
+  constexpr uint32_t kBatch = C::kBatch, kPiece = C::kPiece;
+  constexpr int kLitBits = C::kLitBits, kDistBits = C::kDistBits;
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   bool fixed_tables = false;  // the tables are those of the fixed code
   for (;;) {
@@ -386,7 +419,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
       if (q - sq < kWindowWords && uint32_t(q - sq) * 32 + r + bits <= kWindowWords * 32)
         return uint32_t(q - sq) * 32 + r;
       sq = q;
-      for (uint32_t k = tid; k < kWindowWords; k += kInfThreads) S.words[k] = word_at(aw, q + k, endb);
+      for (uint32_t k = tid; k < kWindowWords; k += N) S.words[k] = word_at(aw, q + k, endb);
       __syncthreads();
       return r;
     };
@@ -406,7 +439,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
         if ((inv ^ 0xFFFFu) != len) { status = kInfData; break; }
         if (src + 4 + len > job.in_len) { status = kInfInput; break; }
         if (op + len > job.out_cap) { status = kInfOutput; break; }
-        for (uint32_t i = tid; i < len; i += kInfThreads) o[op + i] = base[src + 4 + i];
+        for (uint32_t i = tid; i < len; i += N) o[op + i] = base[src + 4 + i];
         op += len;
         P = (src + 4 + len) * 8;
         continue;
@@ -414,7 +447,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
       uint32_t used = r + 3;
       if (type == 1) {
         if (!fixed_tables) {
-          if (tid < 320) S.lens[tid] = tid < 144 ? 8 : tid < 256 ? 9 : tid < 280 ? 7 : tid < 288 ? 8 : 5;
+          for (uint32_t i = tid; i < 320; i += N) S.lens[i] = i < 144 ? 8 : i < 256 ? 9 : i < 280 ? 7 : i < 288 ? 8 : 5;
           __syncthreads();
         }
       } else {
@@ -652,13 +685,13 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
             }
             __syncthreads();
             // bytes before the piece, neighbours by neighbouring threads
-            uint32_t open = 0;  // bytes of this thread (tid + k * kInfThreads) that are not known yet
+            uint32_t open = 0;  // bytes of this thread (tid + k * N) that are not known yet
 #pragma unroll
             for (uint32_t k0 = 0; k0 < 16; k0 += 8) {
               uint32_t v[8];
 #pragma unroll
               for (uint32_t k = 0; k < 8; ++k) {
-                const uint32_t j = tid + (k0 + k) * kInfThreads;
+                const uint32_t j = tid + (k0 + k) * N;
                 v[k] = j < n ? S.value[j] : kDone;
               }
 #pragma unroll
@@ -666,7 +699,7 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
                 if (v[k] & kBefore) v[k] = kHistory | ob[-1 - int(v[k] & 0x7FFFu)];
 #pragma unroll
               for (uint32_t k = 0; k < 8; ++k) {
-                const uint32_t j = tid + (k0 + k) * kInfThreads;
+                const uint32_t j = tid + (k0 + k) * N;
                 if (v[k] & kHistory) S.value[j] = uint16_t(kDone | (v[k] & 255u));
                 else if (!(v[k] & kDone)) open |= 1u << (k0 + k);
               }
@@ -678,18 +711,18 @@ __global__ void __launch_bounds__(kInfThreads, 1) k_inflate(const uint8_t* __res
                 if (!((open >> k0) & 0xFFu)) continue;
                 uint32_t w[8];
 #pragma unroll
-                for (uint32_t k = 0; k < 8; ++k) w[k] = (open >> (k0 + k)) & 1u ? S.value[tid + (k0 + k) * kInfThreads] : 0u;
+                for (uint32_t k = 0; k < 8; ++k) w[k] = (open >> (k0 + k)) & 1u ? S.value[tid + (k0 + k) * N] : 0u;
 #pragma unroll
                 for (uint32_t k = 0; k < 8; ++k) w[k] = S.value[w[k]];
 #pragma unroll
                 for (uint32_t k = 0; k < 8; ++k) {
                   if (!((open >> (k0 + k)) & 1u)) continue;
-                  S.value[tid + (k0 + k) * kInfThreads] = uint16_t(w[k]);
+                  S.value[tid + (k0 + k) * N] = uint16_t(w[k]);
                   if (w[k] & kDone) open &= ~(1u << (k0 + k));
                 }
               }
             }
-            for (uint32_t j = tid; j < n; j += kInfThreads) ob[j] = uint8_t(S.value[j]);
+            for (uint32_t j = tid; j < n; j += N) ob[j] = uint8_t(S.value[j]);
             __syncthreads();
           }
           if (status != kInfOk) break;
@@ -755,18 +788,29 @@ void launch_frame_check(const uint8_t* out, const Stream* streams, InflateJob* j
   if (n) k_frame_check<<<(n + 255) / 256, 256, 0, st>>>(out, streams, jobs, n);
 }
 
-void launch_inflate(const uint8_t* in, uint8_t* out, InflateJob* jobs, const uint32_t* order, uint32_t njobs,
-                    uint32_t* counter, int sms, cudaStream_t st) {
+template <class C>
+static void launch_inflate_t(const uint8_t* in, uint8_t* out, InflateJob* jobs, const uint32_t* order, uint32_t njobs,
+                             uint32_t* counter, int sms, cudaStream_t st) {
   if (!njobs) return;
-  cudaMemsetAsync(counter, 0, 4, st);
-  const uint32_t blocks = njobs < uint32_t(sms) ? njobs : uint32_t(sms);
-  static std::atomic<bool> attr_set[64];
+  static std::atomic<int> ctas_per_sm[64];
   const int ds = device_slot();
-  if (!attr_set[ds].load(std::memory_order_relaxed)) {
-    if (cudaFuncSetAttribute(k_inflate, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(InfSmem))) == cudaSuccess)
-      attr_set[ds].store(true, std::memory_order_relaxed);
+  int per_sm = ctas_per_sm[ds].load(std::memory_order_relaxed);
+  if (!per_sm) {
+    cudaFuncSetAttribute(k_inflate<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(InfSmem<C>)));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_inflate<C>, C::kThreads, sizeof(InfSmem<C>));
+    if (per_sm < 1) per_sm = 1;
+    ctas_per_sm[ds].store(per_sm, std::memory_order_relaxed);
   }
-  k_inflate<<<blocks, kInfThreads, sizeof(InfSmem), st>>>(in, out, jobs, order, njobs, counter);
+  const uint32_t most = uint32_t(sms) * uint32_t(per_sm), blocks = njobs < most ? njobs : most;
+  k_inflate<C><<<blocks, C::kThreads, sizeof(InfSmem<C>), st>>>(in, out, jobs, order, njobs, counter);
+}
+
+void launch_inflate(const uint8_t* in, uint8_t* out, InflateJob* jobs, const uint32_t* order, uint32_t njobs,
+                    uint32_t nlarge, uint32_t* counters, int sms, cudaStream_t st) {
+  if (!njobs) return;
+  cudaMemsetAsync(counters, 0, 8, st);
+  launch_inflate_t<InfLarge>(in, out, jobs, order, nlarge, counters, sms, st);
+  launch_inflate_t<InfSmall>(in, out, jobs, order + nlarge, njobs - nlarge, counters + 1, sms, st);
 }
 
 void launch_inflate_compare(const uint8_t* decoded, const uint8_t* ref, InflateJob* jobs, const uint64_t* ref_off,

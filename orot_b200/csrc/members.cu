@@ -142,7 +142,8 @@ deflate_result gzip_members_decompress(Engine& e, const uint8_t* in, size_t n, u
     return DEFLATE_MEM_ERROR;
   }
   uint8_t* dec = static_cast<uint8_t*>(e.d_out.p);
-  launch_inflate(static_cast<const uint8_t*>(e.d_in.p), dec, d_jobs, d_order, uint32_t(k), d_cnt, e.sms, s);
+  launch_inflate(static_cast<const uint8_t*>(e.d_in.p), dec, d_jobs, d_order, uint32_t(k),
+                 large_streams(jobs.data(), order.data(), uint32_t(k), e.sms), d_cnt, e.sms, s);
   Work w{};
   w.in = dec;
   w.streams = d_st;
