@@ -700,11 +700,13 @@ uint32_t Engine::checksum_host(uint32_t init, const void* data, size_t n, bool a
 
 uint32_t Engine::checksum_device(uint32_t init, const uint8_t* d_data, size_t n, bool adler) {
   if (n == 0) return init;
-  // checksum blocks of the whole buffer
+  // checksum blocks of the whole buffer, from a 16-byte boundary on: k_ck_block
+  // tells by a block's offset whether it can load 16 bytes at a time
+  const uint64_t skew = reinterpret_cast<uint64_t>(d_data) & 15;
   cks.clear();
   for (uint64_t o = 0; o < n; o += 65536) {
     CkBlock c{};
-    c.in_off = o;
+    c.in_off = skew + o;
     c.len = uint32_t(std::min<uint64_t>(65536, n - o));
     c.what = adler ? kCkAdler : kCkCrc;
     cks.push_back(c);
@@ -713,7 +715,7 @@ uint32_t Engine::checksum_device(uint32_t init, const uint8_t* d_data, size_t n,
   if (!d_tables.ensure(ck_bytes + 256)) return init;
   uint32_t* d_res = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(d_tables.p) + align_up(ck_bytes, 256));
   Work w{};
-  w.in = d_data;
+  w.in = d_data - skew;
   w.ck = static_cast<CkBlock*>(d_tables.p);
   w.nck = uint32_t(cks.size());
   uint32_t res = init;

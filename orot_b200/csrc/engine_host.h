@@ -82,8 +82,8 @@ class Engine {
   bool upload(size_t dst_off, const void* src, size_t n);
   bool download(void* dst, const uint8_t* d_src, size_t n);
   uint32_t checksum_host(uint32_t init, const void* data, size_t n, bool adler);
-  // Checksum of n bytes already on the device (d_data 16-byte aligned, with
-  // readable padding after the last byte).
+  // Checksum of n bytes already on the device (in an allocation of its own or
+  // at any place of an arena, with readable padding after the last byte).
   uint32_t checksum_device(uint32_t init, const uint8_t* d_data, size_t n, bool adler);
   // Makes the arenas grow by stream-ordered allocation on the engine's own
   // stream (for engines whose work runs on that stream only).
