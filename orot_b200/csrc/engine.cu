@@ -229,38 +229,44 @@ static uint64_t put_table(std::vector<uint8_t>& buf, const std::vector<T>& v) {
   return off;
 }
 
-// Tiles per CTA of the link and the search kernel (one CTA per SM): a pass takes
-// (waves of CTAs) x (tiles per CTA + `extra`), where `extra` is what a CTA costs
-// beside its tiles, in tiles.  The smallest count within 1/8 of the cheapest is
-// taken, since tiles differ and small groups even that out.  Measured (us):
-//   links, extra 1.6 (the window before a run enters its table): 3 MiB in runs
+// Tiles per CTA of the link and the search kernel (one CTA per SM): a pass is
+// taken to cost (waves of CTAs) x (tiles per CTA + `extra`), where `extra` is what
+// a CTA costs beside its tiles, here in fifths of a tile.  The smallest count
+// within 1/8 of the cheapest is taken, since tiles differ and small groups even
+// that out; the costs themselves have no term for that, and for searches the
+// cheapest by them can be the slowest (3 MiB of mixed data in groups of 6).
+// Measured (us):
+//   links, extra 8 (the window before a run enters its table): 3 MiB in runs
 //   of 2 / 4 / 6 / 8 tiles 94 / 96 / 83 / 105; 16 MiB in 4 / 16 / 32 399 / 390 / 380
-//   search, extra 0.4 to level 6 (staging): 3 MiB of mixed data in groups of 2 /
-//   4 / 6 188 / 247 / 337, 1 MiB of text in 1 / 2 / 4 193 / 167 / 245; above, 2
+//   search, extra 2 to level 6 (staging): 3 MiB of mixed data in groups of 2 /
+//   4 / 6 188 / 247 / 337, 1 MiB of text in 1 / 2 / 4 193 / 167 / 245; above, 10
 //   (the last long chains): 32 MiB of text at level 9 in 2 / 4 / 8 5920 / 4891 / 4432
-uint32_t Engine::lazy_group(uint32_t most, float extra) const {
-  float cost[kLazyRun + 1] = {};
-  float least = 0;
+uint32_t Engine::lazy_group(const TileCounts& counts, uint32_t most, uint32_t extra) const {
+  uint64_t cost[kLazyRun + 1] = {};
+  uint64_t least = ~uint64_t(0);
   for (uint32_t G = 1; G <= most; ++G) {
     uint64_t ctas = 0;
-    for (uint32_t si : lists[kLazySegs]) ctas += (segs[si].tile_count + G - 1) / G;
-    cost[G] = float((ctas + sms - 1) / sms) * (float(G) + extra);
-    if (G == 1 || cost[G] < least) least = cost[G];
+    for (uint32_t t = 1; t <= TileCounts::kFew; ++t) ctas += uint64_t(counts.few[t]) * ((t + G - 1) / G);
+    for (uint32_t t : counts.many) ctas += (t + G - 1) / G;
+    cost[G] = (ctas + sms - 1) / sms * (5 * G + extra);
+    least = std::min(least, cost[G]);
   }
   uint32_t G = 1;
-  while (cost[G] > least * 1.125f) ++G;
+  while (cost[G] * 8 > least * 9) ++G;
   return G;
 }
 
 // The segments of a pass in groups of at most G tiles, as even as can be.
 void Engine::list_groups(int list, uint32_t G) {
+  std::vector<uint32_t>& out = lists[list];
+  out.reserve(2 * lists[kLazySegs].size());
   for (uint32_t si : lists[kLazySegs]) {
     const Segment& g = segs[si];
-    const uint32_t n = (g.tile_count + G - 1) / G;
-    for (uint32_t k = 0, t = 0; k < n; ++k) {
-      const uint32_t c = (g.tile_count - t + (n - k) - 1) / (n - k);
-      lists[list].push_back(g.tile_first + t);
-      lists[list].push_back(c);
+    uint32_t n = g.tile_count <= G ? 1 : (g.tile_count + G - 1) / G;
+    for (uint32_t t = 0; t < g.tile_count; --n) {
+      const uint32_t c = n == 1 ? g.tile_count - t : (g.tile_count - t + n - 1) / n;
+      out.push_back(g.tile_first + t);
+      out.push_back(c);
       t += c;
     }
   }
@@ -437,6 +443,10 @@ bool Engine::plan(const std::vector<Job>& jobs) {
 
   // one host buffer, one upload
   std::vector<uint8_t> buf;
+  size_t expect = 65536 + streams.size() * sizeof(Stream) + segs.size() * sizeof(Segment) + tiles.size() * (sizeof(Tile) + 16) +
+                  cks.size() * sizeof(CkBlock);
+  for (const auto& l : lists) expect += l.size() * sizeof(uint32_t);
+  buf.reserve(expect);
   off_streams = put_table(buf, streams);
   off_segs = put_table(buf, segs);
   off_tiles = put_table(buf, tiles);
@@ -445,11 +455,15 @@ bool Engine::plan(const std::vector<Job>& jobs) {
   // tiles of one segment.
   if (!lists[kLazySegs].empty()) {
     int top = 0;
-    for (uint32_t si : lists[kLazySegs]) top = std::max(top, segs[si].level);
+    TileCounts counts;
+    for (uint32_t si : lists[kLazySegs]) {
+      top = std::max(top, segs[si].level);
+      counts.add(segs[si].tile_count);
+    }
     const uint32_t cap = geometry(total).lazy_run[top <= 6 ? 0 : top <= 9 ? 1 : 2];
     const uint32_t run = lazy_run_override, most = std::max(1u, std::min(kLazyRun, run ? run : cap));
-    list_groups(kLazyRuns, run ? most : lazy_group(most, 1.6f));
-    list_groups(kLazyGroups, run ? std::min(kSearchTiles, run) : lazy_group(std::min(kSearchTiles, most), top <= 6 ? 0.4f : 2.0f));
+    list_groups(kLazyRuns, run ? most : lazy_group(counts, most, 8));
+    list_groups(kLazyGroups, run ? std::min(kSearchTiles, run) : lazy_group(counts, std::min(kSearchTiles, most), top <= 6 ? 2 : 10));
   }
   for (int i = 0; i < kNumLists; ++i) off_lists[i] = put_table(buf, lists[i]);
   off_counters = align_up(buf.size(), 256);
