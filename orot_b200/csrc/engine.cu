@@ -399,9 +399,8 @@ bool Engine::plan(const std::vector<Job>& jobs) {
         g.hdr_off = scratch;
         scratch += 1024;
       }
-      const uint32_t stored_pieces = std::max<uint32_t>(1, uint32_t((len + 65534) / 65535));
       g.piece_off = npieces - s.piece_first;
-      npieces += seg_piece_slots(g.tile_count, stored_pieces);
+      npieces += seg_piece_slots(g.tile_count, g.len);
       segs.push_back(g);
     }
     s.seg_count = uint32_t(segs.size()) - s.seg_first;

@@ -28,7 +28,8 @@ constexpr uint32_t kSegFault = 8u;       // set by a kernel that could not finis
 constexpr uint64_t kNoTable = ~uint64_t(0);
 constexpr uint32_t kNoEntry = ~0u;         // Tile::fix_entry of a tile the fix-up has not parsed yet
 constexpr uint32_t kCarryChunk = 32;       // tiles of a segment whose hash tables are scanned by themselves
-constexpr uint32_t kStoredSplit = 16;      // copies a stored piece of at most 65535 bytes is cut into
+constexpr uint32_t kStoredSplit = 16;      // copies a stored piece of 65535 bytes is cut into
+constexpr uint32_t kStoredPart = 65536 / kStoredSplit;
 
 // Stream error codes written to Stream::error.
 constexpr uint32_t kErrNone = 0, kErrCapacity = 1, kErrInternal = 2;
@@ -127,10 +128,20 @@ struct Piece {
   uint32_t value;
 };
 
+// Stored pieces of a segment (an empty one has one too), and the copies the bytes
+// of a piece are cut into.
+__host__ __device__ inline uint32_t stored_pieces(uint32_t len) { return len ? (len - 1) / 65535 + 1 : 1; }
+__host__ __device__ inline uint32_t stored_copies(uint32_t piece_len) { return (piece_len + kStoredPart - 1) / kStoredPart; }
+
 // Copy slots of a segment: one coded block (header, code table, two per tile,
-// end of block) or its stored pieces (header, length and kStoredSplit copies each).
-__host__ __device__ inline uint32_t seg_piece_slots(uint32_t tiles, uint32_t stored_pieces) {
-  const uint32_t coded = 3 + 2 * tiles, stored = (2 + kStoredSplit) * stored_pieces;
+// end of block) or its stored pieces (header, length and copies each; all but
+// the last have kStoredSplit copies).
+__host__ __device__ inline uint32_t stored_slots(uint32_t len) {
+  const uint32_t full = stored_pieces(len) - 1;
+  return full * (2 + kStoredSplit) + 2 + stored_copies(len - full * 65535);
+}
+__host__ __device__ inline uint32_t seg_piece_slots(uint32_t tiles, uint32_t len) {
+  const uint32_t coded = 3 + 2 * tiles, stored = stored_slots(len);
   return coded > stored ? coded : stored;
 }
 

@@ -217,23 +217,22 @@ __global__ void __launch_bounds__(256) k_plan_pieces(Work wk, uint32_t seg_ctas,
   const uint32_t hdr = bare ? 0 : fmt_header_bytes(s.fmt);
   uint32_t* dst = reinterpret_cast<uint32_t*>(wk.out + s.out_off);
   Piece* pc = wk.pieces + s.piece_first + sg.piece_off;
-  const uint32_t slots = seg_piece_slots(sg.tile_count, max(1u, (sg.len + 65534u) / 65535u));
+  const uint32_t slots = seg_piece_slots(sg.tile_count, sg.len);
   const uint64_t c = uint64_t(hdr) * 8 + sg.bit_off;  // block start in the output slot
   const bool last = (sg.flags & kSegLast) != 0;
   // slots that stay empty: from `used` on, and the code table's of a fixed block
   const bool coded = sg.block_type != kBlkStored;
   const uint32_t used = s.error ? 0u : coded ? 2 + 2 * sg.tile_count + (sg.block_type == kBlkDynamic ? 1u : 0u)
-                                             : (2 + kStoredSplit) * max(1u, (sg.len + 65534u) / 65535u);
+                                             : stored_slots(sg.len);
   for (uint32_t i = used + lane; i < slots; i += N) pc[i].nbits = 0;
   if (s.error) return;
   if (lane == 0 && sg.block_type == kBlkFixed) pc[1].nbits = 0;
   if (sg.block_type == kBlkStored) {
-    const uint32_t P = max(1u, (sg.len + 65534u) / 65535u);
-    const uint64_t c1 = ((c + 3 + 7) & ~uint64_t(7)) + 32 + 8ull * 65535;  // start of piece 1 (when P > 1)
-    // per stored piece its header, its length and kStoredSplit copies of 4 KiB
-    // at most: one warp copies a Piece
+    const uint64_t c1 = ((c + 3 + 7) & ~uint64_t(7)) + 32 + 8ull * 65535;  // start of piece 1 (if there is one)
+    // per stored piece its header, its length and copies of 4 KiB at most: one
+    // warp copies a Piece
     constexpr uint32_t kPer = 2 + kStoredSplit;
-    for (uint32_t x = lane; x < P * kPer; x += N) {
+    for (uint32_t x = lane; x < used; x += N) {
       const uint32_t i = x / kPer, k = x % kPer;
       const uint64_t ci = i == 0 ? c : c1 + uint64_t(i - 1) * (40 + 8ull * 65535);
       const uint32_t off = i * 65535u, n = min(sg.len - off, 65535u);
@@ -244,15 +243,10 @@ __global__ void __launch_bounds__(256) k_plan_pieces(Work wk, uint32_t seg_ctas,
       } else if (k == 1) {
         pc[x] = Piece{nullptr, dst, 0, lenpos, 32, n | ((~n & 0xFFFFu) << 16)};
       } else {
-        constexpr uint32_t kPart = 65536 / kStoredSplit;
-        const uint32_t o = (k - 2) * kPart;
-        if (o >= n) {
-          pc[x].nbits = 0;
-          continue;
-        }
+        const uint32_t o = (k - 2) * kStoredPart;
         const uint64_t a = sg.in_off + off + o;
         pc[x] = Piece{reinterpret_cast<const uint32_t*>(wk.in + (a & ~uint64_t(3))), dst, (a & 3) * 8,
-                      lenpos + 32 + 8ull * o, min(kPart, n - o) * 8, 0};
+                      lenpos + 32 + 8ull * o, min(kStoredPart, n - o) * 8, 0};
       }
     }
     return;
