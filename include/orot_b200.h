@@ -295,6 +295,13 @@ const char* orot_b200_geometry_source(void);
  * counterpart in the reference; needs no GPU).  OROT_B200_TILE, when set, overrides it in a pass. */
 uint32_t orot_b200_geometry_tile(uint64_t pass_bytes, int sms, int hash_bits);
 
+/* Device bytes a stream of `stream_bytes` takes at `level` in a pass of
+ * `pass_bytes` on a device of `sms` SMs, one block per stream: what the server
+ * charges to its device budget for a request (no counterpart in the reference;
+ * needs no GPU).  A stream alone in a small pass takes most per byte, since its
+ * tiles, which carry a hash table each at levels 1-3, are the smallest. */
+uint64_t orot_b200_device_bytes(uint64_t stream_bytes, uint64_t pass_bytes, int sms, int level);
+
 #ifdef __cplusplus
 }
 #endif

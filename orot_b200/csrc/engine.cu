@@ -221,6 +221,31 @@ uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
   return tile_override ? tile_override : plan_tile(total_bytes, sms, hash_bits);
 }
 
+uint64_t stream_device_bytes(uint64_t n, int level, uint32_t tile12, uint32_t tile14) {
+  const int lv = clamp_level(level);
+  // input, output slot and packed output
+  uint64_t bytes = align_up(n, 16) + 2 * align_up(framed_bound(n, kFmtGzip), 16);
+  uint64_t nt = 0;  // tiles
+  if (lv >= 4) {
+    nt = std::max<uint64_t>(1, (n + kLazyTile - 1) / kLazyTile);
+    bytes += (nt - 1) * lazy_stream_bytes(kLazyTile) + lazy_stream_bytes(uint32_t(n - (nt - 1) * kLazyTile));
+    bytes += align_up(n * 4 + 4, 256) + 2 * 320 * 4 + 1024;
+  } else if (lv > 0) {
+    const uint64_t T = lv == 1 ? tile12 : tile14, table = uint64_t(4) << (lv == 1 ? 12 : 14);
+    auto tile = [](uint32_t len) {
+      return 2 * tile_stream_bytes(len) + align_up(uint64_t((len + 31) / 32) * sizeof(WinRec), 256) + align_up(uint64_t(len) * 2 + 64, 256);
+    };
+    nt = std::max<uint64_t>(1, (n + T - 1) / T);
+    bytes += (nt - 1) * (tile(uint32_t(T)) + table) + tile(uint32_t(n - (nt - 1) * T));
+    const uint64_t nc = (nt - 1 + kCarryChunk - 1) / kCarryChunk;
+    if (nc > 1) bytes += nc * table;
+  }
+  // the tables and lists of plan()
+  bytes += sizeof(Stream) + sizeof(Segment) + nt * (sizeof(Tile) + 32) + (n / 65536 + 1) * sizeof(CkBlock) +
+           uint64_t(seg_piece_slots(uint32_t(nt), uint32_t(n))) * sizeof(Piece);
+  return bytes;
+}
+
 template <class T>
 static uint64_t put_table(std::vector<uint8_t>& buf, const std::vector<T>& v) {
   const uint64_t off = align_up(buf.size(), 256);
@@ -870,6 +895,9 @@ const char* orot_b200_geometry_source(void) { return kGeometrySource; }
 
 uint32_t orot_b200_geometry_tile(uint64_t pass_bytes, int sms, int hash_bits) {
   return plan_tile(pass_bytes, sms, hash_bits);
+}
+uint64_t orot_b200_device_bytes(uint64_t stream_bytes, uint64_t pass_bytes, int sms, int level) {
+  return stream_device_bytes(stream_bytes, level, plan_tile(pass_bytes, sms, 12), plan_tile(pass_bytes, sms, 14));
 }
 
 }  // extern "C"

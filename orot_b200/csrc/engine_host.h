@@ -39,6 +39,11 @@ struct HostBuf {
   void release();
 };
 
+// Device bytes that a stream of n bytes and one segment takes in a pass of these
+// tile sizes: input, output, packed output, scratch and tables (as Engine::plan
+// lays them out, without the rounding of whole arenas).
+uint64_t stream_device_bytes(uint64_t n, int level, uint32_t tile12, uint32_t tile14);
+
 // One output stream to produce.
 struct Job {
   uint64_t in_off;      // in the input arena (16-byte aligned)

@@ -35,13 +35,6 @@ namespace orotb {
 
 using Clock = std::chrono::steady_clock;
 
-// Device bytes a buffer of n bytes needs in a pass (input, output slot,
-// scratch), used for admission against the budget.
-static uint64_t device_estimate(uint64_t n, int level) {
-  const int lv = clamp_level(level);
-  return align_up(n, 16) + align_up(framed_bound(n, 2), 16) + (lv >= 4 ? 7 : 6) * n + 4096;
-}
-
 struct Lane {
   Engine eng;
   std::vector<Job> jobs;
@@ -238,16 +231,26 @@ void Server::run() {
       for (Lane* L : lanes) {
         if (L->state != 0 || pending.empty()) continue;
         std::vector<Req*> group;
-        uint64_t bytes = 0, est = 0;
+        uint64_t bytes = 0, est = 0;  // est: device bytes of the group's pass
+        uint32_t t12 = 0, t14 = 0;
         while (!pending.empty()) {
           Req* r = pending.front();
-          const uint64_t e1 = device_estimate(r->n, r->level);
-          if (!group.empty() && (bytes + r->n > max_group || in_use + est + e1 > budget)) break;
-          if (group.empty() && in_use + e1 > budget && in_use > 0) break;  // wait for memory
+          // the tiles, and with them what each stream takes, depend on the whole pass
+          const uint32_t n12 = L->eng.pick_tile(bytes + r->n, 12), n14 = L->eng.pick_tile(bytes + r->n, 14);
+          uint64_t e = est;
+          if (n12 != t12 || n14 != t14) {
+            e = 0;
+            for (const Req* q : group) e += stream_device_bytes(q->n, q->level, n12, n14);
+          }
+          e += stream_device_bytes(r->n, r->level, n12, n14);
+          if (!group.empty() && (bytes + r->n > max_group || in_use + e > budget)) break;
+          if (group.empty() && in_use + e > budget && in_use > 0) break;  // wait for memory
           group.push_back(r);
           pending.pop_front();
           bytes += r->n;
-          est += e1;
+          est = e;
+          t12 = n12;
+          t14 = n14;
         }
         if (group.empty()) break;
         in_use += est;

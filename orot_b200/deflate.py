@@ -70,6 +70,8 @@ def lib() -> ctypes.CDLL:
     L.orot_b200_geometry_source.restype = c.c_char_p
     L.orot_b200_geometry_tile.restype = c.c_uint32
     L.orot_b200_geometry_tile.argtypes = [c.c_uint64, c.c_int, c.c_int]
+    L.orot_b200_device_bytes.restype = c.c_uint64
+    L.orot_b200_device_bytes.argtypes = [c.c_uint64, c.c_uint64, c.c_int, c.c_int]
     L.deflate_gpu_batch_new.restype = c.c_void_p
     L.deflate_gpu_batch_free.argtypes = [c.c_void_p]
     L.deflate_gpu_batch_load.restype = c.c_int
@@ -151,6 +153,12 @@ def geometry_tile(pass_bytes: int, sms: int = 148, hash_bits: int = 12) -> int:
     """Tile bytes the planner uses at levels 1-3 for a pass of `pass_bytes`
     on a device of `sms` SMs (hash_bits 12: level 1, 14: levels 2-3)."""
     return int(lib().orot_b200_geometry_tile(int(pass_bytes), int(sms), int(hash_bits)))
+
+
+def device_bytes(stream_bytes: int, pass_bytes: int, level: int, sms: int = 148) -> int:
+    """Device bytes a stream of `stream_bytes` takes at `level` in a pass of
+    `pass_bytes`: what the server charges to its budget for a request."""
+    return int(lib().orot_b200_device_bytes(int(stream_bytes), int(pass_bytes), int(sms), int(level)))
 
 
 _new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
