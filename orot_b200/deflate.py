@@ -193,6 +193,20 @@ def _ptr(buf) -> tuple[int, int, object]:
     return ctypes.addressof(arr), len(mv), (arr, mv)
 
 
+def _outptr(buf) -> tuple[int, int, object]:
+    """(address, length, keepalive) of a buffer the library writes into; raises
+    TypeError for one that is read-only or not contiguous."""
+    flags = getattr(buf, "flags", None)
+    if hasattr(flags, "writeable"):  # a numpy array
+        ok = flags.writeable and flags.c_contiguous
+    else:
+        mv = memoryview(buf)
+        ok = not mv.readonly and mv.c_contiguous
+    if not ok:
+        raise TypeError("the output needs a writable, contiguous buffer")
+    return _ptr(buf)
+
+
 def compress_bound(n: int, format: Format = Format.Zlib) -> int:
     return lib().deflate_compress_bound(n, int(format))
 
@@ -346,7 +360,7 @@ def compress_packed(concat, sizes: Sequence[int], level: int, format: Format, ou
     (packed_total, offsets, sizes)."""
     L = lib()
     addr, n, keep = _ptr(concat)
-    oaddr, on, okeep = _ptr(out)
+    oaddr, on, okeep = _outptr(out)
     cnt = len(sizes)
     arr = (ctypes.c_size_t * cnt)(*sizes)
     offs = (ctypes.c_uint64 * (cnt + 1))()
@@ -367,7 +381,7 @@ def compress_pipelined(concat, sizes, level: int, format: Format, out, group_byt
     import numpy as np
     L = lib()
     addr, n, keep = _ptr(concat)
-    oaddr, on, okeep = _ptr(out)
+    oaddr, on, okeep = _outptr(out)
     sz = np.ascontiguousarray(sizes, dtype=np.uint64)
     cnt = len(sz)
     offs = np.empty(cnt + 1, np.uint64)
@@ -401,7 +415,7 @@ class Server:
             out = ctypes.create_string_buffer(max(cap, 1))
         else:
             cap = len(out) if out_capacity is None else out_capacity
-        oaddr, _, okeep = _ptr(out)
+        oaddr, _, okeep = _outptr(out)
         t = lib().deflate_gpu_server_submit(self._s, addr if n else None, n, oaddr, cap, int(level), int(format))
         if t == 0:
             raise Error(DEFLATE_PARAM_ERROR, "server submit: " + last_error())
