@@ -153,10 +153,19 @@ Engine::Engine() {
     const long t = std::strtol(v, nullptr, 10);
     if (t >= 32 && t <= 65536 && t % 32 == 0) tile_override = uint32_t(t);
   }
-  // Lazy-level run length override (tiles per CTA, 1..kLazyRun) for tests.
+  // Tiles per CTA of the link kernel and (up to kSearchTiles) the search kernel, for tests.
   if (const char* v = std::getenv("OROT_B200_LAZY_RUN")) {
     const long r = std::strtol(v, nullptr, 10);
     if (r >= 1 && r <= long(kLazyRun)) lazy_run_override = uint32_t(r);
+  }
+  // A row in place of the geometry table's, for the tuner: tile12,tile14,run.
+  if (const char* v = std::getenv("OROT_B200_GEOMETRY")) {
+    unsigned a = 0, b = 0, r = 0;
+    auto tile = [](unsigned t) { return t >= 512 && t <= 65536 && (t & (t - 1)) == 0; };
+    if (std::sscanf(v, "%u,%u,%u", &a, &b, &r) == 3 && tile(a) && tile(b) && r >= 1 && r <= kLazyRun) {
+      row_override = GeometryRow{0, a, b, {r, r, r}};
+      row_set = true;
+    }
   }
 }
 Engine::~Engine() {
@@ -187,7 +196,9 @@ static const GeometryRow& geometry_row(uint64_t total_bytes, int sms) {
   return kGeometry[k];
 }
 
-const GeometryRow& Engine::geometry(uint64_t total_bytes) const { return geometry_row(total_bytes, sms); }
+const GeometryRow& Engine::geometry(uint64_t total_bytes) const {
+  return row_set ? row_override : geometry_row(total_bytes, sms);
+}
 
 // Tile bytes of a pass: the table's, but passes of a few MiB are bound by the
 // time one warp needs for a tile (about 25 us for 1 KiB, once to find candidates
@@ -204,8 +215,7 @@ const GeometryRow& Engine::geometry(uint64_t total_bytes) const { return geometr
 //             1 MiB 314 / 183 / 173 / 218     2 MiB 542 / 335 / 226 / 240
 //             4 MiB 989 / 576 / 386 / 303
 // An empty pass has nothing to cut.
-static uint32_t plan_tile(uint64_t total_bytes, int sms, int hash_bits) {
-  const GeometryRow& g = geometry_row(total_bytes, sms);
+static uint32_t plan_tile(const GeometryRow& g, uint64_t total_bytes, int sms, int hash_bits) {
   const uint32_t most = hash_bits <= 12 ? g.tile12 : g.tile14;
   if (!total_bytes) return most;
   const uint64_t scaled = total_bytes * 148u / uint64_t(std::max(sms, 1));
@@ -218,7 +228,7 @@ static uint32_t plan_tile(uint64_t total_bytes, int sms, int hash_bits) {
   return t;
 }
 uint32_t Engine::pick_tile(uint64_t total_bytes, int hash_bits) const {
-  return tile_override ? tile_override : plan_tile(total_bytes, sms, hash_bits);
+  return tile_override ? tile_override : plan_tile(geometry(total_bytes), total_bytes, sms, hash_bits);
 }
 
 uint64_t stream_device_bytes(uint64_t n, int level, uint32_t tile12, uint32_t tile14) {
@@ -894,10 +904,11 @@ const char* orot_b200_last_error(void) { return g_err.c_str(); }
 const char* orot_b200_geometry_source(void) { return kGeometrySource; }
 
 uint32_t orot_b200_geometry_tile(uint64_t pass_bytes, int sms, int hash_bits) {
-  return plan_tile(pass_bytes, sms, hash_bits);
+  return plan_tile(geometry_row(pass_bytes, sms), pass_bytes, sms, hash_bits);
 }
 uint64_t orot_b200_device_bytes(uint64_t stream_bytes, uint64_t pass_bytes, int sms, int level) {
-  return stream_device_bytes(stream_bytes, level, plan_tile(pass_bytes, sms, 12), plan_tile(pass_bytes, sms, 14));
+  const GeometryRow& g = geometry_row(pass_bytes, sms);
+  return stream_device_bytes(stream_bytes, level, plan_tile(g, pass_bytes, sms, 12), plan_tile(g, pass_bytes, sms, 14));
 }
 
 }  // extern "C"

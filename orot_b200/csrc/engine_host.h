@@ -118,6 +118,8 @@ class Engine {
   cudaGraphExec_t graph_exec = nullptr;
   uint32_t tile_override = 0;
   uint32_t lazy_run_override = 0;
+  GeometryRow row_override{};  // in place of the table's, where row_set
+  bool row_set = false;
 
   // planned tables (host copies)
   std::vector<Stream> streams;

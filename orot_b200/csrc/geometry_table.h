@@ -1,11 +1,10 @@
 // geometry_table.h -- pass geometry per pass-size class, read by Engine::plan.
 //
-// Written by `python -m orot_b200.tune` (the autotuner), which times every
-// candidate on the device and keeps the fastest; this version holds the
-// hand-set rules the tuner starts from.  A class applies to passes of at
-// least min_bytes input bytes (on a 148-SM B200; other devices scale the
-// bounds by their SM count).
-//   tile12, tile14  fast-level tile bytes at 12 hash bits (level 1) and
+// The values were set by hand from sweeps; `python -m orot_b200.tune` (the
+// autotuner) times every candidate on the device and rewrites them.  A class
+// applies to passes of at least min_bytes input bytes (on a 148-SM B200; other
+// devices scale the bounds by their SM count).  Entries are upper limits:
+//   tile12, tile14  largest fast-level tile at 12 hash bits (level 1) and
 //                   14 (levels 2-3): one warp walks one tile
 //                   (passes of a few MiB are cut finer, Engine::pick_tile)
 //   lazy_run[g]     most tiles one CTA links or searches at levels 4-6, 7-9 and
