@@ -276,13 +276,12 @@ static uint64_t put_table(std::vector<uint8_t>& buf, const std::vector<T>& v) {
 //   search, extra 2 to level 6 (staging): 3 MiB of mixed data in groups of 2 /
 //   4 / 6 188 / 247 / 337, 1 MiB of text in 1 / 2 / 4 193 / 167 / 245; above, 10
 //   (the last long chains): 32 MiB of text at level 9 in 2 / 4 / 8 5920 / 4891 / 4432
-uint32_t Engine::lazy_group(const TileCounts& counts, uint32_t most, uint32_t extra) const {
+uint32_t Engine::lazy_group(const std::vector<TileCount>& counts, uint32_t most, uint32_t extra) const {
   uint64_t cost[kLazyRun + 1] = {};
   uint64_t least = ~uint64_t(0);
   for (uint32_t G = 1; G <= most; ++G) {
     uint64_t ctas = 0;
-    for (uint32_t t = 1; t <= TileCounts::kFew; ++t) ctas += uint64_t(counts.few[t]) * ((t + G - 1) / G);
-    for (uint32_t t : counts.many) ctas += (t + G - 1) / G;
+    for (const TileCount& c : counts) ctas += uint64_t(c.segs) * ((c.tiles + G - 1) / G);
     cost[G] = (ctas + sms - 1) / sms * (5 * G + extra);
     least = std::min(least, cost[G]);
   }
@@ -477,7 +476,7 @@ bool Engine::plan(const std::vector<Job>& jobs) {
 
   // one host buffer, one upload
   std::vector<uint8_t> buf;
-  size_t expect = 65536 + streams.size() * sizeof(Stream) + segs.size() * sizeof(Segment) + tiles.size() * (sizeof(Tile) + 16) +
+  size_t expect = 8192 + streams.size() * sizeof(Stream) + segs.size() * sizeof(Segment) + tiles.size() * (sizeof(Tile) + 16) +
                   cks.size() * sizeof(CkBlock);
   for (const auto& l : lists) expect += l.size() * sizeof(uint32_t);
   buf.reserve(expect);
@@ -489,11 +488,16 @@ bool Engine::plan(const std::vector<Job>& jobs) {
   // tiles of one segment.
   if (!lists[kLazySegs].empty()) {
     int top = 0;
-    TileCounts counts;
+    std::vector<TileCount> counts;
+    uint32_t few[65] = {};  // segments of up to 64 tiles, by their tiles
     for (uint32_t si : lists[kLazySegs]) {
+      const uint32_t t = segs[si].tile_count;
       top = std::max(top, segs[si].level);
-      counts.add(segs[si].tile_count);
+      if (t <= 64) ++few[t];
+      else counts.push_back(TileCount{t, 1});
     }
+    for (uint32_t t = 1; t <= 64; ++t)
+      if (few[t]) counts.push_back(TileCount{t, few[t]});
     const uint32_t cap = geometry(total).lazy_run[top <= 6 ? 0 : top <= 9 ? 1 : 2];
     const uint32_t run = lazy_run_override, most = std::max(1u, std::min(kLazyRun, run ? run : cap));
     list_groups(kLazyRuns, run ? most : lazy_group(counts, most, 8));

@@ -64,16 +64,10 @@ enum ListId {
   kNumLists
 };
 
-// Segments by their number of tiles (a batch has thousands of few tiles, and
-// the group rule looks at them for every group size).
-struct TileCounts {
-  static constexpr uint32_t kFew = 64;
-  uint32_t few[kFew + 1] = {};  // segments of that many tiles
-  std::vector<uint32_t> many;   // the tile counts above
-  void add(uint32_t tiles) {
-    if (tiles <= kFew) ++few[tiles];
-    else many.push_back(tiles);
-  }
+// So many segments of so many tiles (a batch has thousands of a few tiles, and the
+// group rule looks at them for every group size).
+struct TileCount {
+  uint32_t tiles, segs;
 };
 
 class Engine {
@@ -107,7 +101,7 @@ class Engine {
   void use_stream_ordered_arenas();
   uint32_t pick_tile(uint64_t total_bytes, int hash_bits) const;
   const GeometryRow& geometry(uint64_t total_bytes) const;
-  uint32_t lazy_group(const TileCounts& counts, uint32_t most, uint32_t extra) const;
+  uint32_t lazy_group(const std::vector<TileCount>& counts, uint32_t most, uint32_t extra) const;
   void list_groups(int list, uint32_t G);
 
   int device = 0, sms = 148;
