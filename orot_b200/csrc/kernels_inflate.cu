@@ -54,7 +54,7 @@
 // parts of 480 bits 2.2.
 // A stream of short blocks pays for each block, not for what lies behind it:
 // words stay staged, the fixed code's tables stay, and the first window of a
-// block is about twice the block before (1 MiB of text in blocks of 100 bytes
+// block is about twice the longer of the two before (1 MiB of text in blocks of 100 bytes
 // each behind a flush: 717 ms with whole windows staged and decoded, now 360;
 // with the fixed code 437 and 189; one warp per stream took 489 and 324).
 //
@@ -153,6 +153,9 @@ struct InfSmem {
   uint32_t groups[10][16];           // build: codes of each length per 32 symbols
   uint8_t lens[320], raw[320];       // code lengths: literal/length at 0, distance at 288; as read
   uint32_t job, type, bad, used, stop;
+  uint64_t staged;                   // the stream's word at words[0]
+  uint64_t block_at;                 // the block's first bit behind its header
+  uint32_t parts[2];                 // twice the sizes of the last two blocks
   static_assert(C::kParts * C::kPartBits + kOverBits + 31 <= C::kWindowWords * 32 && kHeaderBits + 31 <= C::kWindowWords * 32,
                 "a window fits from any bit of its first word");
 };
@@ -393,7 +396,11 @@ __global__ void __launch_bounds__(C::kThreads, 1024 / C::kThreads) k_inflate(con
   bool fixed_tables = false;  // the tables are those of the fixed code
   for (;;) {
     __syncthreads();
-    if (tid == 0) S.job = atomicAdd(counter, 1u);
+    if (tid == 0) {
+      S.job = atomicAdd(counter, 1u);
+      S.staged = uint64_t(1) << 63;  // none
+      S.parts[0] = S.parts[1] = kParts;
+    }
     __syncthreads();
     if (S.job >= njobs) break;
     InflateJob* jp = jobs + order[S.job];
@@ -408,17 +415,15 @@ __global__ void __launch_bounds__(C::kThreads, 1024 / C::kThreads) k_inflate(con
     uint64_t op = 0;  // output position
     int32_t status = kInfOk;
     bool last = false;
-    uint64_t sq = uint64_t(1) << 63;  // the first staged word (none)
-    uint32_t first_parts = kParts;  // parts in the first window of a block
     // stages the words from bit P on unless `bits` from there are staged;
     // returns the bit of P in the staged words
     auto stage = [&](uint32_t bits) -> uint32_t {
       const uint64_t q = (s0 + P) >> 5;
       const uint32_t r = uint32_t((s0 + P) & 31u);
+      const uint64_t w = q - S.staged;
       __syncthreads();  // the words staged before are no longer read
-      if (q - sq < kWindowWords && uint32_t(q - sq) * 32 + r + bits <= kWindowWords * 32)
-        return uint32_t(q - sq) * 32 + r;
-      sq = q;
+      if (w < kWindowWords && uint32_t(w) * 32 + r + bits <= kWindowWords * 32) return uint32_t(w) * 32 + r;
+      if (tid == 0) S.staged = q;
       for (uint32_t k = tid; k < kWindowWords; k += N) S.words[k] = word_at(aw, q + k, endb);
       __syncthreads();
       return r;
@@ -463,9 +468,10 @@ __global__ void __launch_bounds__(C::kThreads, 1024 / C::kThreads) k_inflate(con
       fixed_tables = type == 1;
       P += used - r;
       // What lies behind the block is decoded for nothing, so the window of a
-      // block behind a short one starts at about twice that one's size.
-      const uint64_t block_at = P;
-      uint32_t parts = first_parts;
+      // block behind short ones starts at about twice the longer of the last two
+      // (of the last alone: 12% slower where blocks of 100 bytes and of 60 KB alternate).
+      if (tid == 0) S.block_at = P;
+      uint32_t parts = max(S.parts[0], S.parts[1]);
 
       bool block_end = false;
       while (!block_end) {
@@ -556,7 +562,10 @@ __global__ void __launch_bounds__(C::kThreads, 1024 / C::kThreads) k_inflate(con
         block_end = (stop_end & kEndBlock) != 0;
         P += stop_end & ~kEndFlags;
         parts = kParts;
-        if (block_end) first_parts = uint32_t(min(uint64_t(kParts), (P - block_at) / (kPartBits / 2) + 4));
+        if (block_end && tid == 0) {
+          S.parts[1] = S.parts[0];
+          S.parts[0] = uint32_t(min(uint64_t(kParts), (P - S.block_at) / (kPartBits / 2) + 4));
+        }
 
         // -- tokens, a batch at a time
         constexpr uint32_t kPartWords = kPartBits / 32;
