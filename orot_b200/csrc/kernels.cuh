@@ -130,10 +130,11 @@ constexpr int32_t kInfOk = 0, kInfData = 1, kInfOutput = 2, kInfInput = 3, kInfM
 // large one would wait for the same dozens of steps whatever the stream's length: for
 // short streams, the longer the more rounds of large CTAs they would take, and
 // most of the streams, since the small CTAs start after the large ones.
-// deflate_gpu_batch_verify of zlib level-6-like text (us), all large / small / with
-// the one warp per stream that went before: 300 of 100 to 200 bytes 186 / 134 / 167,
-// 10,000 of them 4300 / 2080 / 2090, 10,000 of 1 to 4 KiB 5200 / 2580 / 3400, 450 of 1
-// to 4 KiB 338 / 329 / 507, 1,000 of 32 to 64 KiB 1560 / 1560 / 5340.
+// deflate_gpu_batch_verify of text at level 6 (us), all large / small / with the one
+// warp per stream that went before: 300 of 100 to 200 bytes 186 / 146 / 163, 10,000
+// of them 4300 / 2080 / 2090, 10,000 of 1 to 4 KiB 5200 / 2580 / 3400, 1,000 of 32 to
+// 64 KiB 1560 / 1560 / 5340.  Limits of 512 bytes a round, or without the
+// majority, made mixed sizes up to 20% slower than all large.
 inline uint32_t large_streams(const InflateJob* jobs, const uint32_t* order, uint32_t n, int sms) {
   auto shorter = [&](uint64_t len) {
     uint32_t k = 0;

@@ -55,8 +55,8 @@
 // A stream of short blocks pays for each block, not for what lies behind it:
 // words stay staged, the fixed code's tables stay, and the first window of a
 // block is about twice the longer of the two before (1 MiB of text in blocks of 100 bytes
-// each behind a flush: 717 ms with whole windows staged and decoded, now 360;
-// with the fixed code 437 and 189; one warp per stream took 489 and 324).
+// each behind a flush: 717 ms with whole windows staged and decoded, now 366;
+// with the fixed code 437 and 193; one warp per stream took 489 and 324).
 //
 // The kernel does not read the zlib / gzip framing; the host strips it and
 // checks the trailer against a checksum of the output (src/formats/*:

@@ -12,7 +12,7 @@
 // next member are the trailer; with at least two members every member is
 // decoded into place (output offsets from the ISIZE fields), each must fill
 // exactly its ISIZE and match its CRC-32.  Here the members are decoded by
-// k_inflate, one warp per member, and their CRC-32s are computed by the
+// k_inflate, one CTA per member, and their CRC-32s are computed by the
 // checksum kernels.
 #include <cuda_runtime.h>
 #include <algorithm>
